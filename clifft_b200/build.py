@@ -10,23 +10,26 @@ the source tree.
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libclifft_gpu.so")
 
-SOURCES = ["clifft_gpu.cu", "svm_kernels_f32.cu", "svm_kernels_f64.cu", "svm_grad.cu", "svm_sample_k.cu"]
-HEADERS = ["svm_kernel.cuh", "svm_dispatch.h", "svm_instantiate.cuh", "svm_grad.h", "svm_sample_k.h"]
+SOURCES = ["clifft_gpu.cu", "svm_dispatch.cu", "svm_grad.cu", "svm_sample_k.cu"]
+INSTANCE = "svm_instance.cu"  # compiled once per row of CGPU_INSTANCES (svm_dispatch.h)
+HEADERS = ["svm_kernel.cuh", "svm_dispatch.h", "svm_grad.h", "svm_sample_k.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-O2", "-shared",
-    "--expt-relaxed-constexpr",
+    "--expt-relaxed-constexpr", "--compress-mode=size",
 ]
 
 
@@ -38,7 +41,7 @@ def nvcc() -> str:
 
 
 def _inputs():
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS]
+    deps = [os.path.join(CSRC, s) for s in [*SOURCES, INSTANCE, *HEADERS]]
     deps += [os.path.join(ROOT, "include", h) for h in ("clifft_gpu.h", "clifft_program_image.h")]
     deps.append(os.path.abspath(__file__))
     return deps
@@ -51,24 +54,39 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(d) <= t for d in _inputs())
 
 
+def _instances():
+    """(name, real, G, NW, dense) of every kernel instance."""
+    with open(os.path.join(CSRC, "svm_dispatch.h")) as f:
+        rows = re.findall(r"X\((\w+), (float|double), (-?\d+), (\d+), ([01])\)", f.read())
+    if not rows:
+        raise RuntimeError("no kernel instances listed in svm_dispatch.h")
+    return rows
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return OUT
     objdir = os.path.join(ROOT, "_build", "clifft_b200")
     os.makedirs(objdir, exist_ok=True)
     flags = [f for f in NVCC_FLAGS if f != "-shared"]
+    if verbose:
+        flags.append("-Xptxas=-v")
     inc = ["-I", os.path.join(ROOT, "include"), "-I", CSRC]
-    procs, objs = [], []
-    for src in SOURCES:
-        obj = os.path.join(objdir, src.replace(".cu", ".o"))
-        cmd = [nvcc(), *flags, *inc, "-c", os.path.join(CSRC, src), "-o", obj]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-        procs.append((src, subprocess.Popen(cmd)))
-        objs.append(obj)
-    for src, pr in procs:
-        if pr.wait() != 0:
-            raise RuntimeError(f"nvcc failed on {src}")
+    # the one-CTA-per-shot instances take longest and go first
+    rows = sorted(_instances(), key=lambda r: int(r[2]) > 0)
+    jobs = [(INSTANCE, name, [f"-DCGPU_NAME={name}", f"-DCGPU_REAL={real}", f"-DCGPU_G={g}", f"-DCGPU_NW={nw}",
+                              f"-DCGPU_DENSE={dense}"]) for name, real, g, nw, dense in rows]
+    jobs += [(src, src.replace(".cu", ""), []) for src in SOURCES]
+
+    def compile_one(job):
+        src, name, defines = job
+        obj = os.path.join(objdir, name + ".o")
+        if subprocess.run([nvcc(), *flags, *defines, *inc, "-c", os.path.join(CSRC, src), "-o", obj]).returncode:
+            raise RuntimeError(f"nvcc failed on {src} ({name})")
+        return obj
+
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        objs = list(pool.map(compile_one, jobs))
     subprocess.run([nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", *objs,
                     "-o", OUT + ".tmp"], check=True)
     os.replace(OUT + ".tmp", OUT)

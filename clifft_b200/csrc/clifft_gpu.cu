@@ -475,7 +475,7 @@ PlanShape plan_shape(const clifft_gpu_program& p, uint32_t precision, uint32_t g
     // that only moves the fused blocks' tiles (the warp-specialised kernel
     // instance, G = -1); the size is settled below for automatic requests
     auto pick_fn = [&](int kg) {
-        L.fn = precision == CLIFFT_GPU_FP32 ? kernel_f32(kg, int(L.nw_words)) : kernel_f64(kg, int(L.nw_words));
+        L.fn = find_kernel(precision == CLIFFT_GPU_FP64, kg, int(L.nw_words));
         cudaFuncAttributes fa{};
         CUDA_OK(cudaFuncGetAttributes(&fa, (const void*)L.fn));
         return std::max(32, (fa.maxThreadsPerBlock / 32) * 32);
@@ -525,7 +525,7 @@ PlanShape plan_shape(const clifft_gpu_program& p, uint32_t precision, uint32_t g
     // dense blocks: only in their own kernel instance (the others hold no
     // tcgen05 instruction), for FP32 CTA groups of 256 compute threads
     L.dense = dense && L.fuse && G == 0 && precision == CLIFFT_GPU_FP32 && L.stages == 3;
-    if (L.dense) L.fn = kernel_f32(ws_shape(uint32_t(L.threads)) ? -1 : 0, int(L.nw_words), true);
+    if (L.dense) L.fn = find_kernel(false, ws_shape(uint32_t(L.threads)) ? -1 : 0, int(L.nw_words), true);
     L.smem = region_bytes(L.state_in_smem) * L.regions + tail(L.threads);
     if (L.smem > smem_cap) invalid("measurement record too large for shared memory");
     {
