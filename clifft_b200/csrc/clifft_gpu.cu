@@ -227,6 +227,85 @@ uint32_t validate(const clifft_program_image& im) {
 }
 
 
+// The device instruction stream: the image's instructions with every star of
+// consecutive FRAME_CNOT (one shared control, or one shared target) or
+// FRAME_CZ (one shared axis) replaced by one DOP_* instruction that carries
+// the other axes as a mask. A compiled Clifford circuit is mostly such stars
+// (the greedy pivot localisation fans out from one axis): the programs under
+// tests/golden/programs shrink 3x to 12x (memory grid 4145 -> 1018, k = 24
+// 8204 -> 692 instructions), and an interpreted frame opcode costs a shot 200
+// to 570 cycles whatever it does. A run of at least kMinStar gates is
+// condensed; a pair costs about the same either way.
+struct CodeStream {
+    std::vector<uint8_t> bytes;    // 32 bytes per instruction
+    std::vector<uint32_t> origin;  // index of each one's (first) instruction in the image
+    std::vector<uint64_t> masks;   // frames wider than one word: nwt words per condensed instruction
+};
+
+CodeStream condense(const clifft_program_image& im, uint32_t nwt) {
+    constexpr uint32_t kMinStar = 2;
+    CodeStream c;
+    const uint32_t n = im.num_instructions;
+    c.bytes.resize(size_t(n) * 32);
+    c.origin.reserve(n);
+    auto word = [&](uint32_t i) { return im.instructions + size_t(i) * 32; };
+    // gates [i, end) that share `axis` in the role the opcode asks for
+    enum Role { kControl, kTarget, kEither };
+    auto star_end = [&](uint32_t i, uint8_t op, uint32_t axis, Role role) {
+        uint32_t j = i;
+        for (; j < n && word(j)[0] == op; ++j) {
+            const uint32_t a = rd16(word(j) + 4), b = rd16(word(j) + 6);
+            const bool in = role == kControl ? a == axis : role == kTarget ? b == axis : (a == axis || b == axis);
+            if (!in || a == b) break;
+        }
+        return j;
+    };
+    for (uint32_t i = 0; i < n;) {
+        const uint8_t* I = word(i);
+        const uint32_t a = rd16(I + 4), b = rd16(I + 6);
+        uint32_t end = i + 1, axis = a, dop = 0;
+        auto consider = [&](uint32_t d, uint32_t ax, Role role) {
+            const uint32_t e = star_end(i, I[0], ax, role);
+            if (e > end && e - i >= kMinStar) {
+                end = e;
+                axis = ax;
+                dop = d;
+            }
+        };
+        if (I[0] == CLIFFT_OP_FRAME_CNOT) {
+            consider(DOP_CNOT_FAN, a, kControl);
+            consider(DOP_CNOT_GATHER, b, kTarget);
+        } else if (I[0] == CLIFFT_OP_FRAME_CZ) {
+            consider(DOP_CZ_FAN, a, kEither);
+            consider(DOP_CZ_FAN, b, kEither);
+        }
+        uint8_t* J = c.bytes.data() + c.origin.size() * 32;
+        c.origin.push_back(i);
+        if (!dop) {
+            std::memcpy(J, I, 32);
+        } else {
+            uint64_t m[kMaxWords] = {};
+            for (uint32_t j = i; j < end; ++j) {
+                const uint32_t x = rd16(word(j) + 4), y = rd16(word(j) + 6), o = x == axis ? y : x;
+                m[o >> 6] ^= 1ull << (o & 63);
+            }
+            J[0] = uint8_t(dop);
+            const uint16_t ax = uint16_t(axis);
+            std::memcpy(J + 4, &ax, 2);
+            if (nwt == 1) {
+                std::memcpy(J + 8, m, 8);
+            } else {
+                const uint32_t entry = uint32_t(c.masks.size() / nwt);
+                std::memcpy(J + 8, &entry, 4);
+                c.masks.insert(c.masks.end(), m, m + nwt);
+            }
+        }
+        i = end;
+    }
+    c.bytes.resize(c.origin.size() * 32);
+    return c;
+}
+
 // Returns the current device's parked spare slab to the device (defined with
 // the spare slabs below); true when there was one.
 bool spare_release_current();
@@ -268,8 +347,10 @@ struct clifft_gpu_program {
     size_t blob_bytes = 0;
     std::vector<uint8_t> expected_host;
     int device = 0;
-    uint64_t content_hash = 0;  // FNV-1a of the device image and the launch-relevant counts
+    uint64_t content_hash = 0;  // of the device image and the launch-relevant counts
     std::vector<uint8_t> instr_host;  // the 32-byte instructions (host copy, for gradient programs)
+    std::vector<uint8_t> code_host;     // the device instruction stream
+    std::vector<uint32_t> code_origin;  // image instruction of each of its instructions
     uint32_t num_rot_params = 0;      // ARRAY_ROT + EXPAND_ROT instructions
     std::vector<double> fault_probs;  // per noise site its total probability, then per readout entry its flip
                                       // probability (clifft::noise_site_probabilities order)
@@ -659,14 +740,14 @@ constexpr uint64_t kTuneMinShots = 1024;
 constexpr uint32_t kSegHeaderBytes = 192;  // saved-state header of a shot between segments (svm_kernel.cuh)
 constexpr uint32_t kMaxSegments = 8;
 
-// Instruction cuts [0, c1, ..., n] for segmented survivor runs: each inner
-// cut follows a POSTSELECT, at about equal numbers of POSTSELECTs per
+// Cuts [0, c1, ..., n] of the device instruction stream for segmented survivor
+// runs: each inner cut follows a POSTSELECT, at about equal numbers of POSTSELECTs per
 // segment. Fewer than two POSTSELECTs give no inner cut.
 std::vector<uint32_t> segment_cuts(const clifft_gpu_program& p) {
     std::vector<uint32_t> post;
-    const uint32_t n = p.meta.num_instructions;
+    const uint32_t n = uint32_t(p.code_origin.size());
     for (uint32_t i = 0; i < n; ++i)
-        if (p.instr_host[size_t(i) * 32] == CLIFFT_OP_POSTSELECT) post.push_back(i);
+        if (p.code_host[size_t(i) * 32] == CLIFFT_OP_POSTSELECT) post.push_back(i);
     std::vector<uint32_t> cuts{0};
     const uint32_t m = std::min<uint32_t>(kMaxSegments, uint32_t(post.size()));
     for (uint32_t j = 1; j < m; ++j) {
@@ -685,6 +766,20 @@ std::map<std::tuple<uint64_t, int, uint32_t>, uint32_t> g_tuned;
 uint64_t fnv1a(const uint8_t* p, size_t n, uint64_t h = 1469598103934665603ull) {
     for (size_t i = 0; i < n; ++i) h = (h ^ p[i]) * 1099511628211ull;
     return h;
+}
+
+// Content hash of a device image: the same recurrence over 8-byte words with
+// a fold of the high half after each, so every input bit reaches the whole
+// word (byte by byte the 0.3 MB image of the k = 24 program took 0.3 ms of its
+// 0.5 ms load).
+uint64_t content_hash(const uint8_t* p, size_t n, uint64_t h = 1469598103934665603ull) {
+    for (; n >= 8; p += 8, n -= 8) {
+        uint64_t w;
+        std::memcpy(&w, p, 8);
+        h = (h ^ w) * 1099511628211ull;
+        h ^= h >> 32;
+    }
+    return fnv1a(p, n, h);
 }
 
 // Least CUDA-core weight (U4 4, U2 2, any other micro-op 1) of a run that the
@@ -799,6 +894,8 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
             psum[s] = acc;
         }
         BlobBuilder b;
+        CodeStream code = condense(im, nwt);
+        b.bytes.reserve(size_t(im.num_instructions) * 32 + code.bytes.size() + (64u << 10));
         size_t o_instr = b.put(im.instructions, size_t(im.num_instructions) * 32);
         auto px = widen(im.pauli_x, im.num_pauli_masks), pz = widen(im.pauli_z, im.num_pauli_masks);
         auto ex = widen(im.exp_val_x, im.num_exp_val_masks), ez = widen(im.exp_val_z, im.num_exp_val_masks);
@@ -836,9 +933,12 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
         {
             const uint32_t counts[] = {im.peak_rank, im.num_measurements, im.total_meas_slots, im.num_detectors,
                                        im.num_observables, im.num_exp_vals, im.num_words, im.num_instructions};
-            p->content_hash = fnv1a(reinterpret_cast<const uint8_t*>(counts), sizeof(counts),
-                                    fnv1a(b.bytes.data(), b.bytes.size()));
+            p->content_hash = content_hash(reinterpret_cast<const uint8_t*>(counts), sizeof(counts),
+                                           content_hash(b.bytes.data(), b.bytes.size()));
         }
+        size_t o_code = b.put(code.bytes.data(), code.bytes.size());
+        size_t o_mask = b.put(code.masks.data(), code.masks.size());
+        b.bytes.resize(b.bytes.size() + 256);
         p->fault_probs.assign(psum.begin(), psum.end());
         for (uint32_t r = 0; r < im.num_readout_noise; ++r) p->fault_probs.push_back(im.readout_prob[r]);
         p->instr_host.assign(static_cast<const uint8_t*>(im.instructions),
@@ -854,6 +954,11 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
         void* B = p->blob;
         d.instr = at<uint4>(B, o_instr);
         d.n_instr = im.num_instructions;
+        d.code = at<uint4>(B, o_code);
+        d.n_code = uint32_t(code.origin.size());
+        d.fmask = at<uint64_t>(B, o_mask);
+        p->code_host = std::move(code.bytes);
+        p->code_origin = std::move(code.origin);
         d.nw = nwt;
         d.peak = im.peak_rank;
         d.num_meas = im.num_measurements;
@@ -933,15 +1038,17 @@ struct DeviceFaults {
 };
 
 // Message for the first device-side error code a launch recorded; `info`
-// points at the launch's eight words of timeout diagnostics.
-std::string device_error_message(int dev_err, const unsigned long long* info) {
+// points at the launch's eight words of timeout diagnostics (its instruction
+// counts in the device stream of `p`).
+std::string device_error_message(const clifft_gpu_program& p, int dev_err, const unsigned long long* info) {
     std::string msg = dev_err == DEV_ERR_ZERO_NORM    ? "active measurement on a zero-norm state"
                       : dev_err == DEV_ERR_TIMEOUT    ? "a bounded wait on a bulk-copy barrier timed out"
                       : dev_err == DEV_ERR_BAD_OPCODE ? "device reported an invalid opcode"
                                                       : "unknown device error " + std::to_string(dev_err);
     if (dev_err == DEV_ERR_TIMEOUT) {
         const unsigned long long* e = info;
-        msg += " (pass " + std::to_string(e[0]) + ", instruction " + std::to_string(e[1]) + ", tile " +
+        msg += " (pass " + std::to_string(e[0]) + ", instruction " +
+               std::to_string(e[1] < p.code_origin.size() ? p.code_origin[e[1]] : e[1]) + ", tile " +
                std::to_string(e[2]) + "/" + std::to_string(e[3]) + ", run log2 " + std::to_string(e[4]) + ", k " +
                std::to_string(e[5]) + ", barrier word " + std::to_string(e[6]) + ", waited " +
                std::to_string(e[7]) + " cycles)";
@@ -1253,7 +1360,7 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
         for (uint64_t s = 0; s < shots && !hpz.empty(); ++s)
             for (uint32_t w = 0; w < nwo; ++w) out->final_pz[s * nwo + w] = hpz[s * nwt + w];
         const int dev_err = static_cast<int>(hs[1] & 0xffffffffu);
-        if (dev_err != 0) throw ApiError(CLIFFT_GPU_EDEVICE, device_error_message(dev_err, hs.data() + scratch_words - 8));
+        if (dev_err != 0) throw ApiError(CLIFFT_GPU_EDEVICE, device_error_message(*prog, dev_err, hs.data() + scratch_words - 8));
         out->passed_shots = hs[2];
         out->logical_errors = hs[3];
         out->dust_clamps = hs[4];
@@ -1407,7 +1514,7 @@ int clifft_gpu_sample_noalloc(clifft_gpu_program* prog, const clifft_gpu_sample_
         CUDA_OK(cudaMemcpyAsync(hs, scratch, words * 8, cudaMemcpyDeviceToHost, st));
         CUDA_OK(cudaStreamSynchronize(st));
         const int dev_err = static_cast<int>(hs[1] & 0xffffffffu);
-        if (dev_err != 0) throw ApiError(CLIFFT_GPU_EDEVICE, device_error_message(dev_err, hs + words - 8));
+        if (dev_err != 0) throw ApiError(CLIFFT_GPU_EDEVICE, device_error_message(*prog, dev_err, hs + words - 8));
         out->passed_shots = hs[2];
         out->logical_errors = hs[3];
         out->dust_clamps = hs[4];

@@ -46,6 +46,12 @@ namespace cgpu {
 struct DevProg {
     const uint4* instr;  // 2 x uint4 per instruction (32 bytes, verbatim)
     uint32_t n_instr;
+    // What the sampling kernel runs: the same instructions with every run of
+    // frame opcodes condensed (DOP_*), n_code of them; fmask holds the axis
+    // masks of the condensed ones for frames wider than one word.
+    const uint4* code;
+    uint32_t n_code;
+    const uint64_t* fmask;
     uint32_t nw;
     uint32_t peak;
     uint32_t num_meas;
@@ -155,6 +161,18 @@ enum : uint32_t {
     KSEG_FIRST = 0x2u,  // shots start from the reset state
     KSEG_LAST = 0x4u,   // shots alive at the end are finished (records written)
 };
+
+// Condensed frame opcodes of the device instruction stream (never in an
+// image): a star of consecutive FRAME_CNOT / FRAME_CZ on one shared axis
+// becomes one instruction with the other axes as a mask. axis_1 is the shared
+// axis; the mask is the 64-bit payload (one-word frames) or entry payload of
+// fmask. FAN: the shared axis controls; GATHER: it is the target.
+enum : uint32_t {
+    DOP_CNOT_FAN = 64,
+    DOP_CNOT_GATHER = 65,
+    DOP_CZ_FAN = 66,
+};
+__host__ __device__ constexpr bool frame_op(uint32_t op) { return op <= CLIFFT_OP_FRAME_SWAP || op >= DOP_CNOT_FAN; }
 
 enum : int {
     DEV_ERR_ZERO_NORM = 1,
@@ -791,54 +809,127 @@ struct Shot {
         Frame<NW>::put(f.z, a, zb);
         Frame<NW>::put(f.z, b, za);
     }
-    // A run of frame opcodes (FRAME_CNOT / CZ / H / S / S_DAG / SWAP: most of
-    // a compiled Clifford circuit) executed with the frame and gamma in
-    // registers and the next instruction word fetched one step ahead. The
-    // updates and their order are those of the per-opcode handlers above.
-    // Returns the first pc at or after `pc` that is not a frame opcode.
+    // axis mask of a condensed frame opcode
+    __device__ __forceinline__ void star_mask(const uint4& w, uint64_t (&m)[NW]) const {
+        if constexpr (NW == 1) {
+            m[0] = ((uint64_t)w.w << 32) | w.z;
+        } else {
+#pragma unroll
+            for (int i = 0; i < NW; ++i) m[i] = __ldg(P.fmask + (size_t)w.z * NW + i);
+        }
+    }
+    // A star of CNOTs / CZs on shared axis a and the axes of mask m (a not
+    // among them), as its gates one by one would do it: the shared axis' x bit
+    // (z bit when a is the target) is not touched by the star, so it gates the
+    // whole mask, and what the star folds into the shared axis is the mask's
+    // parity. Sign flips of gamma are exact, so only their number mod 2 counts.
+    static __device__ __forceinline__ void cnot_fan(Frame<NW>& ff, uint32_t a, const uint64_t (&m)[NW]) {
+        const uint64_t gate = 0ull - (uint64_t)ff.px(a);
+        int par = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            par += __popcll(ff.z[i] & m[i]);
+            ff.x[i] ^= m[i] & gate;
+        }
+        Frame<NW>::flip(ff.z, a, par & 1);
+    }
+    static __device__ __forceinline__ void cnot_gather(Frame<NW>& ff, uint32_t a, const uint64_t (&m)[NW]) {
+        const uint64_t gate = 0ull - (uint64_t)ff.pz(a);
+        int par = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            par += __popcll(ff.x[i] & m[i]);
+            ff.z[i] ^= m[i] & gate;
+        }
+        Frame<NW>::flip(ff.x, a, par & 1);
+    }
+    static __device__ __forceinline__ void cz_fan(Frame<NW>& ff, double2& g, uint32_t a, const uint64_t (&m)[NW]) {
+        const int xa = ff.px(a);
+        const uint64_t gate = 0ull - (uint64_t)xa;
+        int par = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            par += __popcll(ff.x[i] & m[i]);
+            ff.z[i] ^= m[i] & gate;
+        }
+        if (xa & par & 1) g = make_double2(-g.x, -g.y);
+        Frame<NW>::flip(ff.z, a, par & 1);
+    }
+    // One frame opcode on (ff, g).
+    __device__ __forceinline__ void frame_step(const uint4& w, Frame<NW>& ff, double2& g) const {
+        const uint32_t op = w.x & 0xffu;
+        const uint32_t a = w.y & 0xffffu, b = w.y >> 16;
+        switch (op) {
+            case DOP_CNOT_FAN: {
+                uint64_t m[NW];
+                star_mask(w, m);
+                cnot_fan(ff, a, m);
+                break;
+            }
+            case DOP_CNOT_GATHER: {
+                uint64_t m[NW];
+                star_mask(w, m);
+                cnot_gather(ff, a, m);
+                break;
+            }
+            case DOP_CZ_FAN: {
+                uint64_t m[NW];
+                star_mask(w, m);
+                cz_fan(ff, g, a, m);
+                break;
+            }
+            case CLIFFT_OP_FRAME_CNOT: {
+                const int xa = ff.px(a);
+                Frame<NW>::flip(ff.x, b, xa);
+                Frame<NW>::flip(ff.z, a, ff.pz(b));
+                break;
+            }
+            case CLIFFT_OP_FRAME_CZ: {
+                const int xa = ff.px(a), xb = ff.px(b);
+                if (xa & xb) g = make_double2(-g.x, -g.y);
+                Frame<NW>::flip(ff.z, b, xa);
+                Frame<NW>::flip(ff.z, a, xb);
+                break;
+            }
+            case CLIFFT_OP_FRAME_H: {
+                const int xa = ff.px(a), za = ff.pz(a);
+                if (xa & za) g = make_double2(-g.x, -g.y);
+                Frame<NW>::put(ff.x, a, za);
+                Frame<NW>::put(ff.z, a, xa);
+                break;
+            }
+            case CLIFFT_OP_FRAME_S:
+            case CLIFFT_OP_FRAME_S_DAG: {
+                const int xa = ff.px(a);
+                if (xa) g = dmul(g, make_double2(0.0, op == CLIFFT_OP_FRAME_S_DAG ? -1.0 : 1.0));
+                Frame<NW>::flip(ff.z, a, xa);
+                break;
+            }
+            default: {  // FRAME_SWAP
+                const int xa = ff.px(a), xb = ff.px(b), za = ff.pz(a), zb = ff.pz(b);
+                Frame<NW>::put(ff.x, a, xb);
+                Frame<NW>::put(ff.x, b, xa);
+                Frame<NW>::put(ff.z, a, zb);
+                Frame<NW>::put(ff.z, b, za);
+                break;
+            }
+        }
+    }
+    // A run of frame opcodes executed with the frame and gamma in registers
+    // and the next instruction word fetched one step ahead. The updates and
+    // their order are those of the per-opcode handlers above. Returns the
+    // first pc at or after `pc` that is not a frame opcode.
     __device__ __forceinline__ uint32_t frame_run(uint32_t pc, uint32_t n_instr) {
         if (pc >= n_instr) return pc;
-        uint4 w = __ldg(P.instr + 2 * pc);
-        if ((w.x & 0xffu) > CLIFFT_OP_FRAME_SWAP) return pc;
+        uint4 w = __ldg(P.code + 2 * pc);
+        if (!frame_op(w.x & 0xffu)) return pc;
         Frame<NW> ff = f;
         double2 g = gamma;
         for (;;) {
-            const uint32_t op = w.x & 0xffu;
-            if (op > CLIFFT_OP_FRAME_SWAP) break;
-            const uint32_t a = w.y & 0xffffu, b = w.y >> 16;
-            const uint4 nxt = pc + 1 < n_instr ? __ldg(P.instr + 2 * (pc + 1)) : make_uint4(0xffu, 0u, 0u, 0u);
-            const int xa = ff.px(a), xb = ff.px(b);
-            switch (op) {
-                case CLIFFT_OP_FRAME_CNOT:
-                    Frame<NW>::flip(ff.x, b, xa);
-                    Frame<NW>::flip(ff.z, a, ff.pz(b));
-                    break;
-                case CLIFFT_OP_FRAME_CZ:
-                    if (xa & xb) g = make_double2(-g.x, -g.y);
-                    Frame<NW>::flip(ff.z, b, xa);
-                    Frame<NW>::flip(ff.z, a, xb);
-                    break;
-                case CLIFFT_OP_FRAME_H: {
-                    const int za = ff.pz(a);
-                    if (xa & za) g = make_double2(-g.x, -g.y);
-                    Frame<NW>::put(ff.x, a, za);
-                    Frame<NW>::put(ff.z, a, xa);
-                    break;
-                }
-                case CLIFFT_OP_FRAME_S:
-                case CLIFFT_OP_FRAME_S_DAG:
-                    if (xa) g = dmul(g, make_double2(0.0, op == CLIFFT_OP_FRAME_S_DAG ? -1.0 : 1.0));
-                    Frame<NW>::flip(ff.z, a, xa);
-                    break;
-                default: {  // FRAME_SWAP
-                    const int za = ff.pz(a), zb = ff.pz(b);
-                    Frame<NW>::put(ff.x, a, xb);
-                    Frame<NW>::put(ff.x, b, xa);
-                    Frame<NW>::put(ff.z, a, zb);
-                    Frame<NW>::put(ff.z, b, za);
-                    break;
-                }
-            }
+            if (!frame_op(w.x & 0xffu)) break;
+            const uint4 nxt = pc + 1 < n_instr ? __ldg(P.code + 2 * (pc + 1))
+                                               : make_uint4((uint32_t)CLIFFT_NUM_OPCODES, 0u, 0u, 0u);
+            frame_step(w, ff, g);
             ++pc;
             w = nxt;
             if (pc >= n_instr) break;
@@ -985,8 +1076,8 @@ struct Shot {
             Grp::sync();
         }
         account(1ull << k);
-        for (uint32_t c = 0; c < k; ++c)
-            if ((mask >> c) & 1ull) frame_cnot(c, t);
+        uint64_t m[NW] = {mask};
+        cnot_gather(f, t, m);
     }
     // exec_array_multi_cz (svm_kernels.inl:558-635)
     __device__ __forceinline__ void array_multi_cz(uint32_t c, uint64_t mask) {
@@ -1010,8 +1101,8 @@ struct Shot {
             Grp::sync();
         }
         account(1ull << k);
-        for (uint32_t t = 0; t < k; ++t)
-            if ((mask >> t) & 1ull) frame_cz(c, t);
+        uint64_t m[NW] = {mask};
+        cz_fan(f, gamma, c, m);
     }
     // exec_array_h (svm_kernels.inl:639-744): (a +- b) / sqrt(2)
     __device__ __forceinline__ void array_h(uint32_t a) {
@@ -1702,7 +1793,7 @@ struct Shot {
     // svm_kernels.inl:2183-2646; forced opcodes share the sampling handlers).
     __device__ __forceinline__ void exec(uint32_t pc) {
         cur_pc = pc;
-        const uint4* ip = P.instr;
+        const uint4* ip = P.code;
         const uint4 w0 = __ldg(ip + 2 * pc);
         uint32_t op = w0.x & 0xffu;
         const uint32_t fl = (w0.x >> 16) & 0xffu;
@@ -1712,12 +1803,15 @@ struct Shot {
         if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
             op -= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED - CLIFFT_OP_MEAS_DORMANT_STATIC;
             switch (op) {
-            case CLIFFT_OP_FRAME_CNOT: frame_cnot(a1, a2); break;
-            case CLIFFT_OP_FRAME_CZ: frame_cz(a1, a2); break;
-            case CLIFFT_OP_FRAME_H: frame_h(a1); break;
-            case CLIFFT_OP_FRAME_S: frame_s(a1, false); break;
-            case CLIFFT_OP_FRAME_S_DAG: frame_s(a1, true); break;
-            case CLIFFT_OP_FRAME_SWAP: frame_swap(a1, a2); break;
+            case CLIFFT_OP_FRAME_CNOT:
+            case CLIFFT_OP_FRAME_CZ:
+            case CLIFFT_OP_FRAME_H:
+            case CLIFFT_OP_FRAME_S:
+            case CLIFFT_OP_FRAME_S_DAG:
+            case CLIFFT_OP_FRAME_SWAP:
+            case DOP_CNOT_FAN:
+            case DOP_CNOT_GATHER:
+            case DOP_CZ_FAN: frame_step(w0, f, gamma); break;
             case CLIFFT_OP_ARRAY_CNOT: array_cnot(a1, a2); break;
             case CLIFFT_OP_ARRAY_CZ: array_cz(a1, a2); break;
             case CLIFFT_OP_ARRAY_SWAP: array_swap(a1, a2); break;
@@ -2194,7 +2288,7 @@ struct Shot {
         uint32_t term = 0;   // the terminating measurement's pc
         int term_kind = 0;   // 1 diagonal, 2 X-basis, 3 X-basis with a fused swap
         for (; end < limit; ++end) {
-            const uint4 w0 = __ldg(P.instr + 2 * end);
+            const uint4 w0 = __ldg(P.code + 2 * end);
             uint32_t op = w0.x & 0xffu;
             const uint32_t x1 = w0.y & 0xffffu, x2 = w0.y >> 16;
             if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
@@ -2208,7 +2302,10 @@ struct Shot {
                 case CLIFFT_OP_FRAME_H:
                 case CLIFFT_OP_FRAME_S:
                 case CLIFFT_OP_FRAME_S_DAG:
-                case CLIFFT_OP_FRAME_SWAP: break;
+                case CLIFFT_OP_FRAME_SWAP:
+                case DOP_CNOT_FAN:
+                case DOP_CNOT_GATHER:
+                case DOP_CZ_FAN: break;
                 case CLIFFT_OP_ARRAY_CNOT: nd = 1ull << x2; cost = 1; break;          // the target moves
                 case CLIFFT_OP_ARRAY_MULTI_CNOT: nd = 1ull << x1; cost = 1; break;    // the target moves
                 case CLIFFT_OP_ARRAY_SWAP:
@@ -2303,7 +2400,7 @@ struct Shot {
         bool red_local = false;
         uint32_t red_bit = 0;
         if (term_kind) {
-            const uint4 w0 = __ldg(P.instr + 2 * term);
+            const uint4 w0 = __ldg(P.code + 2 * term);
             cur_pc = term;
             tfa = w0.y & 0xffffu;
             tt = term_kind == 3 ? (w0.y >> 16) : tfa;
@@ -2995,7 +3092,7 @@ struct Shot {
     // Whether instruction pc touches the statevector (needs every thread of a
     // CTA group) or only scalar state (frame, gamma, records, noise cursor).
     __device__ __forceinline__ bool needs_all(uint32_t pc) const {
-        const uint4 w0 = __ldg(P.instr + 2 * pc);
+        const uint4 w0 = __ldg(P.code + 2 * pc);
         uint32_t op = w0.x & 0xffu;
         const uint32_t a1 = w0.y & 0xffffu;
         if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
@@ -3082,7 +3179,7 @@ struct Shot {
     // a statevector step executed by every thread (fused block or one opcode)
     __device__ __forceinline__ uint32_t run_all(uint32_t pc, bool fuse_on) {
         uint32_t used = 0;
-        if (tiled(k)) used = run_block(pc, fuse_on ? TC::kMops : 1, P.n_instr);
+        if (tiled(k)) used = run_block(pc, fuse_on ? TC::kMops : 1, P.n_code);
         if (!used) {
             exec(pc);
             used = 1;
@@ -3093,7 +3190,7 @@ struct Shot {
     // for statevector steps, receiving the scalar state through shared memory.
     // Every CTA-wide barrier is reached by all warps at the same program point.
     __device__ void run_cta(bool fuse_on, bool prof) {
-        const uint32_t n_instr = P.n_instr;
+        const uint32_t n_instr = P.n_code;
         const bool ctrl = (threadIdx.x >> 5) == 0;
         uint32_t pc = 0;
         for (;;) {
@@ -3123,7 +3220,7 @@ struct Shot {
             const uint32_t used = run_all(word, fuse_on);
             __syncthreads();
             if (prof) {
-                const uint32_t op = __ldg(P.instr + 2 * word).x & 0xffu;
+                const uint32_t op = __ldg(P.code + 2 * word).x & 0xffu;
                 int cat = used > 1 ? 0 : 3;
                 if ((op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE) ||
                     (op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED))
@@ -3144,7 +3241,7 @@ struct Shot {
         } else {
             reset();
         }
-        const uint32_t n_instr = P.n_instr;
+        const uint32_t n_instr = P.n_code;
         const bool fuse_on = Grp::kCta && (K.flags & KF_FUSE) != 0;
         const bool prof = K.phase_cycles != nullptr && Grp::rank() == 0;
         if (Grp::kCta) {
