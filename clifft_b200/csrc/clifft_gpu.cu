@@ -242,6 +242,27 @@ struct CodeStream {
     std::vector<uint64_t> masks;   // frames wider than one word: nwt words per condensed instruction
 };
 
+// Opcodes that touch the statevector, counted by the active rank before them
+// (a validated program: ranks follow from the opcodes alone).
+std::vector<uint32_t> ops_by_rank(const clifft_program_image& im) {
+    std::vector<uint32_t> n(im.peak_rank + 1, 0);
+    uint32_t k = 0;
+    for (uint32_t i = 0; i < im.num_instructions; ++i) {
+        const uint8_t* I = im.instructions + size_t(i) * 32;
+        uint32_t op = I[0];
+        if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
+            op -= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED - CLIFFT_OP_MEAS_DORMANT_STATIC;
+        if ((op >= CLIFFT_OP_ARRAY_CNOT && op <= CLIFFT_OP_EXPAND_ROT) ||
+            (op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE) || op == CLIFFT_OP_EXP_VAL)
+            n[k]++;
+        if (op >= CLIFFT_OP_EXPAND && op <= CLIFFT_OP_EXPAND_ROT)
+            ++k;
+        else if (op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE)
+            --k;
+    }
+    return n;
+}
+
 CodeStream condense(const clifft_program_image& im, uint32_t nwt) {
     constexpr uint32_t kMinStar = 2;
     CodeStream c;
@@ -351,6 +372,7 @@ struct clifft_gpu_program {
     std::vector<uint8_t> instr_host;  // the 32-byte instructions (host copy, for gradient programs)
     std::vector<uint8_t> code_host;     // the device instruction stream
     std::vector<uint32_t> code_origin;  // image instruction of each of its instructions
+    std::vector<uint32_t> ops_at_k;     // opcodes on the statevector, by the active rank before them
     uint32_t num_rot_params = 0;      // ARRAY_ROT + EXPAND_ROT instructions
     std::vector<double> fault_probs;  // per noise site its total probability, then per readout entry its flip
                                       // probability (clifft::noise_site_probabilities order)
@@ -488,7 +510,14 @@ struct LaunchPlan {
     bool fuse;        // ... and consecutive opcodes fuse into one pass
     uint32_t stages;  // tile buffers per CTA (2 / 3 let three 128-thread / two 256-thread CTAs share an SM)
     bool dense;       // the kernel instance with tensor-core dense blocks (FP32, CTA groups, three stages)
+    uint32_t team;    // CTAs per shot (0: a CTA or less per shot)
+    // statevectors resident at once
+    uint64_t resident() const { return team ? uint64_t(blocks) / team : uint64_t(blocks) * regions * S; }
 };
+
+// Group requests inside the library: the public group_threads values, or a
+// team of CTAs per shot.
+constexpr uint32_t team_request(uint32_t ctas) { return ctas << 16; }
 
 uint32_t nw_template(uint32_t nw) { return nw <= 1 ? 1 : 4; }
 
@@ -541,8 +570,11 @@ PlanShape plan_shape(const clifft_gpu_program& p, uint32_t precision, uint32_t g
     const size_t rec_bytes1 = size_t(rec_words + det_words + obs_words) * 4;
 
     // group_req: 0 = heuristic; 1..32 = lanes per shot; 64..1024 = CTA of that size
+    const bool team = group_req >> 16;
     int G;
-    if (group_req >= 1 && group_req <= 32)
+    if (team)
+        G = 0;
+    else if (group_req >= 1 && group_req <= 32)
         G = int(group_req);
     else if (group_req > 32)
         G = 0;
@@ -592,13 +624,14 @@ PlanShape plan_shape(const clifft_gpu_program& p, uint32_t precision, uint32_t g
         // SM) up to 8 MiB statevectors, else two CTAs with three buffers each:
         // 256 compute threads plus a copy warp when blocks fuse (k = 24: 98 vs
         // 107 ms), 256 threads without fusion
-        int t = group_req > 32 ? int(group_req)
-                               : (state_bytes <= (size_t(8) << 20) ? 128 : (allow_fusion ? int(kWsThreadsHalf) : 256));
-        if (ws_shape(uint32_t(t))) max_threads = pick_fn(-1);
+        int t = team            ? int(kWsThreadsHalf)
+                : group_req > 32 ? int(group_req)
+                                 : (state_bytes <= (size_t(8) << 20) ? 128 : (allow_fusion ? int(kWsThreadsHalf) : 256));
+        if (ws_shape(uint32_t(t))) max_threads = pick_fn(team ? -2 : -1);
         L.threads = std::min(t, max_threads);
         L.regions = 1;
         L.stages = L.threads <= 128 ? 2 : (L.threads <= 256 || L.threads == int(kWsThreadsHalf) ? 3 : 4);
-        L.state_in_smem = region_bytes(true) + tail(L.threads) <= smem_cap;
+        L.state_in_smem = !team && region_bytes(true) + tail(L.threads) <= smem_cap;
     }
     L.tiles = (G == 0 || G == 32) && !L.state_in_smem;
     if (!L.tiles) L.stages = 0;
@@ -622,6 +655,7 @@ PlanShape plan_shape(const clifft_gpu_program& p, uint32_t precision, uint32_t g
     }
     int per_sm = 0;
     CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)L.fn, L.threads, L.smem));
+    L.team = group_req >> 16;
     if (per_sm < 1) invalid("kernel does not fit on an SM with this launch shape");
     L.state_stride = stride;
     return PlanShape{L, per_sm, sms};
@@ -693,6 +727,17 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
     const uint64_t shots_per_block = uint64_t(L.regions) * L.S;
     const uint64_t blocks_needed = (shots + shots_per_block - 1) / shots_per_block;
     uint64_t blocks = uint64_t(per_sm) * sms;
+    if (L.team) {
+        // whole teams only, and never more CTAs than fit on the GPU together
+        size_t free_b = 0, total_b = 0;
+        CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
+        L.team = uint32_t(std::min<uint64_t>(L.team, blocks));
+        uint64_t teams = std::min<uint64_t>(blocks / L.team, (free_b / 2) / state_bytes);
+        if (max_resident) teams = std::min<uint64_t>(teams, max_resident);
+        teams = std::max<uint64_t>(1, std::min<uint64_t>(teams, shots));
+        L.blocks = int(teams * L.team);
+        return L;
+    }
     if (!L.state_in_smem) {
         // global slabs: bound the resident state to ~half of free HBM
         size_t free_b = 0, total_b = 0;
@@ -705,6 +750,73 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
     blocks = std::max<uint64_t>(1, std::min<uint64_t>(blocks, blocks_needed));
     L.blocks = int(blocks);
     return L;
+}
+
+// Team size for an untuned launch of `shots` shots (as a group request), or 0
+// for the one-CTA or one-warp shapes. Statevectors above 1 MiB only: below,
+// a warp per shot keeps more of the GPU busy and a team's CTAs have a handful
+// of tiles each. A launch of C CTAs per shot runs ceil(shots / teams) rounds,
+// each of which costs about
+//     kOpUs x (opcodes on the statevector) + kTileUs x (tiles they cover) / C:
+// every CTA of a team interprets the whole program, so the first part does
+// not shrink with C. Measured (B200, two CTAs per SM; the last third is what a
+// CTA gains from having its SM to itself): k = 24 FP32, 147 opcodes, 117216
+// tiles: 98 ms / C + 1.9 ms; k = 20 FP32, 394 opcodes, 75336 tiles: 110 ms / C
+// + 3.0 ms; k = 18 FP64, 73 opcodes, 2670 tiles: 2.5 ms / C + 1.2 ms. One shot
+// of the k = 24 program takes 2.1 ms with 148 CTAs, 64 ms with one; 148 shots
+// 50 ms with teams of two, 66 ms with one CTA each.
+uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_t shots, uint32_t max_resident) {
+    constexpr double kOpUs = 7.0, kTileUs = 1.0, kAlone = 0.66;
+    constexpr uint32_t kPerSm = 2;
+    const bool fp64 = precision == CLIFFT_GPU_FP64;
+    const size_t state_bytes = (size_t(1) << p.meta.peak_rank) * (fp64 ? 16 : 8);
+    if (state_bytes <= (size_t(1) << 20)) return 0;
+    int dev = 0, sms = 0, coop = 0;
+    size_t free_b = 0, total_b = 0;
+    CUDA_OK(cudaGetDevice(&dev));
+    CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CUDA_OK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
+    if (!coop) return 0;
+    const uint32_t bits = fp64 ? TileCfg<double, true>::kBits : TileCfg<float, true>::kBits;
+    double ops = 0.0, tiles = 0.0;
+    for (uint32_t k = 0; k < p.ops_at_k.size(); ++k) {
+        ops += p.ops_at_k[k];
+        if (k > bits) tiles += double(p.ops_at_k[k]) * double(uint64_t(1) << (k - bits));
+    }
+    const uint64_t cap = uint64_t(kPerSm) * sms;
+    uint64_t most = std::max<uint64_t>(1, std::min<uint64_t>(shots, (free_b / 2) / state_bytes));
+    if (max_resident) most = std::min<uint64_t>(most, max_resident);
+    double best = 0.0;
+    uint32_t ctas = 0;
+    // every split of the GPU into equal teams, finest first: a coarser one has to be better
+    for (uint64_t c = 1; c <= uint64_t(sms); c = c < 8 ? c + 1 : c + c / 4) {
+        const uint64_t teams = std::min<uint64_t>(cap / c, most);
+        const double rounds = double((shots + teams - 1) / teams);
+        const double share = tiles / double(c) * (teams * c <= uint64_t(sms) ? kAlone : 1.0);
+        const double t = rounds * (kOpUs * ops + kTileUs * share);
+        if (!ctas || t < best) {
+            best = t;
+            ctas = uint32_t(c);
+        }
+    }
+    return team_request(ctas);
+}
+
+// One launch of a plan. The CTAs of a team wait for one another, so a team
+// launch is cooperative: it starts only when all its CTAs fit on the GPU.
+void launch_plan(const LaunchPlan& L, const DevProg& prog, const KParams& K, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(L.blocks));
+    cfg.blockDim = dim3(unsigned(L.threads));
+    cfg.dynamicSmemBytes = L.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = L.team ? 1 : 0;
+    CUDA_OK(cudaLaunchKernelEx(&cfg, L.fn, prog, K));
 }
 
 // Launch shapes the autotuner tries (group_threads encoding): sub-warp groups
@@ -957,6 +1069,7 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
         d.code = at<uint4>(B, o_code);
         d.n_code = uint32_t(code.origin.size());
         d.fmask = at<uint64_t>(B, o_mask);
+        p->ops_at_k = ops_by_rank(im);
         p->code_host = std::move(code.bytes);
         p->code_origin = std::move(code.origin);
         d.nw = nwt;
@@ -1128,6 +1241,10 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
                 tune = tune_candidates(*prog, args->precision);
             }
         }
+        // an untuned automatic shape whose statevectors are large: a team of
+        // CTAs per shot when that is the better split of the GPU
+        if (group_req == 0 && tune.empty() && allow_fusion && !(args->flags & CLIFFT_GPU_TENSOR_DENSE))
+            group_req = team_heuristic(*prog, args->precision, shots, args->max_resident);
         const bool want_dense = (args->flags & CLIFFT_GPU_TENSOR_DENSE) && args->precision == CLIFFT_GPU_FP32;
         LaunchPlan L = plan_launch(*prog, args->precision, group_req, shots, rec_words, det_words, obs_words,
                                    allow_fusion, args->max_resident, want_dense);
@@ -1162,7 +1279,15 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             Kx.state_stride = Lx.state_stride;
             Kx.state_global = Lx.state_in_smem
                                   ? nullptr
-                                  : slab.get(size_t(Lx.blocks) * Lx.regions * Lx.S * Lx.state_stride * amp);
+                                  : slab.get(size_t(Lx.resident()) * Lx.state_stride * amp);
+            if (Lx.team) {
+                Kx.team_size = Lx.team;
+                const uint64_t teams = Lx.resident();
+                Kx.team_sums = static_cast<double*>(buf.alloc(size_t(Lx.blocks) * 8 * sizeof(double)));
+                // one 128-byte line per team's arrival counter
+                Kx.team_arrivals = static_cast<uint32_t*>(buf.alloc(size_t(teams) * 128));
+                CUDA_OK(cudaMemsetAsync(Kx.team_arrivals, 0, size_t(teams) * 128, st));
+            }
             Kx.dense_min_weight = dense_min_weight();
         };
         const size_t n_counters = 5 + m.num_observables;
@@ -1268,8 +1393,7 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
                 Kc.phase_cycles = nullptr;
                 Kc.error_info = sc + scratch_words - 8;
                 CUDA_OK(cudaEventRecord(e0, st));
-                Lc.fn<<<Lc.blocks, Lc.threads, Lc.smem, st>>>(prog->dev, Kc);
-                CUDA_OK(cudaGetLastError());
+                launch_plan(Lc, prog->dev, Kc, st);
                 CUDA_OK(cudaEventRecord(e1, st));
                 CUDA_OK(cudaEventSynchronize(e1));
                 ++launches;
@@ -1317,8 +1441,7 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
         }
         CUDA_OK(cudaEventRecord(e0, st));
         if (!nseg) {
-            L.fn<<<L.blocks, L.threads, L.smem, st>>>(prog->dev, K);
-            CUDA_OK(cudaGetLastError());
+            launch_plan(L, prog->dev, K, st);
         } else {
             for (uint32_t sgi = 0; sgi < nseg; ++sgi) {
                 KParams Ks = K;

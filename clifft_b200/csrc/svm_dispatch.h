@@ -9,7 +9,8 @@ using KernelFn = void (*)(const DevProg, const KParams);
 
 // Every kernel instance: X(name, statevector type, G, NW, dense).
 // G = lanes per shot (1, 2, 4, 8, 16, 32), 0 for one CTA per shot, -1 for
-// one CTA per shot whose last warp moves the fused blocks' tiles; NW = frame
+// one CTA per shot whose last warp moves the fused blocks' tiles, -2 for a
+// team of such CTAs per shot; NW = frame
 // words (1, or 2..4 served by the 4-word kernel); dense: with the tensor-core
 // dense blocks. The build reads this list (one translation unit per row).
 #define CGPU_INSTANCES(X)            \
@@ -45,6 +46,10 @@ using KernelFn = void (*)(const DevProg, const KParams);
     X(f64_g32_n4, double, 32, 4, 0)  \
     X(f64_cta_n4, double, 0, 4, 0)   \
     X(f64_ws_n4, double, -1, 4, 0)   \
+    X(f32_team_n1, float, -2, 1, 0)  \
+    X(f32_team_n4, float, -2, 4, 0)  \
+    X(f64_team_n1, double, -2, 1, 0) \
+    X(f64_team_n4, double, -2, 4, 0) \
     X(f32_cta_n1_dense, float, 0, 1, 1) \
     X(f32_cta_n4_dense, float, 0, 4, 1) \
     X(f32_ws_n1_dense, float, -1, 1, 1) \

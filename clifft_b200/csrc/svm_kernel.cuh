@@ -131,6 +131,11 @@ struct KParams {
     uint64_t dump_shots;
     uint32_t fuse_bytes;  // shared bytes per CTA reserved for fused tile sweeps (0 = off)
     uint32_t stages;      // tile buffers per CTA (2..kMaxStages) when fuse_bytes != 0
+    // teams (G = -2): CTAs per shot, one arrival counter per team, and per team
+    // two sets (used in turn) of four partial sums per CTA
+    uint32_t team_size;
+    uint32_t* team_arrivals;
+    double* team_sums;
     uint32_t dense_min_weight;  // KF_DENSE: least CUDA-core weight of a run worth a GEMM (U4 4, U2 2, others 1)
     unsigned long long* phase_cycles;  // optional: SM cycles per executor phase (thread 0 of each group)
     // segmented execution (survivor runs of warp groups): this launch runs
@@ -305,6 +310,7 @@ template <int G>
 struct Lanes {
     static constexpr bool kCta = false;
     static constexpr bool kWS = false;
+    static constexpr bool kTeam = false;
     static constexpr int S = 32 / G;
     __device__ static __forceinline__ int size() { return G; }
     __device__ static __forceinline__ int rank() { return (int)(threadIdx.x & 31) & (G - 1); }
@@ -320,6 +326,7 @@ struct Lanes {
 struct CtaLanes {
     static constexpr bool kCta = true;
     static constexpr bool kWS = false;
+    static constexpr bool kTeam = false;
     static constexpr int S = 1;
     __device__ static __forceinline__ int size() { return blockDim.x; }
     __device__ static __forceinline__ int rank() { return threadIdx.x; }
@@ -343,6 +350,15 @@ struct CtaLanesWS : CtaLanes {
 template <>
 struct GroupOf<-1> {
     using type = CtaLanesWS;
+};
+// Several such CTAs per shot (a team): every CTA interprets the whole program
+// and the passes over the statevector are split between them.
+struct CtaLanesTeam : CtaLanesWS {
+    static constexpr bool kTeam = true;
+};
+template <>
+struct GroupOf<-2> {
+    using type = CtaLanesTeam;
 };
 
 __device__ __forceinline__ uint64_t ins0(uint64_t v, uint32_t pos) {
@@ -670,6 +686,15 @@ struct CtlState {
 };
 constexpr uint32_t kCtlBytes = 512;
 
+// What a CTA of a team keeps across shots (every thread holds the same).
+struct TeamLink {
+    uint32_t rank = 0;      // this CTA within its team
+    uint32_t size = 1;
+    uint32_t arrivals = 0;  // team barriers passed so far
+    uint32_t* counter = nullptr;
+    double* sums = nullptr;
+};
+
 // --------------------------------------------------------------- the shot
 template <typename R, class Grp, int NW, bool DENSE = false>
 struct Shot {
@@ -717,10 +742,159 @@ struct Shot {
     // contiguous run.
     uint64_t xo;
     uint64_t tileF;  // tile axes of the fused block being resolved
+    // teams: while k <= kBits every CTA holds the whole state in its first
+    // tile buffer (idle then) and computes it for itself; above, v is the
+    // team's global statevector and passes are split between the CTAs
+    TeamLink* team;
+    T* team_v;   // the team's global statevector
+    bool priv;
 
     __device__ __forceinline__ Shot(const DevProg& p, const KParams& kp, T* vv, uint32_t* r, uint32_t* d,
                                     uint32_t* o, double* rd, unsigned char* fz, uint32_t* bp, uint64_t s)
         : P(p), K(kp), v(vv), rec(r), det(d), obs(o), red(rd), shot(s), fuse(fz), bar_phase(bp) {}
+
+    // ------------------------------------------------------------- teams
+    // Threads that share a sweep over the current state, and their barrier.
+    __device__ __forceinline__ bool split() const { return Grp::kTeam && !priv; }
+    __device__ __forceinline__ uint32_t wrank() const {
+        if constexpr (Grp::kTeam)
+            return split() ? team->rank * blockDim.x + threadIdx.x : threadIdx.x;
+        else
+            return Grp::rank();
+    }
+    __device__ __forceinline__ uint32_t wsize() const {
+        if constexpr (Grp::kTeam)
+            return split() ? team->size * blockDim.x : blockDim.x;
+        else
+            return Grp::size();
+    }
+    __device__ __forceinline__ void wsync() {
+        if constexpr (Grp::kTeam) {
+            if (split()) {
+                team_sync();
+                return;
+            }
+        }
+        Grp::sync();
+    }
+    // the CTA that writes a shot's outputs
+    __device__ __forceinline__ bool leader() const {
+        if constexpr (Grp::kTeam)
+            return team->rank == 0;
+        else
+            return true;
+    }
+    // Barrier over the CTAs of a team. They are resident together (the launch
+    // is cooperative), and the arrival counter only grows: barrier n is open
+    // once it holds n x size. What any thread of the team wrote before it,
+    // through either proxy, is visible to every thread and bulk copy after it.
+    // The wait is bounded; a CTA that gives up records a device error and
+    // arrives nowhere again, and the others see that error and give up too.
+    __device__ void team_sync() {
+        if constexpr (Grp::kTeam) {
+            fence_async_global();
+            __syncthreads();
+            bool ok = true;
+            if (threadIdx.x == 0) {
+                ok = !(*bar_phase >> 31);
+                if (ok) {
+                    const uint32_t want = (team->arrivals + 1) * team->size;
+                    __threadfence();
+                    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(team->counter) : "memory");
+                    uint32_t seen = 0, polls = 0;
+                    for (;; ++polls) {
+                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(team->counter) : "memory");
+                        if ((int32_t)(seen - want) >= 0) break;
+                        if (polls >= (1u << 23) ||
+                            ((polls & 1023u) == 1023u && *(volatile int*)K.error_word == DEV_ERR_TIMEOUT)) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                    __threadfence();
+                }
+                if (!ok && atomicCAS(K.error_word, 0, DEV_ERR_TIMEOUT) == 0 && K.error_info) {
+                    K.error_info[0] = 9;
+                    K.error_info[1] = cur_pc;
+                    K.error_info[5] = k;
+                    K.error_info[6] = 4000 + team->rank;
+                }
+            }
+            if (__syncthreads_or(!ok)) {
+                *bar_phase |= 1u << 31;
+                stop = true;
+            }
+            team->arrivals++;
+            fence_async_global();
+        }
+    }
+    // Sums over every thread that shares the current state, the same bits in
+    // every thread: per CTA as before, then the CTAs' partial sums in a fixed
+    // order. The two sets of partial sums are used in turn: a CTA writes set
+    // n + 2 only after barrier n + 1, which every reader of set n has reached.
+    template <int N>
+    __device__ __forceinline__ void state_reduce(double (&x)[N]) {
+        group_reduce<Grp, N>(x, red);
+        if constexpr (Grp::kTeam) {
+            if (!split()) return;
+            double* set = team->sums + (size_t)(team->arrivals & 1u) * team->size * 4;
+            if (threadIdx.x == 0)
+#pragma unroll
+                for (int j = 0; j < N; ++j) __stcg(set + team->rank * 4 + j, x[j]);
+            team_sync();
+            if (threadIdx.x < 32) {
+#pragma unroll
+                for (int j = 0; j < N; ++j) x[j] = 0.0;
+                for (uint32_t c = threadIdx.x; c < team->size; c += 32)
+#pragma unroll
+                    for (int j = 0; j < N; ++j) x[j] += __ldcg(set + c * 4 + j);
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                    for (int j = 0; j < N; ++j) x[j] += __shfl_down_sync(0xffffffffu, x[j], off);
+                if (threadIdx.x == 0)
+#pragma unroll
+                    for (int j = 0; j < N; ++j) red[j] = x[j];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < N; ++j) x[j] = red[j];
+            __syncthreads();
+        }
+    }
+    // k <= kBits again: every CTA takes its own copy of the state. The next
+    // write to the team's statevector comes after a team barrier
+    // (leave_private), so no CTA can still be reading it then.
+    __device__ __forceinline__ void enter_private() {
+        if constexpr (Grp::kTeam) {
+            if (priv || k > (uint32_t)TC::kBits) return;
+            T* own = reinterpret_cast<T*>(fuse + TC::kBufOffset);
+            for (uint32_t i = threadIdx.x; i < (1u << k); i += blockDim.x) own[i] = v[i ^ xo];
+            v = own;
+            xo = 0;
+            priv = true;
+            __syncthreads();
+        }
+    }
+    // An expansion at k = kBits: the 2^(k+1) amplitudes go to the team's
+    // statevector, split between the CTAs.
+    __device__ __forceinline__ void leave_private(bool with_phase, T ph) {
+        if constexpr (Grp::kTeam) {
+            const T* own = v;
+            const uint32_t half = 1u << k;
+            team_sync();
+            v = team_v;
+            xo = 0;
+            priv = false;
+            for (uint32_t i = wrank(); i < half; i += wsize()) {
+                const T x = own[i];
+                v[i] = x;
+                v[half + i] = with_phase ? cmul(x, ph) : x;
+            }
+            fence_async_shared();  // the buffer is a target of bulk loads from here on
+            team_sync();
+        }
+    }
 
     __device__ __forceinline__ T& A(uint64_t i) { return v[(kTiles ? (i ^ xo) : i) * S]; }
     // algorithmic bytes of an opcode (per-opcode definition); streamed bytes
@@ -747,7 +921,7 @@ struct Shot {
             uint32_t m = 1u << (idx & 31);
             uint32_t& w = rec[(idx >> 5) * S];
             w = bit ? (w | m) : (w & ~m);
-            if (meas_prob) meas_prob[idx] = prob;
+            if (meas_prob && leader()) meas_prob[idx] = prob;
         }
         rec_dirty = true;
     }
@@ -769,8 +943,8 @@ struct Shot {
                 emit(M_SCALE, 0, 0, 0, 0, 0, c, 1);
                 bytes += 2 * n * sizeof(T);
             } else {
-                for (uint64_t i = Grp::rank(); i < n; i += Grp::size()) A(i) = cscale(A(i), (R)g);
-                Grp::sync();
+                for (uint64_t i = wrank(); i < n; i += wsize()) A(i) = cscale(A(i), (R)g);
+                wsync();
                 account(2 * n);
             }
             gamma.x /= g;
@@ -948,8 +1122,8 @@ struct Shot {
 
     template <class V, int UU = U, class Ld, class St>
     __device__ __forceinline__ void sweep(uint64_t n, Ld ld, St st) {
-        const uint64_t step = (uint64_t)Grp::size();
-        for (uint64_t i0 = Grp::rank(); i0 < n; i0 += step * UU) {
+        const uint64_t step = (uint64_t)wsize();
+        for (uint64_t i0 = wrank(); i0 < n; i0 += step * UU) {
             V val[UU];
 #pragma unroll
             for (int u = 0; u < UU; ++u)
@@ -1192,6 +1366,16 @@ struct Shot {
             if (with_phase && x) phase(make_double2(zr, zi));
             return;
         }
+        if constexpr (Grp::kTeam) {
+            if (k == (uint32_t)TC::kBits) {
+                leave_private(with_phase, ph);
+                account(2ull << k);
+                k++;
+                scale_magnitude(CGPU_EXPAND_SCALE);
+                if (with_phase && x) phase(make_double2(zr, zi));
+                return;
+            }
+        }
         if (tiled(k)) {
             if constexpr (kTiles) {
                 constexpr uint32_t MB = TC::kBits, TN = 1u << MB;
@@ -1204,6 +1388,7 @@ struct Shot {
                         for (uint32_t l = tid; l < TN; l += nthr) buf[l] = cmul(buf[l], ph);
                     Grp::sync();
                 });
+                if constexpr (Grp::kTeam) team_sync();
                 moved += (2ull << k) * sizeof(T);
                 bytes += (2ull << k) * sizeof(T);
                 k++;
@@ -1756,8 +1941,8 @@ struct Shot {
             if (fsign) iph = make_double2(-iph.x, -iph.y);
             double acc[3] = {0.0, 0.0, 0.0};
             const uint64_t dim = 1ull << k;
-            const uint64_t step = (uint64_t)Grp::size();
-            for (uint64_t j0 = Grp::rank(); j0 < dim; j0 += step * U) {
+            const uint64_t step = (uint64_t)wsize();
+            for (uint64_t j0 = wrank(); j0 < dim; j0 += step * U) {
                 T av[U], bv[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u)
@@ -1780,13 +1965,13 @@ struct Shot {
                     }
                 }
             }
-            group_reduce<Grp, 3>(acc, red);
+            state_reduce<3>(acc);
             account(1ull << k);
             double2 num = dmul(make_double2(acc[0], acc[1]), iph);
             if (acc[2] > 0.0) result = num.x / acc[2];
             result = fmin(1.0, fmax(-1.0, result));
         }
-        if (Grp::rank() == 0 && K.out_exp) K.out_exp[shot * P.num_exp + out_idx] = result;
+        if (Grp::rank() == 0 && leader() && K.out_exp) K.out_exp[shot * P.num_exp + out_idx] = result;
     }
 
     // Executes instruction `pc` (the dispatch of execute_internal,
@@ -1933,12 +2118,26 @@ struct Shot {
     // barrier timeout.
     uint32_t cur_pc = 0;   // instruction being executed (diagnostics)
     uint32_t cur_site = 0; // which statevector pass is streaming (diagnostics)
+    // The tiles of a pass that this CTA streams: all of them, or its share of
+    // a team's; `first` is the first one and `base` = pdep(first, C).
+    __device__ __forceinline__ uint64_t my_tiles(uint64_t ntiles, uint64_t C, uint64_t& first, uint64_t& base) const {
+        first = 0;
+        base = 0;
+        if constexpr (Grp::kTeam) {
+            first = ntiles * team->rank / team->size;
+            base = pdep(first, C);
+            return ntiles * (team->rank + 1) / team->size - first;
+        }
+        return ntiles;
+    }
     template <class Compute>
-    __device__ bool stream_tiles(uint64_t ntiles, uint64_t C, uint32_t r, uint64_t load_add, uint64_t store_add,
+    __device__ bool stream_tiles(uint64_t pass_tiles, uint64_t C, uint32_t r, uint64_t load_add, uint64_t store_add,
                                  uint32_t store_runs, uint32_t skip, Compute compute) {
         if constexpr (!Grp::kCta) {
-            return stream_tiles_warp(ntiles, C, r, load_add, store_add, store_runs, skip, compute);
+            return stream_tiles_warp(pass_tiles, C, r, load_add, store_add, store_runs, skip, compute);
         }
+        uint64_t first, base0;
+        const uint64_t ntiles = my_tiles(pass_tiles, C, first, base0);
         constexpr uint32_t MB = TC::kBits;
         constexpr uint32_t TN = 1u << MB;
         T* bufs = reinterpret_cast<T*>(fuse + TC::kBufOffset);
@@ -1967,7 +2166,7 @@ struct Shot {
         // few hundred instructions at 4 KiB, so no division or bit-deposit
         // loop per tile): pdep(t + 1, C) = ((pdep(t, C) | ~C) + 1) & C.
         auto next_base = [C](uint64_t b) { return ((b | ~C) + 1) & C; };
-        uint64_t issue_base = 0;  // pdep(next tile to load, C)
+        uint64_t issue_base = base0;  // pdep(next tile to load, C)
         uint32_t issue_st = 0;    // its stage
         auto issue_next = [&]() {
             if (lane == 0) mbar_expect_tx(&bars[issue_st], load_bytes);
@@ -1986,7 +2185,7 @@ struct Shot {
         long long waited = 0;
         uint64_t t = 0;
         uint32_t st = 0;      // stage of tile t
-        uint64_t tbase = 0;   // pdep(t, C)
+        uint64_t tbase = base0;   // pdep(first + t, C)
         for (; t < ntiles; ++t, tbase = next_base(tbase), st = st + 1 == nst ? 0 : st + 1) {
             const uint32_t parity = (phase >> st) & 1u;
             uint32_t ok = 0;
@@ -2008,7 +2207,7 @@ struct Shot {
                 issue_next();  // tile t + nst - 1
             }
             T* buf = bufs + st * TN;
-            compute(buf, t, tbase);
+            compute(buf, first + t, tbase);
             if (store_runs) {
                 const uint64_t base = store_add + tbase;
                 if constexpr (Grp::kCta) {
@@ -2077,8 +2276,10 @@ struct Shot {
     // mapped to it, so every thread advances its copy of the phase bits the
     // same way.
     template <class Compute>
-    __device__ bool stream_tiles_ws(uint64_t ntiles, uint64_t C, uint32_t r, uint32_t store_runs, uint32_t skip,
+    __device__ bool stream_tiles_ws(uint64_t pass_tiles, uint64_t C, uint32_t r, uint32_t store_runs, uint32_t skip,
                                     Compute compute) {
+        uint64_t first, base0;
+        const uint64_t ntiles = my_tiles(pass_tiles, C, first, base0);
         constexpr uint32_t MB = TC::kBits;
         constexpr uint32_t TN = 1u << MB;
         T* bufs = reinterpret_cast<T*>(fuse + TC::kBufOffset);
@@ -2107,7 +2308,7 @@ struct Shot {
         uint32_t loads[kMaxStages] = {0, 0, 0, 0};  // loads issued per stage (copy warp)
         long long waited = 0;
         if (copier) {
-            uint64_t lbase = 0, lt = 0;
+            uint64_t lbase = base0, lt = 0;
             auto load = [&](uint32_t st) {
                 if (lane == 0) mbar_expect_tx(&full[st], load_bytes);
                 __syncwarp();
@@ -2119,7 +2320,7 @@ struct Shot {
                 ++lt;
             };
             for (uint32_t st = 0; st < nst && lt < ntiles; ++st) load(st);
-            uint64_t sbase = 0;
+            uint64_t sbase = base0;
             uint32_t st = 0;
             for (; t < ntiles; ++t, st = st + 1 == nst ? 0 : st + 1) {
                 const uint32_t parity = (phase >> (8 + st)) & 1u;
@@ -2147,7 +2348,7 @@ struct Shot {
             bulk_wait_all();
             fence_async_global();
         } else {
-            uint64_t tbase = 0;
+            uint64_t tbase = base0;
             uint32_t st = 0;
             for (; t < ntiles; ++t, tbase = next_base(tbase), st = st + 1 == nst ? 0 : st + 1) {
                 const uint32_t parity = (phase >> st) & 1u;
@@ -2160,7 +2361,7 @@ struct Shot {
                     break;
                 }
                 phase ^= 1u << st;
-                compute(bufs + st * TN, t, tbase);  // ends with a compute-warp barrier
+                compute(bufs + st * TN, first + t, tbase);  // ends with a compute-warp barrier
                 // the tile's writes before the copy warp's bulk store reads them
                 fence_async_shared();
                 bar_sync_first(ncomp);
@@ -2520,8 +2721,11 @@ struct Shot {
         else
             stream_tiles(1ull << (kk - MB), C, r, 0, 0, nm ? nruns : 0, skip, body);
         moved += (((1ull << kk) >> __popcll(fresh)) + (nm ? (1ull << kk) : 0ull)) * sizeof(T);
+        if constexpr (Grp::kTeam) {
+            if (!term_kind) team_sync();
+        }
         if (term_kind) {
-            group_reduce<Grp, 2>(acc, red);
+            state_reduce<2>(acc);
             if (!stop) {
                 if (term_kind == 1) {
                     bytes += (1ull << k) * sizeof(T);
@@ -3218,6 +3422,7 @@ struct Shot {
             if (word >> 31) break;
             const long long c1 = prof ? clock64() : 0;
             const uint32_t used = run_all(word, fuse_on);
+            enter_private();
             __syncthreads();
             if (prof) {
                 const uint32_t op = __ldg(P.code + 2 * word).x & 0xffu;
@@ -3243,7 +3448,7 @@ struct Shot {
         }
         const uint32_t n_instr = P.n_code;
         const bool fuse_on = Grp::kCta && (K.flags & KF_FUSE) != 0;
-        const bool prof = K.phase_cycles != nullptr && Grp::rank() == 0;
+        const bool prof = K.phase_cycles != nullptr && Grp::rank() == 0 && leader();
         if (Grp::kCta) {
             run_cta(fuse_on, prof);
         } else {
@@ -3365,6 +3570,10 @@ struct Shot {
         // value; every other amplitude is written by EXPAND before it is read.
         xo = 0;
         tileF = 0;
+        if constexpr (Grp::kTeam) {
+            v = reinterpret_cast<T*>(fuse + TC::kBufOffset);
+            priv = true;
+        }
         f.clear();
         gamma = make_double2(1.0, 0.0);
         k = 0;
@@ -3385,7 +3594,7 @@ struct Shot {
         for (uint32_t i = Grp::rank(); i < K.rec_words; i += Grp::size()) rec[i * S] = 0;
         for (uint32_t i = Grp::rank(); i < K.det_words; i += Grp::size()) det[i * S] = 0;
         for (uint32_t i = Grp::rank(); i < K.obs_words; i += Grp::size()) obs[i * S] = 0;
-        if (meas_prob)
+        if (meas_prob && leader())
             for (uint32_t i = Grp::rank(); i < P.slots; i += Grp::size())
                 meas_prob[i] = __longlong_as_double(0x7ff8000000000000ll);
         if (Grp::rank() == 0) A(0) = Cx<R>::make(1.0, 0.0);
@@ -3413,6 +3622,7 @@ struct Shot {
             for (uint32_t i = 0; i < P.num_obs && i < P.n_expected; ++i)
                 if (P.expected[i]) obs[(i >> 5) * S] ^= 1u << (i & 31);
         Grp::sync();
+        if (!leader()) return;
         if (K.out_meas)
             for (uint32_t w = r; w < K.meas_out_words; w += Grp::size()) {
                 uint64_t lo = rec[2 * w * S];
@@ -3494,7 +3704,8 @@ __host__ __device__ constexpr int shots_per_group_region() {
 }
 
 template <typename R, int G, int NW, bool DENSE = false>
-__global__ void __launch_bounds__(G == 0 ? 512 : (G < 0 ? 544 : 128), G <= 0 ? 1 : 4)
+__global__ void __launch_bounds__(G == 0 ? 512 : (G == -1 ? 544 : (G == -2 ? 288 : 128)),
+                                  G == -2 ? 2 : (G <= 0 ? 1 : 4))
     svm_sample_kernel(const DevProg P, const KParams K) {
     using Grp = typename GroupOf<G>::type;
     using T = typename Cx<R>::T;
@@ -3547,8 +3758,16 @@ __global__ void __launch_bounds__(G == 0 ? 512 : (G < 0 ? 544 : 128), G <= 0 ? 1
             tc_fence_after();
         }
     }
+    TeamLink link;
     T* v;
-    if (K.state_in_smem) {
+    if constexpr (Grp::kTeam) {
+        const uint32_t t = blockIdx.x / K.team_size;
+        link.size = K.team_size;
+        link.rank = blockIdx.x - t * K.team_size;
+        link.counter = K.team_arrivals + (size_t)t * 32;
+        link.sums = K.team_sums + (size_t)t * 8 * K.team_size;
+        v = reinterpret_cast<T*>(K.state_global) + (size_t)t * K.state_stride;
+    } else if (K.state_in_smem) {
         v = reinterpret_cast<T*>(rbase) + Grp::slot();
     } else {
         const size_t gid = (size_t)blockIdx.x * regions + region;
@@ -3556,9 +3775,14 @@ __global__ void __launch_bounds__(G == 0 ? 512 : (G < 0 ? 544 : 128), G <= 0 ? 1
     }
     Tally tally;
     const unsigned long long n_items = K.seg_count_in ? *K.seg_count_in : K.shots;
+    // teams take shots in turn (their CTAs need no common counter for that)
+    unsigned long long team_next = Grp::kTeam ? blockIdx.x / K.team_size : 0u;
     for (;;) {
         unsigned long long base = 0;
-        if (Grp::kCta) {
+        if constexpr (Grp::kTeam) {
+            base = (bar_phase >> 31) ? ~0ull : team_next;
+            team_next += gridDim.x / K.team_size;
+        } else if (Grp::kCta) {
             if (threadIdx.x == 0)
                 *bcast = (bar_phase >> 31) ? ~0ull : atomicAdd(K.work_counter, 1ull);
             __syncthreads();
@@ -3575,6 +3799,10 @@ __global__ void __launch_bounds__(G == 0 ? 512 : (G < 0 ? 544 : 128), G <= 0 ? 1
         if (item < n_items) {
             const unsigned long long shot = K.seg_in ? (unsigned long long)K.seg_in[item] : item;
             Shot<R, Grp, NW, DENSE> s(P, K, v, rec, det, obs, red, fz, &bar_phase, shot);
+            if constexpr (Grp::kTeam) {
+                s.team = &link;
+                s.team_v = v;
+            }
             s.run(tally);
         }
         if (!Grp::kCta) __syncwarp();
