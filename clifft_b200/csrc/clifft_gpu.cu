@@ -24,6 +24,7 @@
 #include "svm_dispatch.h"
 #include "svm_grad.h"
 #include "svm_kernel.cuh"
+#include "svm_plan.h"
 #include "svm_sample_k.h"
 
 using namespace cgpu;
@@ -380,6 +381,14 @@ struct clifft_gpu_program {
     mutable std::mutex plan_mu;
     mutable std::map<std::tuple<uint32_t, uint32_t, bool, uint32_t, uint32_t, uint32_t, bool>, std::vector<uint8_t>>
         plan_cache;
+    // fused blocks of the device stream, planned and uploaded once per tile
+    // geometry (precision, CTA or warp tiles, fusion, teams)
+    struct Plans {
+        void* dev = nullptr;
+        const BlockPlan* blocks = nullptr;
+        const PlanOp* ops = nullptr;
+    };
+    std::map<std::tuple<uint32_t, bool, bool, bool>, Plans> plans;  // under plan_mu
     // Statevector slab kept between calls (mapping tens of GB afresh on every
     // call costs more than a large-k launch's own setup). One call at a time
     // holds it; a concurrent call on the same handle allocates its own.
@@ -545,6 +554,34 @@ int default_group(uint32_t peak) {
     int g = 1;
     while (g < 32 && uint64_t(g) * 32 < amps) g <<= 1;
     return g;
+}
+
+// The fused blocks for a launch shape whose statevectors stream through tiles
+// (built and uploaded on first use).
+clifft_gpu_program::Plans block_plans(clifft_gpu_program& p, uint32_t precision, bool cta, bool fuse, bool team) {
+    std::lock_guard<std::mutex> lock(p.plan_mu);
+    auto& e = p.plans[std::make_tuple(precision, cta, fuse, team)];
+    if (e.dev) return e;
+    auto geometry = [&](auto cfg) {
+        using TC = decltype(cfg);
+        return PlanGeometry{uint32_t(TC::kBits), fuse ? uint32_t(TC::kMops) : 1u, cta, team};
+    };
+    const PlanGeometry g = precision == CLIFFT_GPU_FP32
+                               ? (cta ? geometry(TileCfg<float, true>{}) : geometry(TileCfg<float, false>{}))
+                               : (cta ? geometry(TileCfg<double, true>{}) : geometry(TileCfg<double, false>{}));
+    const PlanSet set = plan_blocks(p.code_host.data(), uint32_t(p.code_origin.size()), g);
+    BlobBuilder b;
+    const size_t o_blocks = b.put(set.blocks.data(), set.blocks.size());
+    const size_t o_ops = b.put(set.ops.data(), set.ops.size());
+    void* dev = nullptr;
+    CUDA_OK(alloc_retry([&] { return cudaMalloc(&dev, b.bytes.size() + 16); }));
+    const cudaError_t up = cudaMemcpy(dev, b.bytes.data(), b.bytes.size(), cudaMemcpyHostToDevice);
+    if (up != cudaSuccess) cudaFree(dev);
+    CUDA_OK(up);
+    e.dev = dev;
+    e.blocks = at<BlockPlan>(dev, o_blocks);
+    e.ops = at<PlanOp>(dev, o_ops);
+    return e;
 }
 
 // Everything of a plan except the grid size, which depends on the shot count
@@ -753,24 +790,31 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
 }
 
 // Team size for an untuned launch of `shots` shots (as a group request), or 0
-// for the one-CTA or one-warp shapes. Statevectors above 1 MiB only: below,
-// a warp per shot keeps more of the GPU busy and a team's CTAs have a handful
-// of tiles each. A launch of C CTAs per shot runs ceil(shots / teams) rounds,
-// each of which costs about
+// when a warp per shot is the better shape. A launch of C CTAs per shot runs
+// ceil(shots / teams) rounds, each of which costs about
 //     kOpUs x (opcodes on the statevector) + kTileUs x (tiles they cover) / C:
 // every CTA of a team interprets the whole program, so the first part does
-// not shrink with C. Measured (B200, two CTAs per SM; the last third is what a
-// CTA gains from having its SM to itself): k = 24 FP32, 147 opcodes, 117216
-// tiles: 98 ms / C + 1.9 ms; k = 20 FP32, 394 opcodes, 75336 tiles: 110 ms / C
-// + 3.0 ms; k = 18 FP64, 73 opcodes, 2670 tiles: 2.5 ms / C + 1.2 ms. One shot
-// of the k = 24 program takes 2.1 ms with 148 CTAs, 64 ms with one; 148 shots
-// 50 ms with teams of two, 66 ms with one CTA each.
+// not shrink with C; a CTA that has its SM to itself computes its tiles
+// faster (kAlone). Warps take all shots in one round, at
+//     kWarpOpUs x opcodes + kWarpTileUs x (warp tiles they cover).
+// Measured (B200): k = 24 FP32, 147 opcodes, 117216 tiles: 76 ms / C + 0.8 ms;
+// k = 20 FP32, 394 opcodes, 75336 tiles: 85 ms / C + 1.5 ms; k = 18 FP64, 73
+// opcodes, 2670 tiles: 2.1 ms / C + 0.5 ms. One shot of the k = 24 program
+// takes 1.0 ms with 296 CTAs, 57 ms with one; 148 shots 41 ms with teams of
+// two, 60 ms with one CTA each. Warps against teams of one, FP32: k = 14, 296
+// shots 0.37 / 0.32 ms, 592 shots 0.38 / 0.64 ms; k = 16, 296 shots 0.89 /
+// 0.51, 592 shots 0.91 / 1.00; k = 17, 592 shots 1.89 / 1.48, 1000 shots
+// 2.1 / 2.8; k = 12 0.16 / 0.18 at any count.
 uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_t shots, uint32_t max_resident) {
-    constexpr double kOpUs = 7.0, kTileUs = 1.0, kAlone = 0.66;
+    constexpr double kOpUs = 3.2, kTileUs = 0.8, kAlone = 0.7, kWarpOpUs = 2.3;
     constexpr uint32_t kPerSm = 2;
     const bool fp64 = precision == CLIFFT_GPU_FP64;
-    const size_t state_bytes = (size_t(1) << p.meta.peak_rank) * (fp64 ? 16 : 8);
-    if (state_bytes <= (size_t(1) << 20)) return 0;
+    const double kWarpTileUs = fp64 ? 0.44 : 0.37;
+    const uint32_t peak = p.meta.peak_rank;
+    const uint32_t bits = fp64 ? TileCfg<double, true>::kBits : TileCfg<float, true>::kBits;
+    const uint32_t warp_bits = fp64 ? TileCfg<double, false>::kBits : TileCfg<float, false>::kBits;
+    if (peak <= bits) return 0;
+    const size_t state_bytes = (size_t(1) << peak) * (fp64 ? 16 : 8);
     int dev = 0, sms = 0, coop = 0;
     size_t free_b = 0, total_b = 0;
     CUDA_OK(cudaGetDevice(&dev));
@@ -778,20 +822,18 @@ uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_
     CUDA_OK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
     if (!coop) return 0;
-    const uint32_t bits = fp64 ? TileCfg<double, true>::kBits : TileCfg<float, true>::kBits;
-    double ops = 0.0, tiles = 0.0;
+    double ops = 0.0, tiles = 0.0, warp_tiles = 0.0;
     for (uint32_t k = 0; k < p.ops_at_k.size(); ++k) {
         ops += p.ops_at_k[k];
         if (k > bits) tiles += double(p.ops_at_k[k]) * double(uint64_t(1) << (k - bits));
+        if (k > warp_bits) warp_tiles += double(p.ops_at_k[k]) * double(uint64_t(1) << (k - warp_bits));
     }
-    const uint64_t cap = uint64_t(kPerSm) * sms;
-    uint64_t most = std::max<uint64_t>(1, std::min<uint64_t>(shots, (free_b / 2) / state_bytes));
+    const uint64_t cap = uint64_t(kPerSm) * sms, peak_tiles = uint64_t(1) << (peak - bits);
+    uint64_t most = std::max<uint64_t>(1, std::min<uint64_t>({shots, cap, (free_b / 2) / state_bytes}));
     if (max_resident) most = std::min<uint64_t>(most, max_resident);
     double best = 0.0;
     uint32_t ctas = 0;
-    // every split of the GPU into equal teams, finest first: a coarser one has to be better
-    for (uint64_t c = 1; c <= uint64_t(sms); c = c < 8 ? c + 1 : c + c / 4) {
-        const uint64_t teams = std::min<uint64_t>(cap / c, most);
+    auto consider = [&](uint64_t teams, uint64_t c) {
         const double rounds = double((shots + teams - 1) / teams);
         const double share = tiles / double(c) * (teams * c <= uint64_t(sms) ? kAlone : 1.0);
         const double t = rounds * (kOpUs * ops + kTileUs * share);
@@ -799,7 +841,15 @@ uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_
             best = t;
             ctas = uint32_t(c);
         }
+    };
+    // every number of teams, each as large as the GPU allows and has tiles
+    // for; or one CTA each, when that leaves every CTA its own SM
+    for (uint64_t teams = most; teams >= 1; --teams) {
+        consider(teams, std::min<uint64_t>(cap / teams, peak_tiles));
+        if (teams <= uint64_t(sms)) consider(teams, 1);
     }
+    // a warp per shot is the default up to 1 MiB
+    if (state_bytes <= (size_t(1) << 20) && kWarpOpUs * ops + kWarpTileUs * warp_tiles <= best) return 0;
     return team_request(ctas);
 }
 
@@ -1121,6 +1171,8 @@ void clifft_gpu_free(clifft_gpu_program* prog) {
     if (prog->blob || prog->slab) {
         cudaDeviceSynchronize();
         if (prog->blob) cudaFree(prog->blob);
+        for (auto& e : prog->plans)
+            if (e.second.dev) cudaFree(e.second.dev);
         if (prog->slab) cudaFree(prog->slab);
     }
     delete prog;
@@ -1275,6 +1327,12 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             if (!dense_ok) Kx.flags &= ~uint32_t(KF_DENSE);
             Kx.fuse_bytes = Lx.tiles ? tile_scratch_bytes(args->precision, Lx.G == 0, Lx.stages, dense_ok) : 0;
             Kx.stages = Lx.stages;
+            Kx.plan = nullptr;
+            if (Lx.tiles) {
+                const auto bp = block_plans(*prog, args->precision, Lx.G == 0, Lx.fuse, Lx.team != 0);
+                Kx.plan = bp.blocks;
+                Kx.plan_ops = bp.ops;
+            }
             Kx.state_in_smem = Lx.state_in_smem ? 1 : 0;
             Kx.state_stride = Lx.state_stride;
             Kx.state_global = Lx.state_in_smem
@@ -1763,6 +1821,11 @@ int clifft_gpu_batch_create(clifft_gpu_program* const* progs, const clifft_gpu_s
                       (a.flags & CLIFFT_GPU_FORCED_FAULTS ? KF_FORCED_FAULTS : 0) | (it.L.fuse ? KF_FUSE : 0);
             K.fuse_bytes = it.L.tiles ? tile_scratch_bytes(a.precision, it.L.G == 0, it.L.stages) : 0;
             K.stages = it.L.stages;
+            if (it.L.tiles) {
+                const auto bp = block_plans(*p, a.precision, it.L.G == 0, it.L.fuse, false);
+                K.plan = bp.blocks;
+                K.plan_ops = bp.ops;
+            }
             K.rec_words = rec_words;
             K.det_words = det_words;
             K.obs_words = obs_words;

@@ -39,6 +39,7 @@
 #include <stdint.h>
 
 #include "clifft_program_image.h"
+#include "svm_plan.h"
 
 namespace cgpu {
 
@@ -131,6 +132,10 @@ struct KParams {
     uint64_t dump_shots;
     uint32_t fuse_bytes;  // shared bytes per CTA reserved for fused tile sweeps (0 = off)
     uint32_t stages;      // tile buffers per CTA (2..kMaxStages) when fuse_bytes != 0
+    // fused blocks of the device stream for this launch's tile geometry
+    // (svm_plan.h); null when no statevector pass streams
+    const BlockPlan* plan;
+    const PlanOp* plan_ops;
     // teams (G = -2): CTAs per shot, one arrival counter per team, and per team
     // two sets (used in turn) of four partial sums per CTA
     uint32_t team_size;
@@ -276,6 +281,10 @@ __device__ __forceinline__ double2 dmul(double2 a, double2 b) {
 #define CGPU_INV_SQRT2 0.70710678118654757
 #define CGPU_EXPAND_SCALE 0.70710678118654746
 
+// one copy of the rarely needed calls (a kernel inlines its handlers)
+static __device__ __noinline__ double hypot_call(double x, double y) { return hypot(x, y); }
+static __device__ __noinline__ double log_call(double x) { return log(x); }
+
 // ---------------------------------------------------------------- philox
 // Philox4x32-10 (Salmon et al., SC'11). Draw d of shot s uses counter
 // (d >> 1, stream, s_lo, s_hi) and key (seed_lo, seed_hi); even draws take
@@ -369,7 +378,9 @@ __device__ __forceinline__ uint64_t ins00(uint64_t v, uint32_t a, uint32_t b) {
     uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
     return ins0(ins0(v, lo), hi);
 }
-// the same on tile-local (32-bit) indices
+// the same on 32-bit indices: tile positions, and every per-opcode sweep
+// (those cover states of at most 2^31 amplitudes: larger ones stream through
+// tiles, and a warp of several shots cannot hold them)
 __device__ __forceinline__ uint32_t ins0_32(uint32_t v, uint32_t pos) {
     const uint32_t m = (1u << pos) - 1u;
     return (v & m) | ((v & ~m) << 1);
@@ -506,7 +517,7 @@ constexpr int kMaxRunsLog2 = 6;    // at most 64 contiguous runs per tile
 // leaves room for four 4-warp CTAs per SM (the register limit). Scratch
 // layout of one group: [2 x kMaxStages mbarriers: tile loaded / tile computed]
 // [dense-block slot: MMA mbarrier, TMEM address, phase][micro-ops][64 run
-// offsets][64-byte axis -> local bit table][stages tile buffers, 128-B
+// offsets][the block's plan][stages tile buffers, 128-B
 // aligned][FP32 CTA groups with three stages: the dense block's B operand,
 // 8 KiB].
 template <typename R, bool CTA>
@@ -518,8 +529,8 @@ struct TileCfg {
     static constexpr uint32_t kDenseSlotOffset = 2u * kMaxStages * 8u;
     static constexpr uint32_t kMopsOffset = kDenseSlotOffset + 16u;
     static constexpr uint32_t kTablesOffset = kMopsOffset + kMops * (uint32_t)sizeof(MOp);
-    static constexpr uint32_t kLbitOffset = kTablesOffset + 64u * 8u;
-    static constexpr uint32_t kBufOffset = (kLbitOffset + 64u + 127u) & ~127u;
+    static constexpr uint32_t kPlanOffset = kTablesOffset + 64u * 8u;
+    static constexpr uint32_t kBufOffset = (kPlanOffset + (uint32_t)sizeof(BlockPlan) + 127u) & ~127u;
     static constexpr uint32_t kDenseBBytes = 8192u;  // B operand of a dense block: TF32 hi + lo, 32 x 32 each
     static __host__ __device__ constexpr bool dense_capable(uint32_t stages) {
         return CTA && sizeof(R) == 4 && stages == 3;
@@ -731,7 +742,6 @@ struct Shot {
     unsigned char* fuse;       // shared scratch: stage barriers, micro-ops, index tables, tile buffers
     uint32_t* bar_phase;       // CTA groups: bit st = parity of the phase stage st's barrier is in;
                                // bit 31 set once a wait timed out (the barriers are then unusable)
-    bool resolving;            // true while a fused block's opcodes emit micro-ops
     bool solo;                 // CTA groups: only the control warp is executing
     int n_mops;
     unsigned long long moved;  // statevector bytes actually streamed
@@ -741,7 +751,12 @@ struct Shot {
     // are all above the tile bits, so the label maps every tile run to one
     // contiguous run.
     uint64_t xo;
-    uint64_t tileF;  // tile axes of the fused block being resolved
+    // fused blocks: the next one on this shot's way (they come in program order)
+    uint32_t plan_at;
+    uint32_t plan_pc;  // and the instruction it starts at
+    // one-shot groups read the instruction stream 32 at a time, one per lane
+    uint4 win;
+    uint32_t win_pc;
     // teams: while k <= kBits every CTA holds the whole state in its first
     // tile buffer (idle then) and computes it for itself; above, v is the
     // team's global statevector and passes are split between the CTAs
@@ -897,11 +912,18 @@ struct Shot {
     }
 
     __device__ __forceinline__ T& A(uint64_t i) { return v[(kTiles ? (i ^ xo) : i) * S]; }
+    __device__ __forceinline__ T& A(uint32_t i) {
+        if constexpr (kTiles)
+            return v[xo ^ i];
+        else
+            return v[(size_t)i * (uint32_t)S];
+    }
     // algorithmic bytes of an opcode (per-opcode definition); streamed bytes
     // are counted separately because a fused block streams the state once
+    template <bool RES = false>
     __device__ __forceinline__ void account(uint64_t amps) {
         bytes += amps * sizeof(T);
-        if (!resolving) moved += amps * sizeof(T);
+        if constexpr (!RES) moved += amps * sizeof(T);
     }
     __device__ __forceinline__ double uniform() { return philox_uniform(K.seed, K.first_shot + shot, draw++); }
     __device__ __forceinline__ void phase(double2 p) { gamma = dmul(gamma, p); }
@@ -929,18 +951,33 @@ struct Shot {
     // SchrodingerState::scale_magnitude (src/clifft/svm/svm.h:177-186). The
     // lazy-renormalisation window is 1e+-100 in FP64 and 1e+-20 in FP32 so the
     // FP32 amplitudes never approach their exponent range.
+    template <bool RES = false>
     __device__ __forceinline__ void scale_magnitude(double s) {
         gamma.x *= s;
         gamma.y *= s;
-        const double hi = sizeof(R) == 8 ? 1e100 : 1e20;
-        const double lo = sizeof(R) == 8 ? 1e-100 : 1e-20;
-        double g = hypot(gamma.x, gamma.y);
+        // |gamma| well inside the window: nothing to do (the square leaves a
+        // margin of 1 %; it neither over- nor underflows near the window)
+        constexpr double hi = sizeof(R) == 8 ? 1e100 : 1e20;
+        constexpr double lo = sizeof(R) == 8 ? 1e-100 : 1e-20;
+        const double g2 = gamma.x * gamma.x + gamma.y * gamma.y;
+        if (g2 < hi * hi * 0.98 && g2 > lo * lo * 1.02) return;
+        rescale<RES>();
+    }
+    template <bool RES>
+    __device__ __forceinline__ void rescale() {
+        constexpr double hi = sizeof(R) == 8 ? 1e100 : 1e20;
+        constexpr double lo = sizeof(R) == 8 ? 1e-100 : 1e-20;
+        const double g = hypot_call(gamma.x, gamma.y);
         if (g > hi || (g < lo && g > 0.0)) {
             uint64_t n = 1ull << k;
-            if (kTiles && resolving) {
-                // inside a fused block: the same scaling as a micro-op at this point
-                const double c[2] = {g, 0.0};
-                emit(M_SCALE, 0, 0, 0, 0, 0, c, 1);
+            if constexpr (RES) {
+                // inside a fused block: the same scaling as a micro-op, in the
+                // slot after the EXPAND that calls for it
+                if (Grp::rank() == 0) {
+                    MOp* m = mops() + n_mops - 1;
+                    m->kind = M_SCALE;
+                    m->c[0] = Cx<R>::make(g, 0.0);
+                }
                 bytes += 2 * n * sizeof(T);
             } else {
                 for (uint64_t i = wrank(); i < n; i += wsize()) A(i) = cscale(A(i), (R)g);
@@ -982,6 +1019,30 @@ struct Shot {
         Frame<NW>::put(f.x, b, xa);
         Frame<NW>::put(f.z, a, zb);
         Frame<NW>::put(f.z, b, za);
+    }
+    // First 16 bytes of instruction pc. A one-shot group's warps run one
+    // instruction stream in step: each lane holds one of 32 consecutive
+    // instructions and passes it on by shuffles, so the stream costs one load
+    // latency per 32 instructions (read one by one, every instruction was an L2
+    // miss: 570 cycles per scalar opcode of a lone CTA). Sub-warp groups may
+    // diverge and share L1 with 15 other warps; they load directly.
+    __device__ __forceinline__ uint4 fetch(uint32_t pc) {
+        if constexpr (kTiles) {
+            if (pc - win_pc >= 32u) {
+                win_pc = pc;
+                const uint32_t at = pc + (threadIdx.x & 31u);
+                win = __ldg(P.code + 2 * (at < P.n_code ? at : P.n_code - 1));
+            }
+            const int l = (int)(pc - win_pc);
+            return make_uint4(__shfl_sync(0xffffffffu, win.x, l), __shfl_sync(0xffffffffu, win.y, l),
+                              __shfl_sync(0xffffffffu, win.z, l), __shfl_sync(0xffffffffu, win.w, l));
+        }
+        return __ldg(P.code + 2 * pc);
+    }
+    // brings a line to L1
+    static __device__ __forceinline__ void touch(const void* p) {
+        uint32_t x;
+        asm volatile("ld.global.nc.u32 %0, [%1];\n" : "=r"(x) : "l"(p));
     }
     // axis mask of a condensed frame opcode
     __device__ __forceinline__ void star_mask(const uint4& w, uint64_t (&m)[NW]) const {
@@ -1095,14 +1156,14 @@ struct Shot {
     // first pc at or after `pc` that is not a frame opcode.
     __device__ __forceinline__ uint32_t frame_run(uint32_t pc, uint32_t n_instr) {
         if (pc >= n_instr) return pc;
-        uint4 w = __ldg(P.code + 2 * pc);
+        uint4 w = fetch(pc);
         if (!frame_op(w.x & 0xffu)) return pc;
         Frame<NW> ff = f;
         double2 g = gamma;
         for (;;) {
             if (!frame_op(w.x & 0xffu)) break;
-            const uint4 nxt = pc + 1 < n_instr ? __ldg(P.code + 2 * (pc + 1))
-                                               : make_uint4((uint32_t)CLIFFT_NUM_OPCODES, 0u, 0u, 0u);
+            const uint4 nxt =
+                pc + 1 < n_instr ? fetch(pc + 1) : make_uint4((uint32_t)CLIFFT_NUM_OPCODES, 0u, 0u, 0u);
             frame_step(w, ff, g);
             ++pc;
             w = nxt;
@@ -1114,213 +1175,197 @@ struct Shot {
     }
 
     // ---------------------------------------------------------- array ops
-    // Generic sweeps (shared-memory statevectors, and global ones smaller than
-    // a tile): one item per thread per step. Larger global statevectors stream
-    // through the bulk-copy tile engine instead (stream_tiles), which keeps many
-    // tiles in flight without holding them in registers.
-    static constexpr int U = 1;
-
-    template <class V, int UU = U, class Ld, class St>
-    __device__ __forceinline__ void sweep(uint64_t n, Ld ld, St st) {
-        const uint64_t step = (uint64_t)wsize();
-        for (uint64_t i0 = wrank(); i0 < n; i0 += step * UU) {
-            V val[UU];
-#pragma unroll
-            for (int u = 0; u < UU; ++u)
-                if (i0 + u * step < n) val[u] = ld(i0 + u * step);
-#pragma unroll
-            for (int u = 0; u < UU; ++u)
-                if (i0 + u * step < n) st(val[u]);
-        }
+    // Per-opcode sweeps (shared-memory statevectors, and global ones smaller
+    // than a tile; larger global statevectors stream through tiles): every
+    // item is loaded, computed and stored by one lane, in no particular order.
+    // One item at a time: two or four loads ahead cost registers that the warp
+    // groups' 128-register limit turns into spills (k = 10 0.40 -> 0.42 / 0.45
+    // ms, k = 16 3.9 -> 4.1 / 4.4 ms for 5000 shots).
+    template <class Ld, class St>
+    __device__ __forceinline__ void sweep(uint32_t n, Ld ld, St st) {
+        const uint32_t step = wsize();
+        for (uint32_t i = wrank(); i < n; i += step) st(ld(i));
+    }
+    // The same for sums: a lane adds its items in order.
+    template <class Ld, class Add>
+    __device__ __forceinline__ void reduce_sweep(uint32_t n, Ld ld, Add add) {
+        for (uint32_t i = Grp::rank(); i < n; i += Grp::size()) add(ld(i));
     }
     struct P2 {
-        uint64_t i;
+        uint32_t i;
         T x, y;
     };
     struct P1 {
-        uint64_t i;
+        uint32_t i;
         T x;
     };
     struct P4 {
-        uint64_t i;
+        uint32_t i;
         T x0, x1, x2, x3;
     };
 
-    // micro-op emission while resolving a fused block (thread 0 writes; every
-    // thread computes the same values)
+    // Resolving a fused block: its micro-ops are already in shared memory, the
+    // opcodes only add what the frame decides (coefficients c, nc complex
+    // values, converted to the statevector's precision as the unfused handlers
+    // convert them; one per thread, so a U4 node costs one load latency).
     using MOp = typename TC::MOp;
-    __device__ __forceinline__ uint8_t local_bit(uint32_t axis) const {
-        return reinterpret_cast<const uint8_t*>(fuse + fuse_lbit_offset())[axis];
-    }
     static __host__ __device__ constexpr uint32_t fuse_bar_offset() { return TC::kBarOffset; }
     static __host__ __device__ constexpr uint32_t fuse_mops_offset() { return TC::kMopsOffset; }
     static __host__ __device__ constexpr uint32_t fuse_tables_offset() { return TC::kTablesOffset; }
-    static __host__ __device__ constexpr uint32_t fuse_lbit_offset() { return TC::kLbitOffset; }
-    // local image of an axis mask (its bits on tile axes)
-    __device__ __forceinline__ uint32_t local_mask(uint64_t axes) const {
-        uint32_t lm = 0;
-        for (uint64_t w = axes & tileF; w; w &= w - 1) lm |= 1u << local_bit((uint32_t)__ffsll((long long)w) - 1);
-        return lm;
-    }
-    // a, b: target axes (tile axes); req / par: condition axes (any);
-    // coefficients c (nc complex values, converted to the statevector's
-    // precision as the unfused handlers convert them)
-    __device__ __forceinline__ void emit(uint8_t kind, uint32_t a, uint32_t b, uint64_t req, uint64_t par,
-                                         uint8_t flags, const double* c, int nc) {
-        MOp* m = reinterpret_cast<MOp*>(fuse + fuse_mops_offset()) + n_mops;
-        if (Grp::rank() == 0) {
-            m->kind = kind;
-            m->a = local_bit(a);
-            m->b = local_bit(b);
-            m->flags = flags;
-            m->req = local_mask(req);
-            m->par = local_mask(par);
-            m->greq = req & ~tileF;
-            m->gpar = par & ~tileF;
-        }
-        // coefficients (up to 16 complex values of a U4 node) converted one
-        // per thread: one global-load latency instead of a serial chain
+    __device__ __forceinline__ MOp* mops() const { return reinterpret_cast<MOp*>(fuse + fuse_mops_offset()); }
+    __device__ __forceinline__ void resolve_op(const double* c, int nc) {
+        MOp* m = mops() + n_mops;
         for (int j = Grp::rank(); j < nc; j += Grp::size()) m->c[j] = Cx<R>::make(c[2 * j], c[2 * j + 1]);
         n_mops++;
     }
 
     // exec_array_cnot (svm_kernels.inl:124-252)
+    template <bool RES>
     __device__ __forceinline__ void array_cnot(uint32_t c, uint32_t t) {
-        const uint64_t n = 1ull << (k - 2), cb = 1ull << c, tb = 1ull << t;
-        if (kTiles && resolving) {
-            emit(M_CNOT, t, t, 1ull << c, 0, 0, nullptr, 0);
+        const uint32_t n = 1u << (k - 2), cb = 1u << c, tb = 1u << t;
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P2>(n, [&](uint64_t i) { P2 p; p.i = ins00(i, c, t) | cb; p.x = A(p.i); p.y = A(p.i | tb); return p; },
+            sweep(n, [&](uint32_t i) { P2 p; p.i = ins00_32(i, c, t) | cb; p.x = A(p.i); p.y = A(p.i | tb); return p; },
                       [&](const P2& p) { A(p.i) = p.y; A(p.i | tb) = p.x; });
             Grp::sync();
         }
-        account(1ull << k);
+        account<RES>(1ull << k);
         frame_cnot(c, t);
     }
     // exec_array_cz (svm_kernels.inl:255-365)
+    template <bool RES>
     __device__ __forceinline__ void array_cz(uint32_t c, uint32_t t) {
-        const uint64_t n = 1ull << (k - 2), both = (1ull << c) | (1ull << t);
-        if (kTiles && resolving) {
-            emit(M_CZ, c, t, (1ull << c) | (1ull << t), 0, 0, nullptr, 0);
+        const uint32_t n = 1u << (k - 2), both = (1u << c) | (1u << t);
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P1>(n, [&](uint64_t i) { P1 p; p.i = ins00(i, c, t) | both; p.x = A(p.i); return p; },
+            sweep(n, [&](uint32_t i) { P1 p; p.i = ins00_32(i, c, t) | both; p.x = A(p.i); return p; },
                       [&](const P1& p) { A(p.i) = cneg(p.x); });
             Grp::sync();
         }
-        account(1ull << (k - 1));
+        account<RES>(1ull << (k - 1));
         frame_cz(c, t);
     }
     // exec_array_swap (svm_kernels.inl:369-458)
+    template <bool RES>
     __device__ __forceinline__ void array_swap(uint32_t a, uint32_t b) {
-        const uint64_t n = 1ull << (k - 2), ab = 1ull << a, bb = 1ull << b;
-        if (kTiles && resolving) {
-            emit(M_SWAP, a, b, 0, 0, 0, nullptr, 0);
+        const uint32_t n = 1u << (k - 2), ab = 1u << a, bb = 1u << b;
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P2>(n, [&](uint64_t i) { P2 p; p.i = ins00(i, a, b); p.x = A(p.i | ab); p.y = A(p.i | bb); return p; },
+            sweep(n, [&](uint32_t i) { P2 p; p.i = ins00_32(i, a, b); p.x = A(p.i | ab); p.y = A(p.i | bb); return p; },
                       [&](const P2& p) { A(p.i | ab) = p.y; A(p.i | bb) = p.x; });
             Grp::sync();
         }
-        account(1ull << k);
+        account<RES>(1ull << k);
         frame_swap(a, b);
     }
     // exec_array_multi_cnot (svm_kernels.inl:464-550)
+    template <bool RES>
     __device__ __forceinline__ void array_multi_cnot(uint32_t t, uint64_t mask) {
-        const uint64_t n = 1ull << (k - 1), tb = 1ull << t;
-        if (kTiles && resolving) {
-            emit(M_MCNOT, t, t, 0, mask & ~tb, MF_PARITY, nullptr, 0);
+        const uint32_t n = 1u << (k - 1), tb = 1u << t, low = (uint32_t)mask;
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P2>(n,
-                      [&](uint64_t i) {
+            sweep(n,
+                      [&](uint32_t i) {
                           P2 p;
-                          p.i = ins0(i, t);
-                          if (__popcll(p.i & mask) & 1) {
+                          p.i = ins0_32(i, t);
+                          if (__popc(p.i & low) & 1) {
                               p.x = A(p.i);
                               p.y = A(p.i | tb);
                           } else {
-                              p.i = ~0ull;
+                              p.i = ~0u;
                           }
                           return p;
                       },
                       [&](const P2& p) {
-                          if (p.i != ~0ull) {
+                          if (p.i != ~0u) {
                               A(p.i) = p.y;
                               A(p.i | tb) = p.x;
                           }
                       });
             Grp::sync();
         }
-        account(1ull << k);
+        account<RES>(1ull << k);
         uint64_t m[NW] = {mask};
         cnot_gather(f, t, m);
     }
     // exec_array_multi_cz (svm_kernels.inl:558-635)
+    template <bool RES>
     __device__ __forceinline__ void array_multi_cz(uint32_t c, uint64_t mask) {
-        const uint64_t n = 1ull << (k - 1), cb = 1ull << c;
-        if (kTiles && resolving) {
-            emit(M_MCZ, c, c, cb, mask, MF_PARITY, nullptr, 0);
+        const uint32_t n = 1u << (k - 1), cb = 1u << c, low = (uint32_t)mask;
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P1>(n,
-                      [&](uint64_t i) {
+            sweep(n,
+                      [&](uint32_t i) {
                           P1 p;
-                          p.i = ins0(i, c) | cb;
-                          if (__popcll(p.i & mask) & 1)
+                          p.i = ins0_32(i, c) | cb;
+                          if (__popc(p.i & low) & 1)
                               p.x = A(p.i);
                           else
-                              p.i = ~0ull;
+                              p.i = ~0u;
                           return p;
                       },
                       [&](const P1& p) {
-                          if (p.i != ~0ull) A(p.i) = cneg(p.x);
+                          if (p.i != ~0u) A(p.i) = cneg(p.x);
                       });
             Grp::sync();
         }
-        account(1ull << k);
+        account<RES>(1ull << k);
         uint64_t m[NW] = {mask};
         cz_fan(f, gamma, c, m);
     }
     // exec_array_h (svm_kernels.inl:639-744): (a +- b) / sqrt(2)
+    template <bool RES>
     __device__ __forceinline__ void array_h(uint32_t a) {
-        const uint64_t n = 1ull << (k - 1), ab = 1ull << a;
+        const uint32_t n = 1u << (k - 1), ab = 1u << a;
         const R s = (R)CGPU_INV_SQRT2;
-        if (kTiles && resolving) {
-            emit(M_H, a, a, 0, 0, 0, nullptr, 0);
+        if constexpr (RES) {
+            resolve_op(nullptr, 0);
         } else {
-            sweep<P2>(n, [&](uint64_t i) { P2 p; p.i = ins0(i, a); p.x = A(p.i); p.y = A(p.i | ab); return p; },
+            sweep(n, [&](uint32_t i) { P2 p; p.i = ins0_32(i, a); p.x = A(p.i); p.y = A(p.i | ab); return p; },
                       [&](const P2& p) {
                           A(p.i) = cscale(cadd(p.x, p.y), s);
                           A(p.i | ab) = cscale(csub(p.x, p.y), s);
                       });
             Grp::sync();
         }
-        account(2ull << k);
+        account<RES>(2ull << k);
         frame_h(a);
     }
     // apply_phase_waterfall (svm_kernels.inl:764-830)
+    template <bool RES>
     __device__ __forceinline__ void phase_sweep(uint32_t a, double re, double im) {
-        const uint64_t n = 1ull << (k - 1), ab = 1ull << a;
-        if (kTiles && resolving) {
+        const uint32_t n = 1u << (k - 1), ab = 1u << a;
+        if constexpr (RES) {
             const double c[2] = {re, im};
-            emit(M_PHASE, a, a, ab, 0, 0, c, 1);
+            resolve_op(c, 1);
         } else {
             const T ph = Cx<R>::make(re, im);
-            sweep<P1>(n, [&](uint64_t i) { P1 p; p.i = ins0(i, a) | ab; p.x = A(p.i); return p; },
+            sweep(n, [&](uint32_t i) { P1 p; p.i = ins0_32(i, a) | ab; p.x = A(p.i); return p; },
                       [&](const P1& p) { A(p.i) = cmul(p.x, ph); });
             Grp::sync();
         }
-        account(1ull << k);
+        account<RES>(1ull << k);
     }
     // exec_array_t / t_dag / rot (svm_kernels.inl:951-988,1044-1061)
+    template <bool RES, bool SV>
     __device__ __forceinline__ void array_rot(uint32_t a, double zr, double zi) {
         int x = f.px(a);
         if (a >= k) {
             if (x) phase(make_double2(zr, zi));
             return;
         }
-        if (x) {
-            phase_sweep(a, zr, -zi);
-            phase(make_double2(zr, zi));
-        } else {
-            phase_sweep(a, zr, zi);
+        if constexpr (SV) {
+            if (x) {
+                phase_sweep<RES>(a, zr, -zi);
+                phase(make_double2(zr, zi));
+            } else {
+                phase_sweep<RES>(a, zr, zi);
+            }
         }
     }
     // Threads that compute on tiles in a fused block (the whole group, or
@@ -1352,26 +1397,28 @@ struct Shot {
 
     // exec_expand / expand_with_phase / exec_expand_{t,t_dag,rot}
     // (svm_kernels.inl:876-1081)
+    template <bool RES>
     __device__ __forceinline__ void expand(uint32_t a, bool with_phase, double zr, double zi) {
         const uint64_t half = 1ull << k;
         int x = with_phase ? f.px(a) : 0;
         const T ph = Cx<R>::make(with_phase ? zr : 1.0, with_phase ? (x ? -zi : zi) : 0.0);
-        if (kTiles && resolving) {
+        if constexpr (RES) {
             // inside a fused block: the new axis is a tile axis and the copy a micro-op
             const double c[2] = {with_phase ? zr : 1.0, with_phase ? (x ? -zi : zi) : 0.0};
-            emit(M_EXPAND, a, a, 0, 0, with_phase ? 0 : MF_COPY, c, 1);
+            resolve_op(c, 1);
+            n_mops++;  // the slot of a renormalisation
             bytes += (2ull << k) * sizeof(T);
             k++;
-            scale_magnitude(CGPU_EXPAND_SCALE);
+            scale_magnitude<RES>(CGPU_EXPAND_SCALE);
             if (with_phase && x) phase(make_double2(zr, zi));
             return;
         }
         if constexpr (Grp::kTeam) {
             if (k == (uint32_t)TC::kBits) {
                 leave_private(with_phase, ph);
-                account(2ull << k);
+                account<RES>(2ull << k);
                 k++;
-                scale_magnitude(CGPU_EXPAND_SCALE);
+                scale_magnitude<RES>(CGPU_EXPAND_SCALE);
                 if (with_phase && x) phase(make_double2(zr, zi));
                 return;
             }
@@ -1392,25 +1439,27 @@ struct Shot {
                 moved += (2ull << k) * sizeof(T);
                 bytes += (2ull << k) * sizeof(T);
                 k++;
-                scale_magnitude(CGPU_EXPAND_SCALE);
+                scale_magnitude<RES>(CGPU_EXPAND_SCALE);
                 if (with_phase && x) phase(make_double2(zr, zi));
                 return;
             }
         }
+        const uint32_t h32 = (uint32_t)half;
         if (!with_phase) {
-            sweep<P1>(half, [&](uint64_t i) { P1 p; p.i = i; p.x = A(i); return p; },
-                      [&](const P1& p) { A(half + p.i) = p.x; });
+            sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i); return p; },
+                  [&](const P1& p) { A(h32 + p.i) = p.x; });
         } else {
-            sweep<P1>(half, [&](uint64_t i) { P1 p; p.i = i; p.x = A(i); return p; },
-                      [&](const P1& p) { A(half + p.i) = cmul(p.x, ph); });
+            sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i); return p; },
+                  [&](const P1& p) { A(h32 + p.i) = cmul(p.x, ph); });
         }
         Grp::sync();
-        account(2ull << k);
+        account<RES>(2ull << k);
         k++;
-        scale_magnitude(CGPU_EXPAND_SCALE);
+        scale_magnitude<RES>(CGPU_EXPAND_SCALE);
         if (with_phase && x) phase(make_double2(zr, zi));
     }
     // exec_array_u2 (svm_kernels.inl:1087-1297)
+    template <bool RES, bool SV>
     __device__ __forceinline__ void array_u2(uint32_t a, uint32_t cp) {
         const double* node = P.u2 + (size_t)cp * CLIFFT_U2_DOUBLES_PER_NODE;
         int st = (f.pz(a) << 1) | f.px(a);
@@ -1419,24 +1468,25 @@ struct Shot {
         uint8_t out = P.u2_out[cp * 4 + st];
         Frame<NW>::put(f.x, a, out & 1);
         Frame<NW>::put(f.z, a, (out >> 1) & 1);
-        if (a >= k) return;
-        if (kTiles && resolving) {
-            emit(M_U2, a, a, 0, 0, 0, m, 4);
-            account(2ull << k);
+        if (!SV || a >= k) return;
+        if constexpr (RES) {
+            resolve_op(m, 4);
+            account<RES>(2ull << k);
             return;
         }
         const T m00 = Cx<R>::make(m[0], m[1]), m01 = Cx<R>::make(m[2], m[3]);
         const T m10 = Cx<R>::make(m[4], m[5]), m11 = Cx<R>::make(m[6], m[7]);
-        const uint64_t n = 1ull << (k - 1), ab = 1ull << a;
-        sweep<P2>(n, [&](uint64_t i) { P2 p; p.i = ins0(i, a); p.x = A(p.i); p.y = A(p.i | ab); return p; },
+        const uint32_t n = 1u << (k - 1), ab = 1u << a;
+        sweep(n, [&](uint32_t i) { P2 p; p.i = ins0_32(i, a); p.x = A(p.i); p.y = A(p.i | ab); return p; },
                   [&](const P2& p) {
                       A(p.i) = cmac(cmul(m00, p.x), m01, p.y);
                       A(p.i | ab) = cmac(cmul(m10, p.x), m11, p.y);
                   });
         Grp::sync();
-        account(2ull << k);
+        account<RES>(2ull << k);
     }
     // exec_array_u4 (svm_kernels.inl:1310-1531)
+    template <bool RES>
     __device__ __forceinline__ void array_u4(uint32_t lo, uint32_t hi, uint32_t cp) {
         const double* node = P.u4 + (size_t)cp * CLIFFT_U4_DOUBLES_PER_NODE;
         int st = (f.pz(hi) << 3) | (f.px(hi) << 2) | (f.pz(lo) << 1) | f.px(lo);
@@ -1447,19 +1497,19 @@ struct Shot {
         Frame<NW>::put(f.z, lo, (out >> 1) & 1);
         Frame<NW>::put(f.x, hi, (out >> 2) & 1);
         Frame<NW>::put(f.z, hi, (out >> 3) & 1);
-        if (kTiles && resolving) {
-            emit(M_U4, lo, hi, 0, 0, 0, e, 16);
-            account(2ull << k);
+        if constexpr (RES) {
+            resolve_op(e, 16);
+            account<RES>(2ull << k);
             return;
         }
-        const uint64_t n = 1ull << (k - 2), lb = 1ull << lo, hb = 1ull << hi;
+        const uint32_t n = 1u << (k - 2), lb = 1u << lo, hb = 1u << hi;
         T m[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) m[j] = Cx<R>::make(e[2 * j], e[2 * j + 1]);
-        sweep<P4, (U > 2 ? 2 : U)>(n,
-                  [&](uint64_t i) {
+        sweep(n,
+                  [&](uint32_t i) {
                       P4 p;
-                      p.i = ins00(i, lo, hi);
+                      p.i = ins00_32(i, lo, hi);
                       p.x0 = A(p.i);
                       p.x1 = A(p.i | lb);
                       p.x2 = A(p.i | hb);
@@ -1482,7 +1532,7 @@ struct Shot {
                       A(p.i | lb | hb) = y[3];
                   });
         Grp::sync();
-        account(2ull << k);
+        account<RES>(2ull << k);
     }
 
     // ------------------------------------------------------- measurements
@@ -1510,7 +1560,7 @@ struct Shot {
             return b;
         }
         double pb = (want ? p1 : p0) / total;
-        log_prob += log(pb);
+        log_prob += log_call(pb);
         *prob = pb;
         return want;
     }
@@ -1536,7 +1586,7 @@ struct Shot {
         int m_abs;
         if (want >= 0) {
             m_abs = want ^ sign;
-            log_prob += log(0.5);
+            log_prob += log_call(0.5);
         } else {
             m_abs = uniform() < 0.5 ? 0 : 1;
         }
@@ -1560,7 +1610,7 @@ struct Shot {
         double acc[2] = {0.0, 0.0};
         const bool tl = tiled(k);
         if (tl) {
-            if constexpr (kTiles) {
+            if constexpr (kTiles && !Grp::kTeam) {  // (a team's are in planned blocks)
                 constexpr uint32_t MB = TC::kBits, TN = 1u << MB;
                 set_runs_low();
                 const int tid = Grp::rank(), nthr = Grp::size();
@@ -1579,22 +1629,12 @@ struct Shot {
                 moved += (1ull << k) * sizeof(T);
             }
         } else {
-            const uint64_t step = (uint64_t)Grp::size();
-            for (uint64_t i0 = Grp::rank(); i0 < half; i0 += step * U) {
-                T x[U], y[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (i0 + u * step < half) {
-                        x[u] = A(i0 + u * step);
-                        y[u] = A(i0 + u * step + half);
-                    }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (i0 + u * step < half) {
-                        acc[0] += cnorm_d(x[u]);
-                        acc[1] += cnorm_d(y[u]);
-                    }
-            }
+            const uint32_t h32 = (uint32_t)half;
+            reduce_sweep(h32, [&](uint32_t i) { P2 p; p.x = A(i); p.y = A(i + h32); return p; },
+                         [&](const P2& p) {
+                             acc[0] += cnorm_d(p.x);
+                             acc[1] += cnorm_d(p.y);
+                         });
         }
         group_reduce<Grp, 2>(acc, red);
         if (tl)
@@ -1629,7 +1669,7 @@ struct Shot {
                 if constexpr (kTiles) xo ^= half;
                 bytes += (1ull << k) * sizeof(T);
             } else if (tiled(k)) {
-                if constexpr (kTiles) {
+                if constexpr (kTiles && !Grp::kTeam) {
                     constexpr uint32_t MB = TC::kBits, TN = 1u << MB;
                     set_runs_low();
                     cur_site = 3;
@@ -1639,8 +1679,9 @@ struct Shot {
                     bytes += (1ull << k) * sizeof(T);
                 }
             } else {
-                sweep<P1>(half, [&](uint64_t i) { P1 p; p.i = i; p.x = A(i + half); return p; },
-                          [&](const P1& p) { A(p.i) = p.x; });
+                const uint32_t h32 = (uint32_t)half;
+                sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i + h32); return p; },
+                      [&](const P1& p) { A(p.i) = p.x; });
                 Grp::sync();
                 account(1ull << k);
             }
@@ -1661,7 +1702,8 @@ struct Shot {
     __device__ __forceinline__ void meas_interfere(uint32_t fa, uint32_t t, uint32_t idx, int sign) {
         const bool swapped = fa != t;
         if (swapped) frame_swap(fa, t);
-        const uint64_t half = 1ull << t, fb = 1ull << fa;
+        const uint64_t fb = 1ull << fa;
+        const uint32_t h32 = 1u << (t & 31u), f32 = 1u << (fa & 31u);  // untiled sweeps
         double acc[2] = {0.0, 0.0};
         // tiled path: the tile spans axes {fa, t} (t is its top local bit);
         // outputs are the tile positions with the t bit clear
@@ -1669,7 +1711,7 @@ struct Shot {
         uint32_t tr = 0, lf = 0;
         uint64_t tC = 0;
         if (tl) {
-            if constexpr (kTiles) {
+            if constexpr (kTiles && !Grp::kTeam) {
                 constexpr uint32_t MB = TC::kBits;
                 const uint64_t F = tile_axes((1ull << t) | fb, tr);
                 tC = ((1ull << k) - 1) & ~F;
@@ -1694,26 +1736,17 @@ struct Shot {
                 moved += (1ull << k) * sizeof(T);
             }
         } else {
-            const uint64_t step = (uint64_t)Grp::size();
-            for (uint64_t i0 = Grp::rank(); i0 < half; i0 += step * U) {
-                T x[U], y[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint64_t i = i0 + u * step;
-                    if (i < half) {
-                        uint64_t a0 = swapped ? ((i & ~fb) | (((i >> fa) & 1ull) << t)) : i;
-                        uint64_t a1 = swapped ? (a0 | fb) : (i + half);
-                        x[u] = A(a0);
-                        y[u] = A(a1);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (i0 + u * step < half) {
-                        acc[0] += cnorm_d(cadd(x[u], y[u]));
-                        acc[1] += cnorm_d(csub(x[u], y[u]));
-                    }
-            }
+            reduce_sweep(h32, [&](uint32_t i) {
+                             const uint32_t a0 = swapped ? ((i & ~f32) | (((i >> fa) & 1u) << t)) : i;
+                             P2 p;
+                             p.x = A(a0);
+                             p.y = A(swapped ? (a0 | f32) : (i + h32));
+                             return p;
+                         },
+                         [&](const P2& p) {
+                             acc[0] += cnorm_d(cadd(p.x, p.y));
+                             acc[1] += cnorm_d(csub(p.x, p.y));
+                         });
         }
         group_reduce<Grp, 2>(acc, red);
         if (tl)
@@ -1734,7 +1767,7 @@ struct Shot {
         }
         const R s = (R)CGPU_INV_SQRT2;
         if (tl) {
-            if constexpr (kTiles) {
+            if constexpr (kTiles && !Grp::kTeam) {
                 constexpr uint32_t MB = TC::kBits;
                 const int tid = Grp::rank(), nthr = Grp::size();
                 const uint32_t lt = MB - 1, lfb = 1u << lf, HN = 1u << lt;
@@ -1763,19 +1796,19 @@ struct Shot {
                 moved += (1ull << k) * sizeof(T) + (1ull << (k - 1)) * sizeof(T);
             }
         } else if (!swapped) {
-            sweep<P2>(half, [&](uint64_t i) { P2 p; p.i = i; p.x = A(i); p.y = A(i + half); return p; },
-                      [&](const P2& p) { A(p.i) = cscale(bx ? csub(p.x, p.y) : cadd(p.x, p.y), s); });
+            sweep(h32, [&](uint32_t i) { P2 p; p.i = i; p.x = A(i); p.y = A(i + h32); return p; },
+                  [&](const P2& p) { A(p.i) = cscale(bx ? csub(p.x, p.y) : cadd(p.x, p.y), s); });
             Grp::sync();
         } else {
-            const uint64_t q = half >> 1;  // outputs with bit fa clear, then set
+            const uint32_t q = h32 >> 1;  // outputs with bit fa clear, then set
             for (int pass = 0; pass < 2; ++pass) {
-                sweep<P2>(q,
-                          [&](uint64_t j) {
+                sweep(q,
+                          [&](uint32_t j) {
                               P2 p;
-                              p.i = ins0(j, fa) | (pass ? fb : 0ull);
-                              uint64_t a0 = pass ? ((p.i & ~fb) | half) : p.i;
+                              p.i = ins0_32(j, fa) | (pass ? f32 : 0u);
+                              const uint32_t a0 = pass ? ((p.i & ~f32) | h32) : p.i;
                               p.x = A(a0);
-                              p.y = A(a0 | fb);
+                              p.y = A(a0 | f32);
                               return p;
                           },
                           [&](const P2& p) { A(p.i) = cscale(bx ? csub(p.x, p.y) : cadd(p.x, p.y), s); });
@@ -1809,9 +1842,10 @@ struct Shot {
     // and summed the two halves' norms (w0 bit t clear, w1 set; each 1/2 of
     // the reference's |x +- y|^2 sums, which leaves every ratio unchanged).
     // Branch bx keeps the half with bit t = bx: the address label flips for
-    // bx = 1. Diagonal measurements go to diag_tail.
+    // bx = 1 (relabel), or that half is copied down (a state held in one
+    // tile). Diagonal measurements go to diag_tail.
     __device__ __forceinline__ void interfere_relabel(uint32_t fa, uint32_t t, uint32_t idx, int sign, double w0,
-                                                      double w1) {
+                                                      double w1, bool relabel) {
         const bool swapped = fa != t;
         if (swapped) frame_swap(fa, t);
         bytes += ((1ull << k) * 2 + (1ull << (k - 1))) * sizeof(T);
@@ -1828,7 +1862,14 @@ struct Shot {
             return;
         }
         if (bx == 1) {
-            if constexpr (kTiles) xo ^= 1ull << t;
+            if (relabel) {
+                if constexpr (kTiles) xo ^= 1ull << t;
+            } else {
+                const uint32_t h32 = 1u << t;
+                sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i + h32); return p; },
+                      [&](const P1& p) { A(p.i) = p.x; });
+                Grp::sync();
+            }
         }
         interfere_tail(swapped, t, idx, sign, pxv, pzv, bx, w0, w1, prob);
     }
@@ -1855,7 +1896,7 @@ struct Shot {
             return;
         }
         double cur = next_noise == 0 ? 0.0 : __ldg(P.hazards + next_noise - 1);
-        double gap = -log(1.0 - uniform());
+        double gap = -log_call(1.0 - uniform());
         double target = cur + gap;
         uint32_t lo = next_noise, hi = n;  // hazards are cumulative: answer >= next_noise
         while (lo < hi) {
@@ -1942,28 +1983,16 @@ struct Shot {
             double acc[3] = {0.0, 0.0, 0.0};
             const uint64_t dim = 1ull << k;
             const uint64_t step = (uint64_t)wsize();
-            for (uint64_t j0 = wrank(); j0 < dim; j0 += step * U) {
-                T av[U], bv[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (j0 + u * step < dim) {
-                        av[u] = A(j0 + u * step);
-                        bv[u] = A((j0 + u * step) ^ xa);
-                    }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint64_t j = j0 + u * step;
-                    if (j < dim) {
-                        double ar = (double)av[u].x, ai = (double)av[u].y;
-                        double br = (double)bv[u].x, bi = -(double)bv[u].y;
-                        acc[2] = __dadd_rn(acc[2], __fma_rn(ar, ar, __dmul_rn(ai, ai)));
-                        double zs = (__popcll(j & za) & 1) ? -1.0 : 1.0;
-                        ar *= zs;
-                        ai *= zs;
-                        acc[0] = __dadd_rn(acc[0], __fma_rn(br, ar, -__dmul_rn(bi, ai)));
-                        acc[1] = __dadd_rn(acc[1], __fma_rn(br, ai, __dmul_rn(bi, ar)));
-                    }
-                }
+            for (uint64_t j = wrank(); j < dim; j += step) {
+                const T av = A(j), bv = A(j ^ xa);
+                double ar = (double)av.x, ai = (double)av.y;
+                const double br = (double)bv.x, bi = -(double)bv.y;
+                acc[2] = __dadd_rn(acc[2], __fma_rn(ar, ar, __dmul_rn(ai, ai)));
+                const double zs = (__popcll(j & za) & 1) ? -1.0 : 1.0;
+                ar *= zs;
+                ai *= zs;
+                acc[0] = __dadd_rn(acc[0], __fma_rn(br, ar, -__dmul_rn(bi, ai)));
+                acc[1] = __dadd_rn(acc[1], __fma_rn(br, ai, __dmul_rn(bi, ar)));
             }
             state_reduce<3>(acc);
             account(1ull << k);
@@ -1974,69 +2003,9 @@ struct Shot {
         if (Grp::rank() == 0 && leader() && K.out_exp) K.out_exp[shot * P.num_exp + out_idx] = result;
     }
 
-    // Executes instruction `pc` (the dispatch of execute_internal,
-    // svm_kernels.inl:2183-2646; forced opcodes share the sampling handlers).
-    __device__ __forceinline__ void exec(uint32_t pc) {
-        cur_pc = pc;
-        const uint4* ip = P.code;
-        const uint4 w0 = __ldg(ip + 2 * pc);
-        uint32_t op = w0.x & 0xffu;
-        const uint32_t fl = (w0.x >> 16) & 0xffu;
-        const uint32_t a1 = w0.y & 0xffffu, a2 = w0.y >> 16;
-        const uint32_t p0 = w0.z, p1 = w0.w;
-        const int sign = (fl & CLIFFT_FLAG_SIGN) ? 1 : 0;
-        if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
-            op -= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED - CLIFFT_OP_MEAS_DORMANT_STATIC;
-            switch (op) {
-            case CLIFFT_OP_FRAME_CNOT:
-            case CLIFFT_OP_FRAME_CZ:
-            case CLIFFT_OP_FRAME_H:
-            case CLIFFT_OP_FRAME_S:
-            case CLIFFT_OP_FRAME_S_DAG:
-            case CLIFFT_OP_FRAME_SWAP:
-            case DOP_CNOT_FAN:
-            case DOP_CNOT_GATHER:
-            case DOP_CZ_FAN: frame_step(w0, f, gamma); break;
-            case CLIFFT_OP_ARRAY_CNOT: array_cnot(a1, a2); break;
-            case CLIFFT_OP_ARRAY_CZ: array_cz(a1, a2); break;
-            case CLIFFT_OP_ARRAY_SWAP: array_swap(a1, a2); break;
-            case CLIFFT_OP_ARRAY_MULTI_CNOT: array_multi_cnot(a1, ((uint64_t)p1 << 32) | p0); break;
-            case CLIFFT_OP_ARRAY_MULTI_CZ: array_multi_cz(a1, ((uint64_t)p1 << 32) | p0); break;
-            case CLIFFT_OP_ARRAY_H: array_h(a1); break;
-            case CLIFFT_OP_ARRAY_S:
-                phase_sweep(a1, 0.0, 1.0);
-                frame_s(a1, false);
-                break;
-            case CLIFFT_OP_ARRAY_S_DAG:
-                phase_sweep(a1, 0.0, -1.0);
-                frame_s(a1, true);
-                break;
-            case CLIFFT_OP_ARRAY_T: array_rot(a1, CGPU_INV_SQRT2, CGPU_INV_SQRT2); break;
-            case CLIFFT_OP_ARRAY_T_DAG: array_rot(a1, CGPU_INV_SQRT2, -CGPU_INV_SQRT2); break;
-            case CLIFFT_OP_ARRAY_ROT: {
-                const uint4 w1 = __ldg(ip + 2 * pc + 1);
-                array_rot(a1, __longlong_as_double(((long long)p1 << 32) | p0),
-                          __longlong_as_double(((long long)w1.y << 32) | w1.x));
-                break;
-            }
-            case CLIFFT_OP_ARRAY_U2: array_u2(a1, p0); break;
-            case CLIFFT_OP_ARRAY_U4: array_u4(a1, a2, p0); break;
-            case CLIFFT_OP_EXPAND: expand(a1, false, 0.0, 0.0); break;
-            case CLIFFT_OP_EXPAND_T: expand(a1, true, CGPU_INV_SQRT2, CGPU_INV_SQRT2); break;
-            case CLIFFT_OP_EXPAND_T_DAG: expand(a1, true, CGPU_INV_SQRT2, -CGPU_INV_SQRT2); break;
-            case CLIFFT_OP_EXPAND_ROT: {
-                const uint4 w1 = __ldg(ip + 2 * pc + 1);
-                expand(a1, true, __longlong_as_double(((long long)p1 << 32) | p0),
-                       __longlong_as_double(((long long)w1.y << 32) | w1.x));
-                break;
-            }
-            case CLIFFT_OP_MEAS_DORMANT_STATIC:
-                meas_dormant_static(a1, p0, sign, (fl & CLIFFT_FLAG_IDENTITY) != 0);
-                break;
-            case CLIFFT_OP_MEAS_DORMANT_RANDOM: meas_dormant_random(a1, p0, sign); break;
-            case CLIFFT_OP_MEAS_ACTIVE_DIAGONAL: meas_diagonal(a1, p0, sign); break;
-            case CLIFFT_OP_MEAS_ACTIVE_INTERFERE: meas_interfere(a1, a1, p0, sign); break;
-            case CLIFFT_OP_SWAP_MEAS_INTERFERE: meas_interfere(a1, a2, p0, sign); break;
+    // Pauli corrections, noise and record opcodes.
+    __device__ __forceinline__ void exec_classical(uint32_t op, uint32_t fl, uint32_t p0, uint32_t p1) {
+        switch (op) {
             case CLIFFT_OP_APPLY_PAULI:
                 flush_records();
                 if (bit_of(rec, p1, S))
@@ -2078,7 +2047,130 @@ struct Shot {
                 if (Grp::rank() == 0 && par) obs[(p1 >> 5) * S] ^= 1u << (p1 & 31);
                 break;
             }
-            case CLIFFT_OP_EXP_VAL: exp_val(p0, p1); break;
+            default: break;
+        }
+    }
+
+    // Executes instruction `pc`, first 16 bytes w0 (the dispatch of
+    // execute_internal, svm_kernels.inl:2183-2646; forced opcodes share the
+    // sampling handlers). Each caller instantiates only the opcodes that can
+    // reach it: kScalar (the control warp of a CTA: opcodes that leave the
+    // statevector alone), kState (every thread of a CTA: the others),
+    // kResolve (inside a fused block: frame and gamma of its opcodes, and
+    // their coefficients) or kAll (warp groups). One copy of everything in
+    // each place made the kernels several times larger, and a lone CTA waited
+    // for instructions more than for anything else.
+    enum : int { kAll, kScalar, kState, kResolve };
+    template <int MODE>
+    __device__ __forceinline__ void exec(uint32_t pc, const uint4& w0) {
+        constexpr bool RES = MODE == kResolve;
+        constexpr bool kSca = MODE == kAll || MODE == kScalar;  // scalar opcodes
+        constexpr bool kSv = MODE != kScalar;                   // opcodes on the statevector
+        constexpr bool kMeas = MODE == kAll || MODE == kState;
+        cur_pc = pc;
+        const uint4* ip = P.code;
+        uint32_t op = w0.x & 0xffu;
+        const uint32_t fl = (w0.x >> 16) & 0xffu;
+        const uint32_t a1 = w0.y & 0xffffu, a2 = w0.y >> 16;
+        const uint32_t p0 = w0.z, p1 = w0.w;
+        const int sign = (fl & CLIFFT_FLAG_SIGN) ? 1 : 0;
+        if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
+            op -= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED - CLIFFT_OP_MEAS_DORMANT_STATIC;
+            switch (op) {
+            case CLIFFT_OP_FRAME_CNOT:
+            case CLIFFT_OP_FRAME_CZ:
+            case CLIFFT_OP_FRAME_H:
+            case CLIFFT_OP_FRAME_S:
+            case CLIFFT_OP_FRAME_S_DAG:
+            case CLIFFT_OP_FRAME_SWAP:
+            case DOP_CNOT_FAN:
+            case DOP_CNOT_GATHER:
+            case DOP_CZ_FAN:
+                if constexpr (MODE != kState) frame_step(w0, f, gamma);
+                break;
+            case CLIFFT_OP_ARRAY_CNOT:
+                if constexpr (kSv) array_cnot<RES>(a1, a2);
+                break;
+            case CLIFFT_OP_ARRAY_CZ:
+                if constexpr (kSv) array_cz<RES>(a1, a2);
+                break;
+            case CLIFFT_OP_ARRAY_SWAP:
+                if constexpr (kSv) array_swap<RES>(a1, a2);
+                break;
+            case CLIFFT_OP_ARRAY_MULTI_CNOT:
+                if constexpr (kSv) array_multi_cnot<RES>(a1, ((uint64_t)p1 << 32) | p0);
+                break;
+            case CLIFFT_OP_ARRAY_MULTI_CZ:
+                if constexpr (kSv) array_multi_cz<RES>(a1, ((uint64_t)p1 << 32) | p0);
+                break;
+            case CLIFFT_OP_ARRAY_H:
+                if constexpr (kSv) array_h<RES>(a1);
+                break;
+            case CLIFFT_OP_ARRAY_S:
+                if constexpr (kSv) {
+                    phase_sweep<RES>(a1, 0.0, 1.0);
+                    frame_s(a1, false);
+                }
+                break;
+            case CLIFFT_OP_ARRAY_S_DAG:
+                if constexpr (kSv) {
+                    phase_sweep<RES>(a1, 0.0, -1.0);
+                    frame_s(a1, true);
+                }
+                break;
+            case CLIFFT_OP_ARRAY_T: array_rot<RES, kSv>(a1, CGPU_INV_SQRT2, CGPU_INV_SQRT2); break;
+            case CLIFFT_OP_ARRAY_T_DAG: array_rot<RES, kSv>(a1, CGPU_INV_SQRT2, -CGPU_INV_SQRT2); break;
+            case CLIFFT_OP_ARRAY_ROT: {
+                const uint4 w1 = __ldg(ip + 2 * pc + 1);
+                array_rot<RES, kSv>(a1, __longlong_as_double(((long long)p1 << 32) | p0),
+                          __longlong_as_double(((long long)w1.y << 32) | w1.x));
+                break;
+            }
+            case CLIFFT_OP_ARRAY_U2: array_u2<RES, kSv>(a1, p0); break;
+            case CLIFFT_OP_ARRAY_U4:
+                if constexpr (kSv) array_u4<RES>(a1, a2, p0);
+                break;
+            case CLIFFT_OP_EXPAND:
+                if constexpr (kSv) expand<RES>(a1, false, 0.0, 0.0);
+                break;
+            case CLIFFT_OP_EXPAND_T:
+                if constexpr (kSv) expand<RES>(a1, true, CGPU_INV_SQRT2, CGPU_INV_SQRT2);
+                break;
+            case CLIFFT_OP_EXPAND_T_DAG:
+                if constexpr (kSv) expand<RES>(a1, true, CGPU_INV_SQRT2, -CGPU_INV_SQRT2);
+                break;
+            case CLIFFT_OP_EXPAND_ROT:
+                if constexpr (kSv) {
+                    const uint4 w1 = __ldg(ip + 2 * pc + 1);
+                    expand<RES>(a1, true, __longlong_as_double(((long long)p1 << 32) | p0),
+                                __longlong_as_double(((long long)w1.y << 32) | w1.x));
+                }
+                break;
+            case CLIFFT_OP_MEAS_DORMANT_STATIC:
+                if constexpr (kSca) meas_dormant_static(a1, p0, sign, (fl & CLIFFT_FLAG_IDENTITY) != 0);
+                break;
+            case CLIFFT_OP_MEAS_DORMANT_RANDOM:
+                if constexpr (kSca) meas_dormant_random(a1, p0, sign);
+                break;
+            case CLIFFT_OP_MEAS_ACTIVE_DIAGONAL:
+                if constexpr (kMeas) meas_diagonal(a1, p0, sign);
+                break;
+            case CLIFFT_OP_MEAS_ACTIVE_INTERFERE:
+            case CLIFFT_OP_SWAP_MEAS_INTERFERE:
+                if constexpr (kMeas) meas_interfere(a1, op == CLIFFT_OP_SWAP_MEAS_INTERFERE ? a2 : a1, p0, sign);
+                break;
+            case CLIFFT_OP_APPLY_PAULI:
+            case CLIFFT_OP_NOISE:
+            case CLIFFT_OP_NOISE_BLOCK:
+            case CLIFFT_OP_READOUT_NOISE:
+            case CLIFFT_OP_DETECTOR:
+            case CLIFFT_OP_POSTSELECT:
+            case CLIFFT_OP_OBSERVABLE:
+                if constexpr (kSca) exec_classical(op, fl, p0, p1);
+                break;
+            case CLIFFT_OP_EXP_VAL:
+                if constexpr (kMeas) exp_val(p0, p1);
+                break;
             default:
                 if (Grp::rank() == 0) atomicCAS(K.error_word, 0, DEV_ERR_BAD_OPCODE);
                 stop = true;
@@ -2458,167 +2550,90 @@ struct Shot {
         return true;
     }
 
-    // Fused block starting at `pc` (one-shot groups, statevector in global
-    // memory, k > tile bits), ending before `limit`. With fusion (max_ops >
-    // 1) EXPANDs join the block and an active measurement ends it. Returns
-    // the number of instructions consumed, 0 when the opcode at `pc` does not
-    // start a block worth streaming.
-    // A fused block, in its dense-block instance when the launch asked for
-    // tensor-core dense blocks: the default instance carries none of that
-    // code, so its register allocation is the plain one. Kernels without
-    // DENSE contain no tcgen05 instruction at all: the instance that holds a
-    // TMEM allocation ran one CTA per SM at a time where shared memory and
-    // registers fit two (296 shots took twice as long as 148), and merely
-    // carrying that code slowed the default k = 24 path by 37 %.
-    __device__ __forceinline__ uint32_t run_block(uint32_t pc, int max_ops, uint32_t limit) {
-        if constexpr (kDenseOk) {
-            if (K.flags & KF_DENSE) return fused_block<true>(pc, max_ops, limit);
+    // The planned block that starts at `pc`, or 0 instructions when there is
+    // none (its opcode is executed alone). Blocks come in program order, so
+    // one cursor finds them.
+    // Tensor-core dense blocks exist only in the kernel instances built for
+    // them: the instance that holds a TMEM allocation ran one CTA per SM at a
+    // time where shared memory and registers fit two (296 shots took twice as
+    // long as 148), and merely carrying that code slowed the default k = 24
+    // path by 37 %.
+    __device__ __forceinline__ void plan_start(uint32_t pc) {
+        plan_at = 0;
+        plan_pc = 0xffffffffu;
+        if constexpr (kTiles) {
+            if (K.plan == nullptr) return;
+            while (__ldg(&K.plan[plan_at].pc) < pc) ++plan_at;
+            plan_pc = __ldg(&K.plan[plan_at].pc);
         }
-        return fused_block<false>(pc, max_ops, limit);
+    }
+    __device__ __forceinline__ uint32_t run_block(uint32_t pc) {
+        if (pc != plan_pc) return 0;
+        if constexpr (kDenseOk) {
+            if (K.flags & KF_DENSE) return fused_block<true>();
+        }
+        return fused_block<false>();
     }
     template <bool WITH_DENSE>
-    __device__ uint32_t fused_block(uint32_t pc, int max_ops, uint32_t limit) {
+    __device__ uint32_t fused_block() {
         constexpr uint32_t MB = TC::kBits;
-        const bool wide = max_ops > 1;
-        uint64_t need = 0;   // axes that must be tile axes
-        uint64_t fresh = 0;  // axes the block's EXPANDs create
-        int slots = 0;       // micro-op slots (an EXPAND reserves one for a renormalisation)
-        int nsweep = 0;      // array opcodes that touch the statevector
-        uint32_t kk = k;     // k after the instructions admitted so far
-        uint32_t end = pc;
-        uint32_t term = 0;   // the terminating measurement's pc
-        int term_kind = 0;   // 1 diagonal, 2 X-basis, 3 X-basis with a fused swap
-        for (; end < limit; ++end) {
-            const uint4 w0 = __ldg(P.code + 2 * end);
-            uint32_t op = w0.x & 0xffu;
-            const uint32_t x1 = w0.y & 0xffffu, x2 = w0.y >> 16;
-            if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
-                op -= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED - CLIFFT_OP_MEAS_DORMANT_STATIC;
-            uint64_t nd = 0;
-            int cost = 0, tk = 0;
-            bool expand_op = false, ok = true;
-            switch (op) {
-                case CLIFFT_OP_FRAME_CNOT:
-                case CLIFFT_OP_FRAME_CZ:
-                case CLIFFT_OP_FRAME_H:
-                case CLIFFT_OP_FRAME_S:
-                case CLIFFT_OP_FRAME_S_DAG:
-                case CLIFFT_OP_FRAME_SWAP:
-                case DOP_CNOT_FAN:
-                case DOP_CNOT_GATHER:
-                case DOP_CZ_FAN: break;
-                case CLIFFT_OP_ARRAY_CNOT: nd = 1ull << x2; cost = 1; break;          // the target moves
-                case CLIFFT_OP_ARRAY_MULTI_CNOT: nd = 1ull << x1; cost = 1; break;    // the target moves
-                case CLIFFT_OP_ARRAY_SWAP:
-                case CLIFFT_OP_ARRAY_U4: nd = (1ull << x1) | (1ull << x2); cost = 1; break;
-                case CLIFFT_OP_ARRAY_H: nd = 1ull << x1; cost = 1; break;
-                case CLIFFT_OP_ARRAY_CZ:
-                case CLIFFT_OP_ARRAY_MULTI_CZ:
-                case CLIFFT_OP_ARRAY_S:
-                case CLIFFT_OP_ARRAY_S_DAG: cost = 1; break;                           // diagonal: any axes
-                case CLIFFT_OP_ARRAY_T:
-                case CLIFFT_OP_ARRAY_T_DAG:
-                case CLIFFT_OP_ARRAY_ROT: cost = x1 < kk ? 1 : 0; break;
-                case CLIFFT_OP_ARRAY_U2:
-                    if (x1 < kk) {
-                        nd = 1ull << x1;
-                        cost = 1;
-                    }
-                    break;
-                case CLIFFT_OP_EXPAND:
-                case CLIFFT_OP_EXPAND_T:
-                case CLIFFT_OP_EXPAND_T_DAG:
-                case CLIFFT_OP_EXPAND_ROT:
-                    ok = wide;
-                    nd = 1ull << kk;
-                    cost = 2;
-                    expand_op = true;
-                    break;
-                case CLIFFT_OP_MEAS_ACTIVE_DIAGONAL: ok = wide; tk = 1; break;
-                case CLIFFT_OP_MEAS_ACTIVE_INTERFERE:
-                    ok = wide;
-                    tk = 2;
-                    nd = 1ull << (kk - 1);
-                    cost = 1;
-                    break;
-                case CLIFFT_OP_SWAP_MEAS_INTERFERE:
-                    ok = wide;
-                    tk = x1 != x2 ? 3 : 2;
-                    nd = (1ull << x1) | (1ull << x2);
-                    cost = tk == 3 ? 2 : 1;
-                    break;
-                default: ok = false;
+        // the block's plan and the fixed part of its micro-ops, from the host
+        const BlockPlan* bp = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset);
+        {
+            constexpr uint32_t HW = sizeof(BlockPlan) / 16, OW = sizeof(PlanOp) / 16;
+            const uint4* head = reinterpret_cast<const uint4*>(K.plan + plan_at);
+            const uint4* src = reinterpret_cast<const uint4*>(K.plan_ops + __ldg(&K.plan[plan_at].first_mop));
+            const uint32_t words = HW + OW * __ldg(&K.plan[plan_at].n_mops);
+            for (uint32_t i = Grp::rank(); i < words; i += Grp::size()) {
+                if (i < HW) {
+                    reinterpret_cast<uint4*>(fuse + TC::kPlanOffset)[i] = __ldg(head + i);
+                } else {
+                    // word 0, 1: the op; 2, 3: rows and columns of its index run,
+                    // kept in coefficient slots an index-map op does not use
+                    const uint32_t q = (i - HW) / OW, w = (i - HW) % OW;
+                    const uint4 x = __ldg(src + (i - HW));
+                    MOp* m = mops() + q;
+                    if (w < 2)
+                        reinterpret_cast<uint4*>(m)[w] = x;
+                    else
+                        run_words(*m)[w - 2] = x;
+                }
             }
-            if (!ok) break;
-            const uint64_t cand = need | nd;
-            if ((uint32_t)__popcll(cand) > MB || slots + cost > max_ops) break;
-            if (nd) {
-                uint32_t rr;
-                tile_axes(cand, rr);
-                if (MB - rr > (uint32_t)kMaxRunsLog2) break;
-            }
-            need = cand;
-            slots += cost;
-            if (expand_op) {
-                fresh |= 1ull << kk;
-                kk++;
-            } else if (cost && !tk) {
-                nsweep++;
-            }
-            if (tk) {
-                term = end++;
-                term_kind = tk;
-                break;
-            }
+            // warm the block's instructions (read one after another below)
+            const uint32_t ni = __ldg(&K.plan[plan_at].n_instr);
+            for (uint32_t i = Grp::rank(); i < ni; i += Grp::size()) touch(P.code + 2 * (plan_pc + i));
         }
-        // a block of EXPANDs alone costs more than the plain expansions
-        if (nsweep < 1 && !term_kind) return 0;
-        uint32_t r;
-        const uint64_t F = tile_axes(need, r);
-        const uint64_t C = ((kk == 64) ? ~0ull : ((1ull << kk) - 1)) & ~F;
-        uint8_t* lbit = reinterpret_cast<uint8_t*>(fuse + fuse_lbit_offset());
-        if (Grp::rank() == 0) {
-            uint32_t j = 0;
-            for (uint32_t a = 0; a < 64; ++a) lbit[a] = ((F >> a) & 1u) ? (uint8_t)j++ : (uint8_t)0xff;
-        }
-        uint32_t skip = 0;  // run-index bits of the new axes: those runs are made, not loaded
-        for (uint64_t w = fresh; w; w &= w - 1) {
-            const uint32_t a = (uint32_t)__ffsll((long long)w) - 1;
-            skip |= 1u << ((uint32_t)__popcll(F & ((1ull << a) - 1)) - r);
-        }
-        tileF = F;
-        set_runs(F, r);
         Grp::sync();
-        // resolve the block's frame-dependent choices into micro-ops
-        resolving = true;
+        const uint32_t pc = bp->pc, n_instr = bp->n_instr, r = bp->r, kk = bp->kk, skip = bp->skip;
+        const uint32_t term_kind = bp->term_kind;
+        const uint64_t F = bp->F, C = bp->C;
+        const bool single = Grp::kTeam && bp->single;
+        const uint32_t red_bit = bp->red_bit;
+        const bool red_local = bp->red_local != 0;
+        if (!single) set_runs(F, r);
+        plan_at++;
+        plan_pc = __ldg(&K.plan[plan_at].pc);
+        // resolve the block's frame-dependent choices
         n_mops = 0;
-        const uint32_t rend = term_kind ? term : end;
-        for (uint32_t q = pc; q < rend; ++q) exec(q);
-        const int n_body = n_mops;  // the micro-ops before a terminator's own
-        (void)n_body;
+        const uint32_t rend = term_kind ? bp->term_pc : pc + n_instr;
+        for (uint32_t q = pc; q < rend; ++q) exec<kResolve>(q, fetch(q));
+        const int nm = (int)bp->n_mops;
         uint32_t tfa = 0, tt = 0, tidx = 0;
         int tsign = 0;
-        bool red_local = false;
-        uint32_t red_bit = 0;
         if (term_kind) {
-            const uint4 w0 = __ldg(P.code + 2 * term);
-            cur_pc = term;
+            cur_pc = rend;
+            const uint4 w0 = fetch(rend);
             tfa = w0.y & 0xffffu;
             tt = term_kind == 3 ? (w0.y >> 16) : tfa;
             tidx = w0.z;
             tsign = (((w0.x >> 16) & 0xffu) & CLIFFT_FLAG_SIGN) ? 1 : 0;
-            if (term_kind == 3) emit(M_SWAP, tfa, tt, 0, 0, 0, nullptr, 0);
-            if (term_kind >= 2) emit(M_H, tt, tt, 0, 0, 0, nullptr, 0);
-            red_local = ((F >> tt) & 1u) != 0;
-            red_bit = red_local ? (uint32_t)__popcll(F & ((1ull << tt) - 1)) : tt;
         }
-        resolving = false;
         if constexpr (kDenseOk && WITH_DENSE) {
             Grp::sync();  // the resolved micro-ops, read by every thread
-            MOp* mm = reinterpret_cast<MOp*>(fuse + fuse_mops_offset());
+            MOp* mm = mops();
             uint32_t dmask = 0;
             int j1 = 0;
-            const int j0 = find_dense(mm, n_body, (int)K.dense_min_weight, local_mask(fresh), dmask, j1);
+            const int j0 = find_dense(mm, (int)bp->n_body, (int)K.dense_min_weight, bp->fresh_local, dmask, j1);
             if (j0 >= 0) {
                 if (Grp::rank() < 16)
                     compose_dense(mm, j0, j1, dmask, Grp::rank(),
@@ -2629,16 +2644,14 @@ struct Shot {
                     mm[j0].kind = M_DENSE;
                     mm[j0].req = dmask;
                     for (int j = j0 + 1; j < j1; ++j) mm[j].kind = M_NOP;
+                    // the dense run split some index runs: compile what is left
+                    compile_index_runs(mm, nm, (1u << MB) / (uint32_t)compute_threads());
                 }
             }
         }
-        if (Grp::rank() == 0)
-            compile_index_runs(reinterpret_cast<MOp*>(fuse + fuse_mops_offset()), n_mops,
-                               (1u << MB) / (uint32_t)compute_threads());
         Grp::sync();
-        const MOp* mops = reinterpret_cast<const MOp*>(fuse + fuse_mops_offset());
+        const MOp* mops = this->mops();
         const int tid = Grp::rank(), nthr = compute_threads();
-        const int nm = n_mops;
         cur_site = 6;
         constexpr uint32_t TN = 1u << MB;
         const uint32_t rpt = TN / (uint32_t)nthr;  // amplitudes per thread in a register-staged run
@@ -2649,11 +2662,11 @@ struct Shot {
         const int nmo = term_kind >= 2 ? nm - 1 : nm;
         auto body = [&](T* buf, uint64_t, uint64_t tbase) {
             for (int j = 0; j < nmo;) {
+                if (mops[j].kind == M_NOP) {
+                    ++j;
+                    continue;
+                }
                 if constexpr (kDenseOk && WITH_DENSE) {
-                    if (mops[j].kind == M_NOP) {
-                        ++j;
-                        continue;
-                    }
                     if (mops[j].kind == M_DENSE) {
                         apply_dense(mops[j].req, buf, tid);
                         csync();
@@ -2682,7 +2695,9 @@ struct Shot {
                 const uint32_t a = red_bit, ab = 1u << a;
                 const R s = (R)CGPU_INV_SQRT2;
                 double q0 = 0.0, q1 = 0.0;
-                for (uint32_t i = tid; i < (TN >> 1); i += nthr) {
+                // (a single tile may be filled only up to 2^kk: its top axis is measured)
+                const uint32_t half = single ? 1u << (kk - 1) : TN >> 1;
+                for (uint32_t i = tid; i < half; i += nthr) {
                     const uint32_t i0 = ins0_32(i, a);
                     const T x = buf[i0], y = buf[i0 | ab];
                     const T u = cscale(cadd(x, y), s), w = cscale(csub(x, y), s);
@@ -2697,7 +2712,8 @@ struct Shot {
                 // the measured axis' two half-norms of this tile
                 double q0 = 0.0, q1 = 0.0;
                 if (red_local) {
-                    for (uint32_t l = tid; l < TN; l += nthr) {
+                    const uint32_t filled = single ? 1u << kk : TN;
+                    for (uint32_t l = tid; l < filled; l += nthr) {
                         const double q = cnorm_d(buf[l]);
                         if ((l >> red_bit) & 1u)
                             q1 += q;
@@ -2716,26 +2732,33 @@ struct Shot {
             }
             csync();
         };
-        if constexpr (Grp::kWS)
-            stream_tiles_ws(1ull << (kk - MB), C, r, nm ? nruns : 0, skip, body);
-        else
-            stream_tiles(1ull << (kk - MB), C, r, 0, 0, nm ? nruns : 0, skip, body);
-        moved += (((1ull << kk) >> __popcll(fresh)) + (nm ? (1ull << kk) : 0ull)) * sizeof(T);
-        if constexpr (Grp::kTeam) {
-            if (!term_kind) team_sync();
+        if (single) {
+            // a team's private state: the tile is in its buffer already
+            if (tid < nthr) body(v, 0, 0);
+            __syncthreads();
+            moved += (nm ? (1ull << kk) : 0ull) * sizeof(T);
+        } else {
+            if constexpr (Grp::kWS)
+                stream_tiles_ws(1ull << (kk - MB), C, r, nm ? nruns : 0, skip, body);
+            else
+                stream_tiles(1ull << (kk - MB), C, r, 0, 0, nm ? nruns : 0, skip, body);
+            moved += (((1ull << kk) >> bp->n_fresh) + (nm ? (1ull << kk) : 0ull)) * sizeof(T);
+            if constexpr (Grp::kTeam) {
+                if (!term_kind) team_sync();
+            }
         }
         if (term_kind) {
             state_reduce<2>(acc);
             if (!stop) {
                 if (term_kind == 1) {
                     bytes += (1ull << k) * sizeof(T);
-                    diag_tail(tt, tidx, tsign, acc[0], acc[1], true);
+                    diag_tail(tt, tidx, tsign, acc[0], acc[1], !single);
                 } else {
-                    interfere_relabel(tfa, tt, tidx, tsign, acc[0], acc[1]);
+                    interfere_relabel(tfa, tt, tidx, tsign, acc[0], acc[1], !single);
                 }
             }
         }
-        return end - pc;
+        return n_instr;
     }
 
     // Micro-ops that map every amplitude to one position (CNOT, SWAP,
@@ -2766,13 +2789,16 @@ struct Shot {
         uint16_t row[3];
         uint8_t n, pad;
     };
-    static __device__ __forceinline__ RunRows* run_rows(MOp& m) { return reinterpret_cast<RunRows*>(&m.c[1]); }
+    // words 2 and 3 of a PlanOp: [RunRows, first column half][columns]; one
+    // 32-byte area behind the coefficient slot an index-map op may use
+    static __device__ __forceinline__ uint4* run_words(MOp& m) { return reinterpret_cast<uint4*>(&m.c[2]); }
+    static __device__ __forceinline__ RunRows* run_rows(MOp& m) { return reinterpret_cast<RunRows*>(&m.c[2]); }
     static __device__ __forceinline__ const RunRows* run_rows(const MOp& m) {
-        return reinterpret_cast<const RunRows*>(&m.c[1]);
+        return reinterpret_cast<const RunRows*>(&m.c[2]);
     }
-    static __device__ __forceinline__ uint16_t* run_cols(MOp& m) { return reinterpret_cast<uint16_t*>(&m.c[4]); }
+    static __device__ __forceinline__ uint16_t* run_cols(MOp& m) { return reinterpret_cast<uint16_t*>(&m.c[2]) + 4; }
     static __device__ __forceinline__ const uint16_t* run_cols(const MOp& m) {
-        return reinterpret_cast<const uint16_t*>(&m.c[4]);
+        return reinterpret_cast<const uint16_t*>(&m.c[2]) + 4;
     }
     // Compiles every run the tile loop will stage (the same boundaries: at
     // least two consecutive index-map ops and rpt <= kMaxRunAmps). Run by one
@@ -3293,10 +3319,9 @@ struct Shot {
         if (tid == 0) slot[3] = state ^ 1u;  // read by the next call after the caller's barrier
     }
 
-    // Whether instruction pc touches the statevector (needs every thread of a
+    // Whether an instruction touches the statevector (needs every thread of a
     // CTA group) or only scalar state (frame, gamma, records, noise cursor).
-    __device__ __forceinline__ bool needs_all(uint32_t pc) const {
-        const uint4 w0 = __ldg(P.code + 2 * pc);
+    __device__ __forceinline__ bool needs_all(const uint4& w0) const {
         uint32_t op = w0.x & 0xffu;
         const uint32_t a1 = w0.y & 0xffffu;
         if (op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
@@ -3381,11 +3406,11 @@ struct Shot {
         return c->pc | (c->cmd << 31);
     }
     // a statevector step executed by every thread (fused block or one opcode)
-    __device__ __forceinline__ uint32_t run_all(uint32_t pc, bool fuse_on) {
+    __device__ __forceinline__ uint32_t run_all(uint32_t pc) {
         uint32_t used = 0;
-        if (tiled(k)) used = run_block(pc, fuse_on ? TC::kMops : 1, P.n_code);
+        if constexpr (kTiles) used = run_block(pc);
         if (!used) {
-            exec(pc);
+            exec<kState>(pc, fetch(pc));
             used = 1;
         }
         return used;
@@ -3393,7 +3418,7 @@ struct Shot {
     // CTA groups: warp 0 interprets the bytecode; the other warps join only
     // for statevector steps, receiving the scalar state through shared memory.
     // Every CTA-wide barrier is reached by all warps at the same program point.
-    __device__ void run_cta(bool fuse_on, bool prof) {
+    __device__ void run_cta(bool prof) {
         const uint32_t n_instr = P.n_code;
         const bool ctrl = (threadIdx.x >> 5) == 0;
         uint32_t pc = 0;
@@ -3403,8 +3428,10 @@ struct Shot {
                 const long long c0 = prof ? clock64() : 0;
                 while (pc < n_instr && !stop) {
                     pc = frame_run(pc, n_instr);
-                    if (pc >= n_instr || needs_all(pc)) break;
-                    exec(pc);
+                    if (pc >= n_instr) break;
+                    const uint4 w0 = fetch(pc);
+                    if (needs_all(w0)) break;
+                    exec<kScalar>(pc, w0);
                     ++pc;
                 }
                 flush_records();
@@ -3421,7 +3448,7 @@ struct Shot {
             solo = false;
             if (word >> 31) break;
             const long long c1 = prof ? clock64() : 0;
-            const uint32_t used = run_all(word, fuse_on);
+            const uint32_t used = run_all(word);
             enter_private();
             __syncthreads();
             if (prof) {
@@ -3441,19 +3468,19 @@ struct Shot {
     // ------------------------------------------------------------ driver
     __device__ __forceinline__ void run(Tally& tally) {
         const bool seg = (K.seg_flags & KSEG_ON) != 0;
+        win_pc = 0x80000000u;  // no window yet
         if (seg && !(K.seg_flags & KSEG_FIRST)) {
             load_state();
         } else {
             reset();
         }
+        plan_start(seg ? K.seg_begin : 0);
         const uint32_t n_instr = P.n_code;
-        const bool fuse_on = Grp::kCta && (K.flags & KF_FUSE) != 0;
         const bool prof = K.phase_cycles != nullptr && Grp::rank() == 0 && leader();
         if (Grp::kCta) {
-            run_cta(fuse_on, prof);
+            run_cta(prof);
         } else {
             const uint32_t end = seg ? K.seg_end : n_instr;
-            const int max_ops = (K.flags & KF_FUSE) ? TC::kMops : 1;
             for (uint32_t pc = seg ? K.seg_begin : 0; pc < end;) {
                 pc = frame_run(pc, end);
                 if (pc >= end) break;
@@ -3461,10 +3488,10 @@ struct Shot {
                 if constexpr (kTiles) {
                     // a warp running one shot streams its global statevector
                     // through the tile engine like a CTA group
-                    if (tiled(k)) used = run_block(pc, max_ops, end);
+                    used = run_block(pc);
                 }
                 if (!used) {
-                    exec(pc);
+                    exec<kAll>(pc, fetch(pc));
                     used = 1;
                 }
                 pc += used;
@@ -3524,7 +3551,6 @@ struct Shot {
     }
     __device__ __forceinline__ void load_state() {
         xo = 0;  // amplitudes come back in logical order
-        tileF = 0;
         const unsigned char* d = K.seg_state + shot * K.seg_stride;
         const uint64_t* w = reinterpret_cast<const uint64_t*>(d);
 #pragma unroll
@@ -3550,7 +3576,6 @@ struct Shot {
         stop = false;
         discarded = (q[7] & 2u) != 0;
         reachable = (q[7] & 4u) != 0;
-        resolving = false;
         solo = false;
         n_mops = 0;
         rec_dirty = false;
@@ -3569,7 +3594,6 @@ struct Shot {
         // SchrodingerState::reset (svm_state.cc:220-267): only v[0] needs a
         // value; every other amplitude is written by EXPAND before it is read.
         xo = 0;
-        tileF = 0;
         if constexpr (Grp::kTeam) {
             v = reinterpret_cast<T*>(fuse + TC::kBufOffset);
             priv = true;
@@ -3585,7 +3609,6 @@ struct Shot {
         dust = 0;
         bytes = 0;
         moved = 0;
-        resolving = false;
         solo = false;
         n_mops = 0;
         rec_dirty = false;
@@ -3597,7 +3620,7 @@ struct Shot {
         if (meas_prob && leader())
             for (uint32_t i = Grp::rank(); i < P.slots; i += Grp::size())
                 meas_prob[i] = __longlong_as_double(0x7ff8000000000000ll);
-        if (Grp::rank() == 0) A(0) = Cx<R>::make(1.0, 0.0);
+        if (Grp::rank() == 0) A(0u) = Cx<R>::make(1.0, 0.0);
         if (K.flags & KF_FORCED_FAULTS) {
             ff_pos = K.fault_off[shot];
             ff_end = K.fault_end ? K.fault_end[shot] : K.fault_off[shot + 1];
