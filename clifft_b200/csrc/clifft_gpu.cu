@@ -24,6 +24,7 @@
 #include "svm_dispatch.h"
 #include "svm_grad.h"
 #include "svm_kernel.cuh"
+#include "svm_phase_grad.h"
 #include "svm_plan.h"
 #include "svm_sample_k.h"
 
@@ -389,6 +390,19 @@ struct clifft_gpu_program {
         const PlanOp* ops = nullptr;
     };
     std::map<std::tuple<uint32_t, bool, bool, bool>, Plans> plans;  // under plan_mu
+    // what every gradient call of the program needs, uploaded by the first one
+    struct Gradient {
+        void* dev = nullptr;
+        uint32_t n_exp = 0;
+        const int32_t* rot_index = nullptr;
+        const uint32_t* exp_pc = nullptr;
+        const uint32_t* exp_out = nullptr;
+        bool phase_polynomial = false;  // the one-pass kernel applies (svm_phase_grad.cu) ...
+        bool unit_payloads = false;     // ... to the program's own rotations too
+        uint32_t max_k = 0, max_probes = 0;
+        PhaseParams phase{};
+    };
+    Gradient gradient;  // under plan_mu
     // Statevector slab kept between calls (mapping tens of GB afresh on every
     // call costs more than a large-k launch's own setup). One call at a time
     // holds it; a concurrent call on the same handle allocates its own.
@@ -1173,6 +1187,7 @@ void clifft_gpu_free(clifft_gpu_program* prog) {
         if (prog->blob) cudaFree(prog->blob);
         for (auto& e : prog->plans)
             if (e.second.dev) cudaFree(e.second.dev);
+        if (prog->gradient.dev) cudaFree(prog->gradient.dev);
         if (prog->slab) cudaFree(prog->slab);
     }
     delete prog;
@@ -2005,6 +2020,93 @@ bool grad_supported(uint32_t op) {
     }
 }
 
+// Checks that the program has gradients (measurement-free, noise-free,
+// rotations as ARRAY_ROT / EXPAND_ROT) and returns what a call needs of it,
+// uploaded once per program.
+clifft_gpu_program::Gradient gradient_plan(clifft_gpu_program& p) {
+    std::lock_guard<std::mutex> lock(p.plan_mu);
+    auto& g = p.gradient;
+    if (g.dev) return g;
+    const clifft_program_image& m = p.meta;
+    const uint32_t n = m.num_instructions;
+    std::vector<int32_t> rot_index(n, -1);
+    std::vector<uint32_t> exp_pc, exp_out;
+    std::vector<uint8_t> seen_out(m.num_exp_vals, 0);
+    uint32_t np = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint8_t* ins = p.instr_host.data() + size_t(i) * 32;
+        const uint32_t op = ins[0];
+        if (!grad_supported(op)) {
+            std::string why = (op == CLIFFT_OP_ARRAY_U2 || op == CLIFFT_OP_ARRAY_U4)
+                                  ? " (fused U2 / U4 nodes hide the rotation angles: compile gradient "
+                                    "programs without the single-axis / tile-axis fusion passes)"
+                                  : "";
+            invalid("clifft_gpu_expval_grad needs a measurement-free, noise-free program: instruction " +
+                    std::to_string(i) + " is " + opcode_name(op) + why);
+        }
+        if (op == CLIFFT_OP_ARRAY_ROT || op == CLIFFT_OP_EXPAND_ROT) rot_index[i] = int32_t(np++);
+        if (op == CLIFFT_OP_EXP_VAL) {
+            uint32_t out_idx = 0;
+            std::memcpy(&out_idx, ins + 12, 4);
+            if (out_idx >= m.num_exp_vals || seen_out[out_idx]) invalid("EXP_VAL output rows must be distinct");
+            seen_out[out_idx] = 1;
+            exp_pc.push_back(i);
+            exp_out.push_back(out_idx);
+        }
+    }
+    if (np != p.num_rot_params) invalid("internal: rotation count mismatch");
+    if (exp_pc.empty()) return g;
+    PhasePlan plan;
+    const bool phase = build_phase_plan(p.instr_host.data(), n, plan);
+    BlobBuilder b;
+    const size_t o_rot = b.put(rot_index.data(), rot_index.size());
+    const size_t o_pc = b.put(exp_pc.data(), exp_pc.size());
+    const size_t o_out = b.put(exp_out.data(), exp_out.size());
+    const size_t o_stage = b.put(plan.stages.data(), plan.stages.size());
+    const size_t o_mask = b.put(plan.factor_mask.data(), plan.factor_mask.size());
+    const size_t o_begin = b.put(plan.term_begin.data(), plan.term_begin.size());
+    const size_t o_term = b.put(plan.terms.data(), plan.terms.size());
+    const size_t o_cz = b.put(plan.cz.data(), plan.cz.size());
+    const size_t o_probe = b.put(plan.probes.data(), plan.probes.size());
+    const size_t o_param = b.put(plan.param_mask.data(), plan.param_mask.size());
+    CUDA_OK(cudaSetDevice(p.device));
+    void* dev = nullptr;
+    CUDA_OK(alloc_retry([&] { return cudaMalloc(&dev, b.bytes.size() + 16); }));
+    const cudaError_t up = cudaMemcpy(dev, b.bytes.data(), b.bytes.size(), cudaMemcpyHostToDevice);
+    if (up != cudaSuccess) cudaFree(dev);
+    CUDA_OK(up);
+    g.n_exp = uint32_t(exp_pc.size());
+    g.rot_index = at<int32_t>(dev, o_rot);
+    g.exp_pc = at<uint32_t>(dev, o_pc);
+    g.exp_out = at<uint32_t>(dev, o_out);
+    g.phase_polynomial = phase;
+    g.unit_payloads = plan.unit_payloads;
+    g.max_k = plan.max_k;
+    for (const PhaseStage& s : plan.stages) g.max_probes = std::max(g.max_probes, s.n_probes);
+    g.phase.n_out = m.num_exp_vals;
+    g.phase.n_params = np;
+    g.phase.n_stages = uint32_t(plan.stages.size());
+    g.phase.stages = at<PhaseStage>(dev, o_stage);
+    g.phase.factor_mask = at<uint32_t>(dev, o_mask);
+    g.phase.term_begin = at<uint32_t>(dev, o_begin);
+    g.phase.terms = at<PhaseTerm>(dev, o_term);
+    g.phase.cz = at<uint32_t>(dev, o_cz);
+    g.phase.probes = at<PhaseProbe>(dev, o_probe);
+    g.phase.param_mask = at<uint32_t>(dev, o_param);
+    g.dev = dev;
+    return g;
+}
+
+// Dynamic shared memory limit of a kernel; only ever raised.
+void raise_smem_limit(const void* fn, uint32_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes cur{};
+    CUDA_OK(cudaFuncGetAttributes(&cur, fn));
+    if (cur.maxDynamicSharedSizeBytes < int(bytes))
+        CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+}
+
 }  // namespace
 
 extern "C" {
@@ -2021,38 +2123,13 @@ int clifft_gpu_expval_grad(clifft_gpu_program* prog, const clifft_gpu_grad_args*
         if (args->precision != CLIFFT_GPU_FP32 && args->precision != CLIFFT_GPU_FP64)
             invalid("precision must be CLIFFT_GPU_FP32 or CLIFFT_GPU_FP64");
         const bool dev_ptrs = (args->flags & CLIFFT_GPU_DEVICE_PTRS) != 0;
-        // the program: measurement-free, noise-free, rotations as ARRAY_ROT / EXPAND_ROT
-        const uint32_t n = m.num_instructions;
-        std::vector<int32_t> rot_index(n, -1);
-        std::vector<uint32_t> exp_pc, exp_out;
-        std::vector<uint8_t> seen_out(m.num_exp_vals, 0);
-        uint32_t np = 0;
-        for (uint32_t i = 0; i < n; ++i) {
-            const uint8_t* ins = prog->instr_host.data() + size_t(i) * 32;
-            const uint32_t op = ins[0];
-            if (!grad_supported(op)) {
-                std::string why = (op == CLIFFT_OP_ARRAY_U2 || op == CLIFFT_OP_ARRAY_U4)
-                                      ? " (fused U2 / U4 nodes hide the rotation angles: compile gradient "
-                                        "programs without the single-axis / tile-axis fusion passes)"
-                                      : "";
-                invalid("clifft_gpu_expval_grad needs a measurement-free, noise-free program: instruction " +
-                        std::to_string(i) + " is " + opcode_name(op) + why);
-            }
-            if (op == CLIFFT_OP_ARRAY_ROT || op == CLIFFT_OP_EXPAND_ROT) rot_index[i] = int32_t(np++);
-            if (op == CLIFFT_OP_EXP_VAL) {
-                uint32_t out_idx = 0;
-                std::memcpy(&out_idx, ins + 12, 4);
-                if (out_idx >= m.num_exp_vals || seen_out[out_idx]) invalid("EXP_VAL output rows must be distinct");
-                seen_out[out_idx] = 1;
-                exp_pc.push_back(i);
-                exp_out.push_back(out_idx);
-            }
-        }
-        if (np != prog->num_rot_params) invalid("internal: rotation count mismatch");
+        const clifft_gpu_program::Gradient gr = gradient_plan(*prog);
+        const uint32_t np = prog->num_rot_params;
         const uint64_t batch = args->batch;
-        if (batch == 0 || exp_pc.empty()) return;
+        if (batch == 0 || gr.n_exp == 0) return;
         if (np > 0 && !grads) invalid("grads output is null");
         CUDA_OK(cudaSetDevice(prog->device));
+        keep_pool_memory(prog->device);
         cudaStream_t st = static_cast<cudaStream_t>(args->stream);
         StreamBuffers buf(st);
         auto up = [&](const void* src, size_t bytes) -> void* {
@@ -2060,29 +2137,72 @@ int clifft_gpu_expval_grad(clifft_gpu_program* prog, const clifft_gpu_grad_args*
             if (d) CUDA_OK(cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, st));
             return d;
         };
+        const double* phases = nullptr;
+        if (args->phases && np)
+            phases = dev_ptrs ? args->phases
+                              : static_cast<const double*>(up(args->phases, size_t(batch) * np * 8));
+        const size_t out_e = size_t(batch) * m.num_exp_vals * 8, out_g = size_t(batch) * m.num_exp_vals * np * 8;
+        double* d_exp = dev_ptrs ? exp_vals : static_cast<double*>(buf.alloc(out_e));
+        double* d_grad = dev_ptrs ? grads : static_cast<double*>(buf.alloc(std::max<size_t>(out_g, 8)));
+        // rows of EXP_VAL outputs no instruction writes stay zero
+        if (gr.n_exp < m.num_exp_vals) {
+            CUDA_OK(cudaMemsetAsync(d_exp, 0, out_e, st));
+            if (out_g) CUDA_OK(cudaMemsetAsync(d_grad, 0, out_g, st));
+        }
+        auto finish = [&] {
+            if (!dev_ptrs) {
+                CUDA_OK(cudaMemcpyAsync(exp_vals, d_exp, out_e, cudaMemcpyDeviceToHost, st));
+                if (out_g) CUDA_OK(cudaMemcpyAsync(grads, d_grad, out_g, cudaMemcpyDeviceToHost, st));
+            }
+            CUDA_OK(cudaStreamSynchronize(st));
+        };
+        int sms = 0;
+        CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, prog->device));
+        // FP64 programs without ARRAY_H whose phases are unit phases: one pass
+        // per (vector, EXP_VAL). FP32 keeps the general kernel's FP32 state.
+        if (args->precision == CLIFFT_GPU_FP64 && gr.phase_polynomial && (phases || gr.unit_payloads)) {
+            PhaseParams G = gr.phase;
+            G.batch = batch;
+            G.phases = phases;
+            G.out_exp = d_exp;
+            G.out_grad = d_grad;
+            PhaseGradFn fn = phase_grad_kernel_fn(gr.max_k);
+            const uint32_t smem = phase_grad_smem(gr.max_k);
+            raise_smem_limit((const void*)fn, smem);
+            int per_sm = 0;
+            CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kPhaseThreads, smem));
+            const uint64_t slots = uint64_t(std::max(per_sm, 1)) * sms, units = batch * G.n_stages;
+            // CTAs per (vector, stage): building the state costs about two
+            // probes, so the split that leaves the shortest sequence of them
+            uint64_t best = ~0ull;
+            for (uint32_t c = 1; c <= gr.max_probes; ++c) {
+                const uint64_t t = ((units * c + slots - 1) / slots) * (2 + (gr.max_probes + c - 1) / c);
+                if (t < best) {
+                    best = t;
+                    G.splits = c;
+                }
+            }
+            if (units * G.splits > 0x7fffffffull) invalid("gradient batch too large; split the call");
+            fn<<<unsigned(units * G.splits), kPhaseThreads, smem, st>>>(prog->dev, G);
+            CUDA_OK(cudaGetLastError());
+            finish();
+            return;
+        }
         GradParams G{};
         G.batch = batch;
-        G.n_exp = uint32_t(exp_pc.size());
+        G.n_exp = gr.n_exp;
         G.n_out = m.num_exp_vals;
         G.n_params = np;
-        G.rot_index = static_cast<const int32_t*>(up(rot_index.data(), rot_index.size() * 4));
-        G.exp_pc = static_cast<const uint32_t*>(up(exp_pc.data(), exp_pc.size() * 4));
-        G.exp_out = static_cast<const uint32_t*>(up(exp_out.data(), exp_out.size() * 4));
-        if (args->phases && np) {
-            G.phases = dev_ptrs ? args->phases
-                                : static_cast<const double*>(up(args->phases, size_t(batch) * np * 8));
-        }
-        const size_t out_e = size_t(batch) * m.num_exp_vals * 8, out_g = size_t(batch) * m.num_exp_vals * np * 8;
-        G.out_exp = dev_ptrs ? exp_vals : static_cast<double*>(buf.alloc(out_e));
-        G.out_grad = dev_ptrs ? grads : static_cast<double*>(buf.alloc(std::max<size_t>(out_g, 8)));
-        // rows of EXP_VAL outputs no instruction writes stay zero
-        CUDA_OK(cudaMemsetAsync(G.out_exp, 0, out_e, st));
-        if (out_g) CUDA_OK(cudaMemsetAsync(G.out_grad, 0, out_g, st));
+        G.rot_index = gr.rot_index;
+        G.exp_pc = gr.exp_pc;
+        G.exp_out = gr.exp_out;
+        G.phases = phases;
+        G.out_exp = d_exp;
+        G.out_grad = d_grad;
         const bool fp32 = args->precision == CLIFFT_GPU_FP32;
         ExpvalGradFn fn = expval_grad_kernel_fn(fp32);
-        int per_sm = 0, sms = 0;
+        int per_sm = 0;
         CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExpvalGradThreads, 0));
-        CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, prog->device));
         const uint64_t tasks = batch * G.n_exp;
         G.stride = uint64_t(1) << m.peak_rank;
         const size_t amp = fp32 ? 8 : 16;
@@ -2096,11 +2216,7 @@ int clifft_gpu_expval_grad(clifft_gpu_program* prog, const clifft_gpu_grad_args*
         G.work = work;
         fn<<<unsigned(blocks), kExpvalGradThreads, 0, st>>>(prog->dev, G);
         CUDA_OK(cudaGetLastError());
-        if (!dev_ptrs) {
-            CUDA_OK(cudaMemcpyAsync(exp_vals, G.out_exp, out_e, cudaMemcpyDeviceToHost, st));
-            if (out_g) CUDA_OK(cudaMemcpyAsync(grads, G.out_grad, out_g, cudaMemcpyDeviceToHost, st));
-        }
-        CUDA_OK(cudaStreamSynchronize(st));
+        finish();
     });
 }
 

@@ -1,0 +1,354 @@
+// svm_phase_grad.cu -- gradients of expectation values without walking back.
+//
+// In a measurement-free program without ARRAY_H every opcode multiplies
+// amplitudes by phases (T, S, ROT, CZ), permutes them (CNOT, SWAP) or opens an
+// axis (EXPAND: the lower half copied to the upper half, times a phase), and
+// the Pauli frame stays the identity. Then
+//   * the state is v[i] = prod_f F_f^{parity(i & mask_f)} (times CZ signs), with
+//     the masks pulled back through the permutations: no pass over a
+//     statevector is needed to build it;
+//   * w = conj(lambda) v, lambda = O v, is what a reverse walk carries: diagonal
+//     opcodes leave it as it is, permutations permute it, undoing an EXPAND
+//     adds its two halves. So the derivative with respect to the phase of a
+//     rotation on the axis with pulled-back mask m,
+//         -2 Im( sum over parity(i & m) odd of w[i] ) / <v|v>,
+//     is a difference of two Walsh-Hadamard coefficients of Im w:
+//         (W(m) - W(0)) / <v|v>.
+// The general kernel (svm_grad.cu) ran the program forward and backward once
+// per (vector, EXP_VAL); this one builds the state once per vector and spends
+// one transform per EXP_VAL. 256 vectors, 32 rotations, 16 probes, k = 13:
+// the whole call with its torch autograd 2.5 -> 0.36 ms, of which the kernel
+// 0.15 ms. What bounds the kernel: FP64 and shared-memory traffic of the
+// transforms, one CTA of 16 warps per SM (192 KiB).
+//
+// A transform runs over the top k - 9 axes in registers (a thread holds the
+// 2^(k-9) indices that agree in the low 9 bits), over axes 5..8 in registers
+// again after one exchange through shared memory, and over axes 0..4 only for
+// the coefficients that are read: one warp reduction each.
+
+#include "svm_phase_grad.h"
+
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <cstring>
+#include <map>
+
+#include "svm_kernel.cuh"
+
+namespace cgpu {
+
+namespace {
+
+constexpr int NT = kPhaseThreads;
+constexpr uint32_t kLowBits = 9;  // log2(NT)
+
+template <int NQ>
+__device__ __forceinline__ void butterflies(double (&x)[NQ]) {
+#pragma unroll
+    for (int h = 1; h < NQ; h <<= 1)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            if (!(q & h)) {
+                const double a = x[q], b = x[q | h];
+                x[q] = a + b;
+                x[q | h] = a - b;
+            }
+}
+
+// axes 5 .. 5 + log2(NB) - 1 of the 2^k values in ws
+template <int NB>
+__device__ __forceinline__ void middle_axes(double* ws, uint32_t k) {
+    const uint32_t units = (1u << k) / NB;
+    for (uint32_t u = threadIdx.x; u < units; u += NT) {
+        double* p = ws + (u >> 5) * (32u * NB) + (u & 31u);
+        double x[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) x[q] = p[32 * q];
+        butterflies(x);
+#pragma unroll
+        for (int q = 0; q < NB; ++q) p[32 * q] = x[q];
+    }
+}
+
+// sum over the low five axes of row `mask >> 5`, with the sign of the mask
+__device__ __forceinline__ double coefficient(const double* ws, uint32_t k, uint32_t mask) {
+    const uint32_t lane = threadIdx.x & 31u;
+    double x = 0.0;
+    if (lane < (1u << k)) {
+        x = ws[(mask & ~31u) + lane];
+        if (__popc(mask & lane) & 1) x = -x;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// fixed-order sum over the CTA, the same bits in every thread
+__device__ __forceinline__ double cta_sum(double x, double* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) t += red[i];
+    return t;
+}
+
+// NQ: indices per thread at the largest k of the plan
+template <int NQ>
+__global__ void __launch_bounds__(NT) phase_grad_kernel(const DevProg P, const PhaseParams G) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint64_t task = blockIdx.x;
+    const uint32_t split = (uint32_t)(task % G.splits);
+    const uint32_t si = (uint32_t)(task / G.splits % G.n_stages);
+    const uint64_t row = task / G.splits / G.n_stages;
+    const PhaseStage S = G.stages[si];
+    const uint32_t first = (uint32_t)((uint64_t)S.n_probes * split / G.splits);
+    const uint32_t last = (uint32_t)((uint64_t)S.n_probes * (split + 1) / G.splits);
+    if (first == last) return;
+    const uint32_t k = S.k, dim = 1u << k, tid = threadIdx.x;
+    double2* vs = reinterpret_cast<double2*>(smem);
+    double* ws = reinterpret_cast<double*>(vs + dim);
+    double2* term = reinterpret_cast<double2*>(ws + dim);
+    double2* factor = term + kPhaseMaxTerms;
+    double* red = reinterpret_cast<double*>(factor + kPhaseMaxTerms);
+    // the stage's phases, then their products per mask
+    const uint32_t t0 = G.term_begin[S.factor0], nt = G.term_begin[S.factor0 + S.n_factors] - t0;
+    for (uint32_t i = tid; i < nt; i += NT) {
+        const PhaseTerm t = G.terms[t0 + i];
+        double2 ph = make_double2(t.re, t.im);
+        if (t.param >= 0 && G.phases) sincos(G.phases[row * G.n_params + (uint32_t)t.param], &ph.y, &ph.x);
+        term[i] = ph;
+    }
+    __syncthreads();
+    for (uint32_t f = tid; f < S.n_factors; f += NT) {
+        const uint32_t b = G.term_begin[S.factor0 + f] - t0, e = G.term_begin[S.factor0 + f + 1] - t0;
+        double2 x = term[b];
+        for (uint32_t i = b + 1; i < e; ++i) x = dmul(x, term[i]);
+        factor[f] = x;
+    }
+    __syncthreads();
+    // v at this thread's indices i = tid + q * NT
+    double2 v[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = make_double2(1.0, 0.0);
+    for (uint32_t f = 0; f < S.n_factors; ++f) {
+        const uint32_t m = __ldg(G.factor_mask + S.factor0 + f);
+        const double2 ph = factor[f];
+        const uint32_t low = (uint32_t)__popc(m & tid) & 1u;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            if (((uint32_t)__popc((m >> kLowBits) & (uint32_t)q) ^ low) & 1u) v[q] = dmul(v[q], ph);
+    }
+    for (uint32_t c = 0; c < S.n_cz; ++c) {
+        const uint32_t m0 = __ldg(G.cz + 2 * (S.cz0 + c)), m1 = __ldg(G.cz + 2 * (S.cz0 + c) + 1);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const uint32_t i = tid + (uint32_t)q * NT;
+            if (__popc(m0 & i) & __popc(m1 & i) & 1) v[q] = make_double2(-v[q].x, -v[q].y);
+        }
+    }
+    double n2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const uint32_t i = tid + (uint32_t)q * NT;
+        if (i < dim) {
+            vs[i] = v[q];
+            n2 += v[q].x * v[q].x + v[q].y * v[q].y;
+        }
+    }
+    const double norm = cta_sum(n2, red), inv_norm = 1.0 / norm;  // (its barriers publish vs)
+    for (uint32_t p = first; p < last; ++p) {
+        const PhaseProbe pr = G.probes[S.probe0 + p];
+        const uint64_t* mx = P.exp_x + (size_t)pr.mask * P.nw;
+        const uint64_t* mz = P.exp_z + (size_t)pr.mask * P.nw;
+        bool dormant = (mx[0] >> k) != 0;
+        for (uint32_t w = 1; w < P.nw; ++w) dormant |= mx[w] != 0;
+        double* grow = G.out_grad + (row * G.n_out + pr.row) * (size_t)G.n_params;
+        if (dormant) {  // X / Y support on a dormant axis: the value and every derivative are 0
+            if (tid == 0) G.out_exp[row * G.n_out + pr.row] = 0.0;
+            for (uint32_t j = tid; j < G.n_params; j += NT) grow[j] = 0.0;
+            continue;
+        }
+        const uint32_t xa = (uint32_t)mx[0] & (dim - 1), za = (uint32_t)mz[0] & (dim - 1);
+        const int yz = (__popc(xa & za) + (P.exp_sign[pr.mask] ? 2 : 0)) & 3;  // lambda = i^yz (-1)^.. v
+        // w = conj(i^yz) (-1)^{parity((i ^ xa) & za)} conj(v[i ^ xa]) v[i]
+        double x[NQ], re = 0.0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const uint32_t i = tid + (uint32_t)q * NT;
+            x[q] = 0.0;
+            if (i < dim) {
+                const double2 u = vs[i ^ xa];
+                double wr = u.x * v[q].x + u.y * v[q].y, wi = u.x * v[q].y - u.y * v[q].x;
+                if (yz & 1) {  // times -i
+                    const double t = wr;
+                    wr = wi;
+                    wi = -t;
+                }
+                if ((((uint32_t)yz >> 1) ^ (uint32_t)__popc((i ^ xa) & za)) & 1u) {
+                    wr = -wr;
+                    wi = -wi;
+                }
+                re += wr;
+                x[q] = wi;
+            }
+        }
+        butterflies(x);
+        const double value = cta_sum(re, red);  // (its first barrier: the previous probe's readers of ws are done)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const uint32_t i = tid + (uint32_t)q * NT;
+            if (i < dim) ws[i] = x[q];
+        }
+        __syncthreads();
+        if (k >= 9)
+            middle_axes<16>(ws, k);
+        else if (k == 8)
+            middle_axes<8>(ws, k);
+        else if (k == 7)
+            middle_axes<4>(ws, k);
+        else if (k == 6)
+            middle_axes<2>(ws, k);
+        __syncthreads();
+        if (tid == 0) G.out_exp[row * G.n_out + pr.row] = fmin(1.0, fmax(-1.0, value * inv_norm));
+        const double w0 = coefficient(ws, k, 0);
+        for (uint32_t j = tid >> 5; j < G.n_params; j += NT / 32) {
+            const uint32_t m = __ldg(G.param_mask + S.param0 + j);
+            const double g = m ? (coefficient(ws, k, m) - w0) * inv_norm : 0.0;
+            if ((tid & 31u) == 0) grow[j] = g;
+        }
+    }
+}
+
+}  // namespace
+
+PhaseGradFn phase_grad_kernel_fn(uint32_t max_k) {
+    switch (max_k > kLowBits ? max_k - kLowBits : 0) {
+        case 0: return phase_grad_kernel<1>;
+        case 1: return phase_grad_kernel<2>;
+        case 2: return phase_grad_kernel<4>;
+        case 3: return phase_grad_kernel<8>;
+        default: return phase_grad_kernel<16>;
+    }
+}
+
+bool build_phase_plan(const uint8_t* code, uint32_t n, PhasePlan& out) {
+    out = PhasePlan{};
+    auto op_of = [&](uint32_t pc) { return uint32_t(code[size_t(pc) * 32]); };
+    auto read = [&](uint32_t pc, uint32_t off, auto& x) { std::memcpy(&x, code + size_t(pc) * 32 + off, sizeof x); };
+    auto changes_state = [&](uint32_t op) { return op >= CLIFFT_OP_ARRAY_CNOT && op <= CLIFFT_OP_EXPAND_ROT; };
+    auto is_expand = [&](uint32_t op) { return op >= CLIFFT_OP_EXPAND && op <= CLIFFT_OP_EXPAND_ROT; };
+    std::vector<int32_t> param(n, -1);
+    std::vector<uint32_t> rank(n);  // before each instruction
+    uint32_t np = 0, k = 0;
+    for (uint32_t pc = 0; pc < n; ++pc) {
+        const uint32_t op = op_of(pc);
+        if (op == CLIFFT_OP_ARRAY_H) return false;
+        rank[pc] = k;
+        if (op == CLIFFT_OP_ARRAY_ROT || op == CLIFFT_OP_EXPAND_ROT) {
+            param[pc] = int32_t(np++);
+            double c, s;
+            read(pc, 8, c);
+            read(pc, 16, s);
+            if (!(std::fabs(c * c + s * s - 1.0) < 1e-12)) out.unit_payloads = false;
+        }
+        if (is_expand(op)) ++k;
+    }
+    out.term_begin.push_back(0);
+    for (uint32_t pc = 0; pc < n; ++pc) {
+        if (op_of(pc) != CLIFFT_OP_EXP_VAL) continue;
+        // every EXP_VAL up to the next change of the state reads the same stage
+        PhaseStage s{};
+        s.k = rank[pc];
+        if (s.k > kPhaseMaxK) return false;
+        s.probe0 = uint32_t(out.probes.size());
+        uint32_t end = pc;
+        for (; end < n && !changes_state(op_of(end)); ++end)
+            if (op_of(end) == CLIFFT_OP_EXP_VAL) {
+                PhaseProbe p{};
+                read(end, 8, p.mask);
+                read(end, 12, p.row);
+                out.probes.push_back(p);
+            }
+        s.n_probes = uint32_t(out.probes.size()) - s.probe0;
+        s.param0 = uint32_t(out.param_mask.size());
+        out.param_mask.resize(out.param_mask.size() + np, 0u);
+        s.cz0 = uint32_t(out.cz.size() / 2);
+        // walk back from here: row[a] = axis a of the index at that time, as a
+        // parity of bits of the index here
+        std::vector<uint32_t> row(s.k);
+        for (uint32_t a = 0; a < s.k; ++a) row[a] = 1u << a;
+        std::map<uint32_t, std::vector<PhaseTerm>> factors;
+        auto phase = [&](uint32_t at, uint32_t mask, double re, double im) {
+            factors[mask].push_back(PhaseTerm{re, im, param[at], 0});
+            if (param[at] >= 0) out.param_mask[s.param0 + uint32_t(param[at])] = mask;
+        };
+        const double r = CGPU_INV_SQRT2;
+        for (uint32_t q = pc; q-- > 0;) {
+            const uint32_t op = op_of(q), kq = rank[q];
+            uint16_t a, b;
+            uint64_t mask;
+            double c, sn;
+            read(q, 4, a);
+            read(q, 6, b);
+            read(q, 8, mask);
+            read(q, 8, c);
+            read(q, 16, sn);
+            auto parity_row = [&] {
+                uint32_t x = 0;
+                for (uint64_t w = mask; w; w &= w - 1) x ^= row[uint32_t(__builtin_ctzll(w))];
+                return x;
+            };
+            switch (op) {
+                case CLIFFT_OP_ARRAY_CNOT: row[b] ^= row[a]; break;
+                case CLIFFT_OP_ARRAY_SWAP: std::swap(row[a], row[b]); break;
+                case CLIFFT_OP_ARRAY_MULTI_CNOT: row[a] ^= parity_row(); break;
+                case CLIFFT_OP_ARRAY_CZ:
+                    out.cz.push_back(row[a]);
+                    out.cz.push_back(row[b]);
+                    break;
+                case CLIFFT_OP_ARRAY_MULTI_CZ:
+                    out.cz.push_back(row[a]);
+                    out.cz.push_back(parity_row());
+                    break;
+                case CLIFFT_OP_ARRAY_S: phase(q, row[a], 0.0, 1.0); break;
+                case CLIFFT_OP_ARRAY_S_DAG: phase(q, row[a], 0.0, -1.0); break;
+                case CLIFFT_OP_ARRAY_T:
+                    if (a < kq) phase(q, row[a], r, r);
+                    break;
+                case CLIFFT_OP_ARRAY_T_DAG:
+                    if (a < kq) phase(q, row[a], r, -r);
+                    break;
+                case CLIFFT_OP_ARRAY_ROT:
+                    if (a < kq) phase(q, row[a], c, sn);
+                    break;
+                case CLIFFT_OP_EXPAND: row.resize(kq); break;
+                case CLIFFT_OP_EXPAND_T: phase(q, row[kq], r, r); row.resize(kq); break;
+                case CLIFFT_OP_EXPAND_T_DAG: phase(q, row[kq], r, -r); row.resize(kq); break;
+                case CLIFFT_OP_EXPAND_ROT: phase(q, row[kq], c, sn); row.resize(kq); break;
+                default: break;  // frame opcodes and other EXP_VALs
+            }
+        }
+        s.n_cz = uint32_t(out.cz.size() / 2) - s.cz0;
+        s.factor0 = uint32_t(out.factor_mask.size());
+        const uint32_t t0 = uint32_t(out.terms.size());
+        for (auto& f : factors) {
+            out.factor_mask.push_back(f.first);
+            out.terms.insert(out.terms.end(), f.second.rbegin(), f.second.rend());  // program order
+            out.term_begin.push_back(uint32_t(out.terms.size()));
+        }
+        s.n_factors = uint32_t(factors.size());
+        out.max_k = std::max(out.max_k, s.k);
+        out.max_factors = std::max(out.max_factors, s.n_factors);
+        out.max_terms = std::max(out.max_terms, uint32_t(out.terms.size()) - t0);
+        out.stages.push_back(s);
+        pc = end - 1;
+    }
+    return !out.stages.empty() && out.max_terms <= kPhaseMaxTerms;
+}
+
+}  // namespace cgpu

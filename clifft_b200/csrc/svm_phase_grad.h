@@ -1,0 +1,75 @@
+// svm_phase_grad.h -- expectation-value gradients of programs whose state is a
+// phase polynomial (svm_phase_grad.cu), shared with the host side.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+namespace cgpu {
+
+struct DevProg;
+
+// A point of the program at which EXP_VALs read the state. Every amplitude of
+// the 2^k state is a product of unit phases: factor f multiplies index i when
+// the parity of (i & mask[f]) is odd, and a CZ pair flips the sign when both
+// parities are. Offsets index the arrays of PhasePlan.
+struct PhaseStage {
+    uint32_t k;
+    uint32_t factor0, n_factors;
+    uint32_t cz0, n_cz;
+    uint32_t probe0, n_probes;
+    uint32_t param0;  // n_params gradient masks (0: the parameter does not reach this stage)
+};
+// One phase of a factor: parameter `param` (e^{i phi}), or the constant (re, im) when param < 0.
+struct PhaseTerm {
+    double re, im;
+    int32_t param;
+    uint32_t pad;
+};
+struct PhaseProbe {
+    uint32_t mask;  // EXP_VAL mask index
+    uint32_t row;   // output row
+};
+
+struct PhasePlan {
+    std::vector<PhaseStage> stages;
+    std::vector<uint32_t> factor_mask, term_begin;  // term_begin: one more entry than factors
+    std::vector<PhaseTerm> terms;
+    std::vector<uint32_t> cz;  // two masks per pair
+    std::vector<PhaseProbe> probes;
+    std::vector<uint32_t> param_mask;
+    uint32_t max_k = 0, max_factors = 0, max_terms = 0;
+    // payloads of the rotations are unit phases (a call without phases uses them)
+    bool unit_payloads = true;
+};
+
+constexpr int kPhaseThreads = 512;
+constexpr uint32_t kPhaseMaxK = 13;  // 2^13 complex doubles and as many doubles: 192 KiB of shared memory
+constexpr uint32_t kPhaseMaxTerms = 256;
+
+// False when the program has an opcode that mixes amplitudes (ARRAY_H) or is
+// too large; `code`: the image's 32-byte instructions, all of them accepted by
+// the gradient entry point.
+bool build_phase_plan(const uint8_t* code, uint32_t n, PhasePlan& out);
+
+struct PhaseParams {
+    uint64_t batch;
+    uint32_t n_out, n_params, n_stages;
+    uint32_t splits;  // CTAs that share the probes of one (vector, stage)
+    const PhaseStage* stages;
+    const uint32_t* factor_mask;
+    const uint32_t* term_begin;
+    const PhaseTerm* terms;
+    const uint32_t* cz;
+    const PhaseProbe* probes;
+    const uint32_t* param_mask;
+    const double* phases;  // batch x n_params, or null = the payloads
+    double* out_exp;
+    double* out_grad;
+};
+
+using PhaseGradFn = void (*)(const DevProg, const PhaseParams);
+PhaseGradFn phase_grad_kernel_fn(uint32_t max_k);
+constexpr uint32_t phase_grad_smem(uint32_t k) { return (24u << k) + kPhaseMaxTerms * 32u + 512u; }
+
+}  // namespace cgpu
