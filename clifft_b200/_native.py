@@ -28,6 +28,7 @@ CLIFFT_GPU_NO_AUTOTUNE = 0x100
 CLIFFT_GPU_NO_SEGMENTS = 0x200
 CLIFFT_GPU_RAW_PARITY = 0x400
 CLIFFT_GPU_TENSOR_DENSE = 0x800
+CLIFFT_GPU_BYTE_RECORDS = 0x1000
 
 STATUS = {0: "ok", -1: "invalid argument", -2: "CUDA error", -3: "device error", -4: "out of memory"}
 

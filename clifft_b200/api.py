@@ -89,7 +89,8 @@ def run(program: Program, shots: int, seed: Optional[int] = None, *, precision: 
         dust_eps: float = 0.0, want_records: bool = True, fusion: Optional[bool] = None,
         profile: bool = False, autotune: bool = True, k_faults: Optional[int] = None,
         segments: bool = True, max_resident: int = 0, raw_parity: bool = False,
-        tensor_dense: bool = False) -> Dict[str, object]:
+        tensor_dense: bool = False, byte_records: bool = False,
+        outputs: Optional[Sequence[str]] = None) -> Dict[str, object]:
     """Low-level call of clifft_gpu_sample with host buffers; returns packed
     records plus everything the call reports. `fusion`: None / True = runs of
     consecutive opcodes share one pass over a global-memory statevector,
@@ -102,7 +103,9 @@ def run(program: Program, shots: int, seed: Optional[int] = None, *, precision: 
     detectors / observables without their expected parities and POSTSELECT
     recorded instead of discarding (CLIFFT_GPU_RAW_PARITY). `tensor_dense`:
     FP32 dense blocks of fused sweeps on the tensor cores
-    (CLIFFT_GPU_TENSOR_DENSE)."""
+    (CLIFFT_GPU_TENSOR_DENSE). `byte_records`: the records as uint8 arrays
+    "meas", "det" and "obs" (shots, count) instead of packed words. `outputs`:
+    the per-shot arrays to bring back (None = every one of the mode)."""
     if precision not in _PRECISIONS:
         raise ValueError(f"precision must be one of {sorted(_PRECISIONS)}")
     if shots < 0:
@@ -149,26 +152,38 @@ def run(program: Program, shots: int, seed: Optional[int] = None, *, precision: 
         flags |= N.CLIFFT_GPU_NO_FUSION
     elif fusion is True:
         flags |= N.CLIFFT_GPU_FORCE_FUSION
+    if byte_records:
+        flags |= N.CLIFFT_GPU_BYTE_RECORDS
     a.flags = flags
     o = N.Outputs()
+
+    def want(key, shape, dtype):
+        if outputs is None or key in outputs:
+            res[key] = np.empty(shape, dtype)  # the call fills every row
+
+    if want_records and byte_records:
+        want("meas", (shots, p.num_measurements), np.uint8)
+        want("det", (shots, p.num_detectors), np.uint8)
+        want("obs", (shots, p.num_observables), np.uint8)
+    elif want_records:
+        want("meas_words", (shots, mw), np.uint64)
+        want("det_words", (shots, dw), np.uint64)
+        want("obs_words", (shots, ow), np.uint64)
     if want_records:
-        res["meas_words"] = np.zeros((shots, mw), np.uint64)
-        res["det_words"] = np.zeros((shots, dw), np.uint64)
-        res["obs_words"] = np.zeros((shots, ow), np.uint64)
-        res["exp_vals"] = np.zeros((shots, p.num_exp_vals), np.float64)
-    res["survived"] = np.zeros(shots, np.uint8)
+        want("exp_vals", (shots, p.num_exp_vals), np.float64)
+    want("survived", shots, np.uint8)
     if trace:
-        res["meas_prob"] = np.zeros((shots, p.total_meas_slots), np.float64)
-        res["log_prob"] = np.zeros(shots, np.float64)
-        res["final_k"] = np.zeros(shots, np.uint32)
-        res["final_gamma"] = np.zeros((shots, 2), np.float64)
-        res["final_px"] = np.zeros((shots, p.num_words), np.uint64)
-        res["final_pz"] = np.zeros((shots, p.num_words), np.uint64)
+        want("meas_prob", (shots, p.total_meas_slots), np.float64)
+        want("log_prob", shots, np.float64)
+        want("final_k", shots, np.uint32)
+        want("final_gamma", (shots, 2), np.float64)
+        want("final_px", (shots, p.num_words), np.uint64)
+        want("final_pz", (shots, p.num_words), np.uint64)
         if dump_shots:
-            res["final_v"] = np.zeros((min(dump_shots, shots), 1 << p.peak_rank, 2), np.float64)
+            want("final_v", (min(dump_shots, shots), 1 << p.peak_rank, 2), np.float64)
             o.dump_shots = min(dump_shots, shots)
     names = {"meas_words": "meas", "det_words": "det", "obs_words": "obs", "exp_vals": "exp_vals",
-             "survived": "survived", "meas_prob": "meas_prob", "log_prob": "log_prob",
+             "meas": "meas", "det": "det", "obs": "obs", "survived": "survived", "meas_prob": "meas_prob", "log_prob": "log_prob",
              "final_k": "final_k", "final_gamma": "final_gamma", "final_px": "final_px",
              "final_pz": "final_pz", "final_v": "final_v"}
     for key, field in names.items():
@@ -197,6 +212,9 @@ def run(program: Program, shots: int, seed: Optional[int] = None, *, precision: 
     return res
 
 
+_RECORDS = ("meas", "det", "obs", "exp_vals")
+
+
 def _stats(r) -> dict:
     return {k: r[k] for k in ("kernel_ms", "kernel_launches", "group_threads", "state_in_smem",
                               "dust_clamps", "algorithmic_bytes", "streamed_bytes", "fused")}
@@ -211,11 +229,9 @@ def sample(program: Program, shots: int, seed: Optional[int] = None, *,
             "sample() cannot be used with post-selected programs because it returns a fixed "
             "number of rows and cannot discard shots. Use sample_survivors(program, shots, "
             "keep_records=True) instead.")
-    r = run(program, shots, seed, precision=precision, group_threads=group_threads, first_shot=first_shot)
-    return SampleResult(_unpack(r["meas_words"], program.num_measurements),
-                        _unpack(r["det_words"], program.num_detectors),
-                        _unpack(r["obs_words"], program.num_observables),
-                        exp_vals=r["exp_vals"], stats=_stats(r))
+    r = run(program, shots, seed, precision=precision, group_threads=group_threads, first_shot=first_shot,
+            byte_records=True, outputs=_RECORDS)
+    return SampleResult(r["meas"], r["det"], r["obs"], exp_vals=r["exp_vals"], stats=_stats(r))
 
 
 def sample_survivors(program: Program, shots: int, seed: Optional[int] = None,
@@ -225,7 +241,7 @@ def sample_survivors(program: Program, shots: int, seed: Optional[int] = None,
 
     Rows are the surviving shots in shot order."""
     r = run(program, shots, seed, precision=precision, survivors=True,
-            group_threads=group_threads, want_records=keep_records)
+            group_threads=group_threads, want_records=keep_records, outputs=None if keep_records else ())
     return _survivor_result(program, r, keep_records, shots)
 
 
@@ -298,7 +314,8 @@ def record_probabilities(program: Program, records: np.ndarray, *,
         raise ValueError("record_probabilities: hidden measurement slots are not supported")
     if n == 0:
         return np.zeros(0, np.float64)
-    r = run(p, n, 0, precision=precision, forced_meas=rec, trace=True, want_records=False)
+    r = run(p, n, 0, precision=precision, forced_meas=rec, trace=True, want_records=False,
+            outputs=("log_prob", "survived"))
     out = r["log_prob"].copy()
     out[r["survived"] == 0] = np.finfo(np.float64).min
     return out
@@ -318,11 +335,9 @@ def sample_k(program: Program, shots: int, k: int, seed: Optional[int] = None, *
              precision: str = "fp32", group_threads: int = 0) -> SampleResult:
     """clifft.sample_k (src/clifft/svm/svm.cc:548-613): every shot conditioned
     on exactly k fault events."""
-    r = run(program, shots, seed, precision=precision, group_threads=group_threads, k_faults=k)
-    return SampleResult(_unpack(r["meas_words"], program.num_measurements),
-                        _unpack(r["det_words"], program.num_detectors),
-                        _unpack(r["obs_words"], program.num_observables),
-                        exp_vals=r["exp_vals"], stats=_stats(r))
+    r = run(program, shots, seed, precision=precision, group_threads=group_threads, k_faults=k,
+            byte_records=True, outputs=_RECORDS)
+    return SampleResult(r["meas"], r["det"], r["obs"], exp_vals=r["exp_vals"], stats=_stats(r))
 
 
 def sample_k_survivors(program: Program, shots: int, k: int, seed: Optional[int] = None,
@@ -331,5 +346,5 @@ def sample_k_survivors(program: Program, shots: int, k: int, seed: Optional[int]
     """clifft.sample_k_survivors (src/clifft/svm/svm.cc:615-711). Rows are the
     surviving shots in shot order."""
     r = run(program, shots, seed, precision=precision, survivors=True, group_threads=group_threads,
-            want_records=keep_records, k_faults=k)
+            want_records=keep_records, k_faults=k, outputs=None if keep_records else ())
     return _survivor_result(program, r, keep_records, shots)

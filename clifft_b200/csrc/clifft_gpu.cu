@@ -18,6 +18,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "clifft_gpu.h"
@@ -500,6 +501,110 @@ struct SlabLease {
 }  // namespace
 
 namespace {
+
+// ------------------------------------------------------- results to the host
+// A call's outputs and counters leave the device in one copy into pinned
+// memory, and go from there into the caller's arrays (which are pageable: one
+// copy per array straight into them ran at 3-6 GB/s plus 10-20 us each). One
+// pinned buffer per process, at most kStageMax, kept between calls and
+// returned by clifft_gpu_trim; a call that finds it taken by another thread
+// uses ordinary memory.
+constexpr size_t kStageMax = size_t(64) << 20;
+struct PinnedBuffer {
+    std::mutex mu;
+    uint8_t* ptr = nullptr;
+    size_t bytes = 0;
+    void drop() {
+        if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;
+        bytes = 0;
+    }
+};
+PinnedBuffer g_pinned;
+
+class HostStage {
+    std::unique_lock<std::mutex> lock;
+    std::unique_ptr<uint8_t[]> own;
+
+public:
+    uint8_t* data = nullptr;
+    explicit HostStage(size_t bytes) : lock(g_pinned.mu, std::try_to_lock) {
+        if (lock.owns_lock() && bytes <= kStageMax) {
+            if (g_pinned.bytes < bytes) {
+                g_pinned.drop();
+                size_t want = size_t(1) << 20;
+                while (want < bytes) want <<= 1;
+                if (cudaHostAlloc(reinterpret_cast<void**>(&g_pinned.ptr), want, cudaHostAllocPortable) == cudaSuccess)
+                    g_pinned.bytes = want;
+                else
+                    cudaGetLastError();
+            }
+            if (g_pinned.bytes >= bytes) data = g_pinned.ptr;
+        }
+        if (!data) {
+            own.reset(new uint8_t[bytes]);
+            data = own.get();
+        }
+    }
+};
+
+// One output array: `rows` rows of src_row bytes at src, copied to dst, or
+// (bits > 0) unpacked to `bits` bytes per row.
+struct HostOut {
+    const uint8_t* src;
+    uint8_t* dst;
+    size_t rows, src_row;
+    uint32_t bits;
+    size_t out_bytes() const { return rows * (bits ? bits : src_row); }
+};
+
+// bits of rows [r0, r1) to bytes, eight at a time through a table
+void unpack_rows(const HostOut& o, size_t r0, size_t r1) {
+    static const std::vector<uint64_t> spread = [] {
+        std::vector<uint64_t> t(256);
+        for (uint32_t b = 0; b < 256; ++b)
+            for (uint32_t i = 0; i < 8; ++i) t[b] |= uint64_t((b >> i) & 1u) << (8 * i);
+        return t;
+    }();
+    const uint64_t* lut = spread.data();
+    const uint32_t whole = o.bits / 8, rest = o.bits % 8;
+    for (size_t r = r0; r < r1; ++r) {
+        const uint8_t* s = o.src + r * o.src_row;
+        uint8_t* d = o.dst + r * o.bits;
+        for (uint32_t i = 0; i < whole; ++i) std::memcpy(d + 8 * i, &lut[s[i]], 8);
+        if (rest) std::memcpy(d + 8 * whole, &lut[s[whole]], rest);
+    }
+}
+
+// Fills the caller's arrays, over several threads when there is much to write
+// (fresh pages cost more than the copy; 16 bytes per ns is what one core
+// unpacks, a tenth of that with page faults).
+void deliver(const std::vector<HostOut>& outs) {
+    size_t total = 0;
+    for (const HostOut& o : outs) total += o.out_bytes();
+    auto part = [&](size_t t, size_t n) {
+        for (const HostOut& o : outs) {
+            const size_t r0 = o.rows * t / n, r1 = o.rows * (t + 1) / n;
+            if (o.bits)
+                unpack_rows(o, r0, r1);
+            else
+                std::memcpy(o.dst + r0 * o.src_row, o.src + r0 * o.src_row, (r1 - r0) * o.src_row);
+        }
+    };
+    constexpr size_t kPerThread = size_t(1) << 19;
+    const size_t n = std::max<size_t>(
+        1, std::min<size_t>({total / kPerThread, size_t(8), size_t(std::thread::hardware_concurrency())}));
+    std::vector<std::thread> more;
+    size_t done = 1;  // part 0 is this thread's
+    try {
+        for (; done < n; ++done) more.emplace_back(part, done, n);
+    } catch (const std::exception&) {
+        // no further threads: the rest is done here
+    }
+    part(0, n);
+    for (size_t t = done; t < n; ++t) part(t, n);
+    for (auto& t : more) t.join();
+}
 
 struct BlobBuilder {
     std::vector<uint8_t> bytes;
@@ -1200,6 +1305,8 @@ void clifft_gpu_trim(void) {
         all.swap(g_spare);
     }
     for (auto& kv : all) cudaFree(kv.second.first);
+    std::lock_guard<std::mutex> lock(g_pinned.mu);
+    g_pinned.drop();
 }
 
 uint32_t clifft_gpu_program_peak_rank(const clifft_gpu_program* prog) { return prog ? prog->meta.peak_rank : 0; }
@@ -1255,6 +1362,8 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             invalid("CLIFFT_GPU_FORCED_MEAS needs forced_meas");
         if (forced_faults && (!args->fault_offsets || !args->readout_offsets))
             invalid("CLIFFT_GPU_FORCED_FAULTS needs fault_offsets and readout_offsets");
+        const bool byte_records = (args->flags & CLIFFT_GPU_BYTE_RECORDS) != 0;
+        if (byte_records && dev_ptrs) invalid("CLIFFT_GPU_BYTE_RECORDS needs host output buffers");
         out->passed_shots = 0;
         out->logical_errors = 0;
         out->dust_clamps = 0;
@@ -1366,7 +1475,44 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
         const size_t n_counters = 5 + m.num_observables;
         const bool profile = (args->flags & CLIFFT_GPU_PROFILE) != 0;
         const size_t scratch_words = 2 + n_counters + (profile ? 8 : 0) + 8;
-        auto* scratch = static_cast<unsigned long long*>(buf.alloc(scratch_words * 8 + 64));
+        // one device block: scratch, then every output that goes to the host
+        struct Out {
+            void* host;
+            void* field;  // the kernel parameter that holds its device address
+            size_t at, rows, row_bytes;
+            uint32_t bits;  // > 0: unpacked to that many bytes per row
+        };
+        std::vector<Out> outs;
+        size_t block_bytes = (scratch_words * 8 + 64 + 255) & ~size_t(255);
+        auto stage_out = [&](auto& field, void* host, size_t rows, size_t row_bytes, uint32_t bits = 0) {
+            if (!host || rows * row_bytes == 0) return;
+            if (dev_ptrs) {
+                field = static_cast<std::remove_reference_t<decltype(field)>>(host);
+                return;
+            }
+            outs.push_back({host, &field, block_bytes, rows, row_bytes,
+                            byte_records ? bits : 0u});
+            block_bytes += (rows * row_bytes + 255) & ~size_t(255);
+        };
+        stage_out(K.out_meas, out->meas, shots, K.meas_out_words * 8, m.num_measurements);
+        stage_out(K.out_det, out->det, shots, K.det_out_words * 8, m.num_detectors);
+        stage_out(K.out_obs, out->obs, shots, K.obs_out_words * 8, m.num_observables);
+        stage_out(K.out_exp, out->exp_vals, shots, size_t(m.num_exp_vals) * 8);
+        stage_out(K.out_survived, out->survived, shots, 1);
+        if (args->flags & CLIFFT_GPU_TRACE) {
+            stage_out(K.out_meas_prob, out->meas_prob, shots, size_t(m.total_meas_slots) * 8);
+            stage_out(K.out_log_prob, out->log_prob, shots, 8);
+            stage_out(K.out_final_k, out->final_k, shots, 4);
+            stage_out(K.out_final_gamma, out->final_gamma, shots, 16);
+            K.dump_shots = std::min<uint64_t>(out->dump_shots, shots);
+            stage_out(K.out_final_v, out->final_v, K.dump_shots, (size_t(1) << m.peak_rank) * 16);
+        }
+        auto* block = static_cast<uint8_t*>(buf.alloc(block_bytes));
+        for (const Out& o : outs) {
+            void* dev = block + o.at;
+            std::memcpy(o.field, &dev, sizeof dev);
+        }
+        auto* scratch = reinterpret_cast<unsigned long long*>(block);
         CUDA_OK(cudaMemsetAsync(scratch, 0, scratch_words * 8 + 64, st));
         K.phase_cycles = profile ? scratch + 2 + n_counters : nullptr;
         K.error_info = scratch + scratch_words - 8;
@@ -1408,37 +1554,11 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             }
         }
 
-        // outputs
-        struct Out {
-            void* host;
-            void* dev;
-            size_t bytes;
-        };
-        std::vector<Out> outs;
-        auto stage_out = [&](void* host, size_t bytes) -> void* {
-            if (!host || bytes == 0) return nullptr;
-            if (dev_ptrs) return host;
-            void* d = buf.alloc(bytes);
-            outs.push_back({host, d, bytes});
-            return d;
-        };
-        K.out_meas = static_cast<uint64_t*>(stage_out(out->meas, shots * K.meas_out_words * 8));
-        K.out_det = static_cast<uint64_t*>(stage_out(out->det, shots * K.det_out_words * 8));
-        K.out_obs = static_cast<uint64_t*>(stage_out(out->obs, shots * K.obs_out_words * 8));
-        K.out_exp = static_cast<double*>(stage_out(out->exp_vals, shots * m.num_exp_vals * 8));
-        K.out_survived = static_cast<uint8_t*>(stage_out(out->survived, shots));
         if (args->flags & CLIFFT_GPU_TRACE) {
-            K.out_meas_prob = static_cast<double*>(stage_out(out->meas_prob, shots * m.total_meas_slots * 8));
-            K.out_log_prob = static_cast<double*>(stage_out(out->log_prob, shots * 8));
-            K.out_final_k = static_cast<uint32_t*>(stage_out(out->final_k, shots * 4));
-            K.out_final_gamma = static_cast<double*>(stage_out(out->final_gamma, shots * 16));
-            // px/pz are written at the kernel's template width; narrow below
+            // px/pz are written at the kernel's template width; narrowed below
             const uint32_t nwt = L.nw_words;
             K.out_final_px = static_cast<uint64_t*>(buf.alloc(out->final_px ? shots * nwt * 8 : 0));
             K.out_final_pz = static_cast<uint64_t*>(buf.alloc(out->final_pz ? shots * nwt * 8 : 0));
-            K.dump_shots = std::min<uint64_t>(out->dump_shots, shots);
-            K.out_final_v = static_cast<double*>(
-                stage_out(out->final_v, K.dump_shots * (uint64_t(1) << m.peak_rank) * 16));
         }
 
         CallEvents& ce = call_events(prog->device);
@@ -1534,9 +1654,26 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
         }
         CUDA_OK(cudaEventRecord(e1, st));
 
-        for (auto& o : outs) CUDA_OK(cudaMemcpyAsync(o.host, o.dev, o.bytes, cudaMemcpyDeviceToHost, st));
-        std::vector<unsigned long long> hs(scratch_words);
-        CUDA_OK(cudaMemcpyAsync(hs.data(), scratch, hs.size() * 8, cudaMemcpyDeviceToHost, st));
+        // small results in one copy; large ones straight into the caller's arrays
+        const bool staged = block_bytes <= kStageMax;
+        HostStage stage(staged ? block_bytes : scratch_words * 8);
+        std::vector<HostOut> deliveries;
+        std::vector<std::unique_ptr<uint8_t[]>> packed;
+        CUDA_OK(cudaMemcpyAsync(stage.data, block, staged ? block_bytes : scratch_words * 8, cudaMemcpyDeviceToHost, st));
+        for (const Out& o : outs) {
+            const uint8_t* src = stage.data + o.at;
+            if (!staged) {
+                uint8_t* dst = static_cast<uint8_t*>(o.host);
+                if (o.bits) {
+                    packed.emplace_back(new uint8_t[o.rows * o.row_bytes]);
+                    dst = packed.back().get();
+                }
+                CUDA_OK(cudaMemcpyAsync(dst, block + o.at, o.rows * o.row_bytes, cudaMemcpyDeviceToHost, st));
+                if (!o.bits) continue;
+                src = dst;
+            }
+            deliveries.push_back({src, static_cast<uint8_t*>(o.host), o.rows, o.row_bytes, o.bits});
+        }
         std::vector<uint64_t> hpx, hpz;
         const uint32_t nwt = L.nw_words;
         if (K.out_final_px) {
@@ -1548,6 +1685,9 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             CUDA_OK(cudaMemcpyAsync(hpz.data(), K.out_final_pz, hpz.size() * 8, cudaMemcpyDeviceToHost, st));
         }
         CUDA_OK(cudaStreamSynchronize(st));
+        std::vector<unsigned long long> hs(scratch_words);
+        std::memcpy(hs.data(), stage.data, scratch_words * 8);
+        deliver(deliveries);
         float ms = 0.f;
         CUDA_OK(cudaEventElapsedTime(&ms, e0, e1));
         const uint32_t nwo = std::max<uint32_t>(m.num_words, 1);

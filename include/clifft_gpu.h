@@ -81,6 +81,9 @@ extern "C" {
                                          amplitudes stay within FP32 tolerance but are not bit-identical to the
                                          CUDA-core path, hence opt-in */
 
+#define CLIFFT_GPU_BYTE_RECORDS 0x1000u /* outputs meas / det / obs are bytes (0/1), one per record: shots x num_* uint8
+                                         instead of packed words; host buffers only */
+
 typedef struct clifft_gpu_program clifft_gpu_program;
 
 typedef struct clifft_gpu_sample_args {
@@ -110,7 +113,8 @@ typedef struct clifft_gpu_sample_args {
 
 typedef struct clifft_gpu_outputs {
     /* Per-shot bit-packed records, little-endian bit order inside u64 words:
-     * bit i of row s is word[s * words + i / 64] >> (i % 64). Any may be NULL. */
+     * bit i of row s is word[s * words + i / 64] >> (i % 64). Any may be NULL.
+     * (CLIFFT_GPU_BYTE_RECORDS: one byte per record instead.) */
     uint64_t* meas;       /* shots x ceil(num_measurements / 64) */
     uint64_t* det;        /* shots x ceil(num_detectors / 64) */
     uint64_t* obs;        /* shots x ceil(num_observables / 64), XOR expected_observables */
@@ -147,7 +151,8 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
 /* Release a handle (waits for the device) and the statevector slab that
  * sampling calls keep on it between calls. */
 void clifft_gpu_free(clifft_gpu_program* prog);
-/* Return any spare statevector slab the library holds to the device. */
+/* Return any spare statevector slab the library holds to the device, and its
+ * pinned staging buffer to the host. */
 void clifft_gpu_trim(void);
 /* Sample. See the flags above for survivors / forced / trace behaviour.
  * Survivor compaction: with CLIFFT_GPU_SURVIVORS, at least four resident waves
