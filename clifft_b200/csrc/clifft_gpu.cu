@@ -389,8 +389,11 @@ struct clifft_gpu_program {
         void* dev = nullptr;
         const BlockPlan* blocks = nullptr;
         const PlanOp* ops = nullptr;
+        const PlanGroup* groups = nullptr;
+        const uint64_t* cols = nullptr;
     };
-    std::map<std::tuple<uint32_t, bool, bool, bool>, Plans> plans;  // under plan_mu
+    std::map<std::tuple<uint32_t, bool, bool, bool, bool>, Plans> plans;  // under plan_mu
+    std::vector<uint64_t> exp_x0, exp_z0;  // first words of the EXP_VAL masks
     // what every gradient call of the program needs, uploaded by the first one
     struct Gradient {
         void* dev = nullptr;
@@ -675,23 +678,40 @@ int default_group(uint32_t peak) {
     return g;
 }
 
+// Least CUDA-core weight (U4 4, U2 2, any other micro-op 1) of a run that the
+// dense-block path puts on the tensor cores: CLIFFT_GPU_DENSE_MIN_WEIGHT, else
+// the default below.
+uint32_t dense_min_weight() {
+    static const uint32_t w = [] {
+        const char* e = std::getenv("CLIFFT_GPU_DENSE_MIN_WEIGHT");
+        const long v = e ? std::strtol(e, nullptr, 10) : 0;
+        return v > 0 ? (uint32_t)v : 4u;
+    }();
+    return w;
+}
+
 // The fused blocks for a launch shape whose statevectors stream through tiles
 // (built and uploaded on first use).
-clifft_gpu_program::Plans block_plans(clifft_gpu_program& p, uint32_t precision, bool cta, bool fuse, bool team) {
+clifft_gpu_program::Plans block_plans(clifft_gpu_program& p, uint32_t precision, const LaunchPlan& L) {
+    const bool cta = L.G == 0, team = L.team != 0;
     std::lock_guard<std::mutex> lock(p.plan_mu);
-    auto& e = p.plans[std::make_tuple(precision, cta, fuse, team)];
+    auto& e = p.plans[std::make_tuple(precision, cta, L.fuse, team, L.dense)];
     if (e.dev) return e;
     auto geometry = [&](auto cfg) {
         using TC = decltype(cfg);
-        return PlanGeometry{uint32_t(TC::kBits), fuse ? uint32_t(TC::kMops) : 1u, cta, team};
+        return PlanGeometry{uint32_t(TC::kBits), L.fuse ? uint32_t(TC::kMops) : 1u, team,
+                            L.dense ? dense_min_weight() : 0u};
     };
     const PlanGeometry g = precision == CLIFFT_GPU_FP32
                                ? (cta ? geometry(TileCfg<float, true>{}) : geometry(TileCfg<float, false>{}))
                                : (cta ? geometry(TileCfg<double, true>{}) : geometry(TileCfg<double, false>{}));
-    const PlanSet set = plan_blocks(p.code_host.data(), uint32_t(p.code_origin.size()), g);
+    const PlanSet set =
+        plan_blocks(p.code_host.data(), uint32_t(p.code_origin.size()), g, p.exp_x0.data(), p.exp_z0.data(), 1);
     BlobBuilder b;
     const size_t o_blocks = b.put(set.blocks.data(), set.blocks.size());
     const size_t o_ops = b.put(set.ops.data(), set.ops.size());
+    const size_t o_groups = b.put(set.groups.data(), set.groups.size());
+    const size_t o_cols = b.put(set.cols.data(), set.cols.size());
     void* dev = nullptr;
     CUDA_OK(alloc_retry([&] { return cudaMalloc(&dev, b.bytes.size() + 16); }));
     const cudaError_t up = cudaMemcpy(dev, b.bytes.data(), b.bytes.size(), cudaMemcpyHostToDevice);
@@ -700,6 +720,8 @@ clifft_gpu_program::Plans block_plans(clifft_gpu_program& p, uint32_t precision,
     e.dev = dev;
     e.blocks = at<BlockPlan>(dev, o_blocks);
     e.ops = at<PlanOp>(dev, o_ops);
+    e.groups = at<PlanGroup>(dev, o_groups);
+    e.cols = at<uint64_t>(dev, o_cols);
     return e;
 }
 
@@ -1063,18 +1085,6 @@ uint64_t content_hash(const uint8_t* p, size_t n, uint64_t h = 14695981039346656
     return fnv1a(p, n, h);
 }
 
-// Least CUDA-core weight (U4 4, U2 2, any other micro-op 1) of a run that the
-// dense-block path puts on the tensor cores: CLIFFT_GPU_DENSE_MIN_WEIGHT, else
-// the default below.
-uint32_t dense_min_weight() {
-    static const uint32_t w = [] {
-        const char* e = std::getenv("CLIFFT_GPU_DENSE_MIN_WEIGHT");
-        const long v = e ? std::strtol(e, nullptr, 10) : 0;
-        return v > 0 ? (uint32_t)v : 4u;
-    }();
-    return w;
-}
-
 // Persisted tuning results: with CLIFFT_GPU_TUNE_CACHE naming a file, every
 // tuned shape is appended as "program-hash device-signature mode group" and
 // earlier lines are consulted before timing trials. The device signature is
@@ -1220,6 +1230,10 @@ int clifft_gpu_load(const clifft_program_image* image, clifft_gpu_program** out)
         size_t o_code = b.put(code.bytes.data(), code.bytes.size());
         size_t o_mask = b.put(code.masks.data(), code.masks.size());
         b.bytes.resize(b.bytes.size() + 256);
+        for (uint32_t i = 0; i < im.num_exp_val_masks; ++i) {
+            p->exp_x0.push_back(ex[size_t(i) * nwt]);
+            p->exp_z0.push_back(ez[size_t(i) * nwt]);
+        }
         p->fault_probs.assign(psum.begin(), psum.end());
         for (uint32_t r = 0; r < im.num_readout_noise; ++r) p->fault_probs.push_back(im.readout_prob[r]);
         p->instr_host.assign(static_cast<const uint8_t*>(im.instructions),
@@ -1453,9 +1467,11 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
             Kx.stages = Lx.stages;
             Kx.plan = nullptr;
             if (Lx.tiles) {
-                const auto bp = block_plans(*prog, args->precision, Lx.G == 0, Lx.fuse, Lx.team != 0);
+                const auto bp = block_plans(*prog, args->precision, Lx);
                 Kx.plan = bp.blocks;
                 Kx.plan_ops = bp.ops;
+                Kx.plan_groups = bp.groups;
+                Kx.plan_cols = bp.cols;
             }
             Kx.state_in_smem = Lx.state_in_smem ? 1 : 0;
             Kx.state_stride = Lx.state_stride;
@@ -1470,7 +1486,6 @@ void sample_impl(clifft_gpu_program* prog, const clifft_gpu_sample_args* args, c
                 Kx.team_arrivals = static_cast<uint32_t*>(buf.alloc(size_t(teams) * 128));
                 CUDA_OK(cudaMemsetAsync(Kx.team_arrivals, 0, size_t(teams) * 128, st));
             }
-            Kx.dense_min_weight = dense_min_weight();
         };
         const size_t n_counters = 5 + m.num_observables;
         const bool profile = (args->flags & CLIFFT_GPU_PROFILE) != 0;
@@ -1977,9 +1992,11 @@ int clifft_gpu_batch_create(clifft_gpu_program* const* progs, const clifft_gpu_s
             K.fuse_bytes = it.L.tiles ? tile_scratch_bytes(a.precision, it.L.G == 0, it.L.stages) : 0;
             K.stages = it.L.stages;
             if (it.L.tiles) {
-                const auto bp = block_plans(*p, a.precision, it.L.G == 0, it.L.fuse, false);
+                const auto bp = block_plans(*p, a.precision, it.L);
                 K.plan = bp.blocks;
                 K.plan_ops = bp.ops;
+                K.plan_groups = bp.groups;
+                K.plan_cols = bp.cols;
             }
             K.rec_words = rec_words;
             K.det_words = det_words;

@@ -136,12 +136,13 @@ struct KParams {
     // (svm_plan.h); null when no statevector pass streams
     const BlockPlan* plan;
     const PlanOp* plan_ops;
+    const PlanGroup* plan_groups;
+    const uint64_t* plan_cols;
     // teams (G = -2): CTAs per shot, one arrival counter per team, and per team
     // two sets (used in turn) of four partial sums per CTA
     uint32_t team_size;
     uint32_t* team_arrivals;
     double* team_sums;
-    uint32_t dense_min_weight;  // KF_DENSE: least CUDA-core weight of a run worth a GEMM (U4 4, U2 2, others 1)
     unsigned long long* phase_cycles;  // optional: SM cycles per executor phase (thread 0 of each group)
     // segmented execution (survivor runs of warp groups): this launch runs
     // instructions [seg_begin, seg_end) for the items of seg_in; shots alive
@@ -469,68 +470,58 @@ struct Tally {
 };
 
 // ------------------------------------------------------------- fused sweeps
-// A fused block is a run of consecutive opcodes applied to the statevector in
-// one streamed pass: tile by tile through shared memory, every micro-op of
-// the block on a tile before it is written back. A tile covers the tile axes
-// F (2^TILE_BITS amplitudes: every index with fixed values of the other,
-// tile-global axes). The block's frame-dependent choices (conjugated phases,
-// U2 / U4 variants, EXPAND phases) are resolved once per shot into micro-ops
-// on tile-local bit positions; each amplitude sees the same arithmetic in the
-// same order as the unfused opcode sequence.
-//   * Axes an op moves amplitudes along (targets of CNOT / SWAP / H / U2 / U4,
-//     the new axis of an EXPAND) must be tile axes. Control and parity axes
-//     may be tile-global: their bits are constant over a tile and enter the
-//     micro-op's condition through `greq` / `gpar`. Diagonal ops (CZ,
-//     multi-CZ, phases) therefore fuse whatever their axes.
+// A fused block is a run of opcodes applied to the statevector in one streamed
+// pass: tile by tile through shared memory, every micro-op of the block on a
+// tile before it is written back. The host plans the blocks (svm_plan.h): which
+// opcodes, which tile, which conditions and directions. A shot resolves the
+// frame-dependent coefficients (conjugated phases, U2 / U4 variants, EXPAND
+// phases), and each amplitude sees the same arithmetic in the same order as in
+// the unfused opcode sequence.
+//   * CNOT, multi-CNOT and SWAP move nothing: they relabel the amplitudes, and
+//     the plan folds the labels into the conditions and directions of the other
+//     opcodes and into `xl` (what measurement outcomes add to the labels).
 //   * EXPAND is a micro-op (copy the new axis' clear half onto its set half,
 //     times the phase); the block loads only the runs of each tile whose new
 //     axes are clear.
+//   * Opcodes that leave the statevector alone run where they stand while the
+//     block is resolved.
 //   * An active measurement on axis k-1 ends a block: its two half-norms are
-//     summed from the tile after the block's micro-ops (an X-basis
-//     measurement first folds with an H micro-op, a fused swap with a SWAP
-//     micro-op), and the collapse to the upper half flips the shot's address
-//     label (`xo`) instead of copying it.
+//     summed from the tile in the registers of the block's last group, and the
+//     collapse to the upper half flips the shot's address label (`xo`) instead
+//     of copying it.
 //   * With KF_DENSE (FP32 CTA groups) a run of micro-ops that stays on at
 //     most four tile-local bits and holds an H / U2 / U4 is composed into one
-//     16 x 16 complex matrix, applied as a batched GEMM on the tensor cores
-//     (M_DENSE; the rest of the run becomes M_NOP).
-enum : uint8_t { M_CNOT, M_CZ, M_SWAP, M_MCNOT, M_MCZ, M_H, M_PHASE, M_U2, M_U4, M_EXPAND, M_SCALE, M_DENSE, M_NOP };
-enum : uint8_t {
-    MF_PARITY = 0x1,  // the condition also needs odd parity of (index & par) ^ (global bits & gpar)
-    MF_COPY = 0x2,    // EXPAND without a phase: a plain copy
-};
-template <typename T>
-struct MicroOpT {
-    uint8_t kind, a, b, flags;  // a, b: tile-local target bits
-    uint32_t req;               // tile-local bits that must all be set
-    uint32_t par;               // tile-local parity bits (MF_PARITY)
-    uint32_t pad;
-    uint64_t greq;              // tile-global index bits that must all be set
-    uint64_t gpar;              // tile-global parity bits (MF_PARITY)
-    T c[16];                    // coefficients, already in the statevector's precision
-};
+//     16 x 16 complex matrix, applied as a batched GEMM on the tensor cores.
+//     Such programs, and those with a POSTSELECT, are not relabelled.
+// Measured (B200), kernel ms, blocks that end at a scalar opcode and move
+// amplitudes for CNOT and SWAP -> these: k = 16 FP32, 10^4 shots 7.0 -> 6.4 and
+// k = 14 2.84 -> 2.42 (warps); k = 18 FP32, 4000 shots 16.8 -> 10.9; k = 20,
+// 394 opcodes, 150 shots 69 -> 53; k = 24, 148 shots 41 -> 26, one shot 1.02 ->
+// 0.86. The streamed bytes shrink 2.2 to 3.3 times, so HBM is no longer the
+// bound; what is: the instructions per tile, at 16 warps per SM.
 constexpr int kMaxStages = 4;      // tile buffers (tiles in flight) per shot group: 2..4, chosen per launch
 constexpr int kMaxRunsLog2 = 6;    // at most 64 contiguous runs per tile
 // Tile-engine geometry of a one-shot group. A CTA streams 32 KiB tiles and
-// fuses up to 24 opcodes per pass; a warp running one shot streams 4 KiB
-// tiles through two buffers and fuses up to 24 (FP32) / 16 (FP64), which
-// leaves room for four 4-warp CTAs per SM (the register limit). Scratch
-// layout of one group: [2 x kMaxStages mbarriers: tile loaded / tile computed]
-// [dense-block slot: MMA mbarrier, TMEM address, phase][micro-ops][64 run
-// offsets][the block's plan][stages tile buffers, 128-B
-// aligned][FP32 CTA groups with three stages: the dense block's B operand,
-// 8 KiB].
+// has up to 24 micro-ops per pass; a warp running one shot streams 4 KiB
+// tiles through two buffers and has up to 16, which leaves room for four
+// 4-warp CTAs per SM (the register limit). Scratch layout of one group:
+// [2 x kMaxStages mbarriers: tile loaded / tile computed][dense-block slot: MMA
+// mbarrier, TMEM address, phase][the block's plan][micro-ops][their groups]
+// [coefficients][64 run offsets][stages tile buffers, 128-B aligned][FP32 CTA
+// groups with three stages: the dense block's B operand, 8 KiB].
 template <typename R, bool CTA>
 struct TileCfg {
-    using MOp = MicroOpT<typename Cx<R>::T>;
     static constexpr int kBits = CTA ? (sizeof(R) == 4 ? 12 : 11) : (sizeof(R) == 4 ? 9 : 8);
-    static constexpr int kMops = CTA ? 24 : (sizeof(R) == 4 ? 24 : 16);
+    static constexpr int kMops = CTA ? 24 : 16;
     static constexpr uint32_t kBarOffset = 0;
     static constexpr uint32_t kDenseSlotOffset = 2u * kMaxStages * 8u;
-    static constexpr uint32_t kMopsOffset = kDenseSlotOffset + 16u;
-    static constexpr uint32_t kTablesOffset = kMopsOffset + kMops * (uint32_t)sizeof(MOp);
-    static constexpr uint32_t kPlanOffset = kTablesOffset + 64u * 8u;
-    static constexpr uint32_t kBufOffset = (kPlanOffset + (uint32_t)sizeof(BlockPlan) + 127u) & ~127u;
+    static constexpr uint32_t kPlanOffset = kDenseSlotOffset + 16u;
+    static constexpr uint32_t kMopsOffset = kPlanOffset + (uint32_t)sizeof(BlockPlan);
+    static constexpr uint32_t kGroupsOffset = kMopsOffset + (kMops + kExtraOps) * (uint32_t)sizeof(PlanOp);
+    // at most one group per micro-op, and a closing one for a measurement
+    static constexpr uint32_t kCoefOffset = kGroupsOffset + (kMops + kExtraOps + 1) * (uint32_t)sizeof(PlanGroup);
+    static constexpr uint32_t kTablesOffset = kCoefOffset + kMops * 16u * 2u * (uint32_t)sizeof(R);
+    static constexpr uint32_t kBufOffset = (kTablesOffset + 64u * 8u + 127u) & ~127u;
     static constexpr uint32_t kDenseBBytes = 8192u;  // B operand of a dense block: TF32 hi + lo, 32 x 32 each
     static __host__ __device__ constexpr bool dense_capable(uint32_t stages) {
         return CTA && sizeof(R) == 4 && stages == 3;
@@ -743,7 +734,8 @@ struct Shot {
     uint32_t* bar_phase;       // CTA groups: bit st = parity of the phase stage st's barrier is in;
                                // bit 31 set once a wait timed out (the barriers are then unusable)
     bool solo;                 // CTA groups: only the control warp is executing
-    int n_mops;
+    int n_slots;               // coefficient slots resolved so far in the current block
+    bool any_scale;            // the current block renormalises after one of its EXPANDs
     unsigned long long moved;  // statevector bytes actually streamed
     // Address label of a one-shot group's global statevector: logical
     // amplitude i lives at v[i ^ xo]. A measurement that keeps the upper half
@@ -751,6 +743,9 @@ struct Shot {
     // are all above the tile bits, so the label maps every tile run to one
     // contiguous run.
     uint64_t xo;
+    // What outcomes add to the physical index of a relabelled state: logical
+    // amplitude i lies at M i ^ xl (M: svm_plan.h), i.e. at v[(M i ^ xl) ^ xo]
+    uint64_t xl;
     // fused blocks: the next one on this shot's way (they come in program order)
     uint32_t plan_at;
     uint32_t plan_pc;  // and the instruction it starts at
@@ -763,6 +758,7 @@ struct Shot {
     TeamLink* team;
     T* team_v;   // the team's global statevector
     bool priv;
+    uint32_t undo_n;  // columns of M staged in the run table for the way back to logical order
 
     __device__ __forceinline__ Shot(const DevProg& p, const KParams& kp, T* vv, uint32_t* r, uint32_t* d,
                                     uint32_t* o, double* rd, unsigned char* fz, uint32_t* bp, uint64_t s)
@@ -884,9 +880,12 @@ struct Shot {
         if constexpr (Grp::kTeam) {
             if (priv || k > (uint32_t)TC::kBits) return;
             T* own = reinterpret_cast<T*>(fuse + TC::kBufOffset);
-            for (uint32_t i = threadIdx.x; i < (1u << k); i += blockDim.x) own[i] = v[i ^ xo];
+            // (the block that got here staged the columns to undo, if any)
+            for (uint32_t i = threadIdx.x; i < (1u << k); i += blockDim.x) own[i] = v[mapped(i, undo_n) ^ xo];
             v = own;
             xo = 0;
+            xl = 0;
+            undo_n = 0;
             priv = true;
             __syncthreads();
         }
@@ -972,12 +971,9 @@ struct Shot {
             uint64_t n = 1ull << k;
             if constexpr (RES) {
                 // inside a fused block: the same scaling as a micro-op, in the
-                // slot after the EXPAND that calls for it
-                if (Grp::rank() == 0) {
-                    MOp* m = mops() + n_mops - 1;
-                    m->kind = M_SCALE;
-                    m->c[0] = Cx<R>::make(g, 0.0);
-                }
+                // slot after that of the EXPAND that calls for it
+                if (Grp::rank() == 0) coef((uint32_t)n_slots - 1)[0] = Cx<R>::make(g, 1.0);
+                any_scale = true;
                 bytes += 2 * n * sizeof(T);
             } else {
                 for (uint64_t i = wrank(); i < n; i += wsize()) A(i) = cscale(A(i), (R)g);
@@ -1205,27 +1201,34 @@ struct Shot {
     };
 
     // Resolving a fused block: its micro-ops are already in shared memory, the
-    // opcodes only add what the frame decides (coefficients c, nc complex
-    // values, converted to the statevector's precision as the unfused handlers
-    // convert them; one per thread, so a U4 node costs one load latency).
-    using MOp = typename TC::MOp;
+    // opcodes only add what the frame decides, in the order of their slots
+    // (coefficients c, nc complex values, converted to the statevector's
+    // precision as the unfused handlers convert them; one per thread, so a U4
+    // node costs one load latency).
     static __host__ __device__ constexpr uint32_t fuse_bar_offset() { return TC::kBarOffset; }
-    static __host__ __device__ constexpr uint32_t fuse_mops_offset() { return TC::kMopsOffset; }
     static __host__ __device__ constexpr uint32_t fuse_tables_offset() { return TC::kTablesOffset; }
-    __device__ __forceinline__ MOp* mops() const { return reinterpret_cast<MOp*>(fuse + fuse_mops_offset()); }
+    __device__ __forceinline__ PlanOp* ops() const { return reinterpret_cast<PlanOp*>(fuse + TC::kMopsOffset); }
+    __device__ __forceinline__ T* coef(uint32_t slot) const {
+        return reinterpret_cast<T*>(fuse + TC::kCoefOffset) + 16 * slot;
+    }
     __device__ __forceinline__ void resolve_op(const double* c, int nc) {
-        MOp* m = mops() + n_mops;
-        for (int j = Grp::rank(); j < nc; j += Grp::size()) m->c[j] = Cx<R>::make(c[2 * j], c[2 * j + 1]);
-        n_mops++;
+        T* d = coef((uint32_t)n_slots++);
+        for (int j = Grp::rank(); j < nc; j += Grp::size()) d[j] = Cx<R>::make(c[2 * j], c[2 * j + 1]);
+    }
+    // M i ^ xl from the n columns staged in the run table (0: logical order)
+    __device__ __forceinline__ uint64_t mapped(uint32_t i, uint32_t n) const {
+        if (n == 0) return i;
+        const uint64_t* cols = reinterpret_cast<const uint64_t*>(fuse + fuse_tables_offset());
+        uint64_t p = xl;
+        for (uint32_t a = 0; a < n; ++a) p ^= ((i >> a) & 1u) ? cols[a] : 0ull;
+        return p;
     }
 
     // exec_array_cnot (svm_kernels.inl:124-252)
     template <bool RES>
     __device__ __forceinline__ void array_cnot(uint32_t c, uint32_t t) {
         const uint32_t n = 1u << (k - 2), cb = 1u << c, tb = 1u << t;
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n, [&](uint32_t i) { P2 p; p.i = ins00_32(i, c, t) | cb; p.x = A(p.i); p.y = A(p.i | tb); return p; },
                       [&](const P2& p) { A(p.i) = p.y; A(p.i | tb) = p.x; });
             Grp::sync();
@@ -1237,9 +1240,7 @@ struct Shot {
     template <bool RES>
     __device__ __forceinline__ void array_cz(uint32_t c, uint32_t t) {
         const uint32_t n = 1u << (k - 2), both = (1u << c) | (1u << t);
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n, [&](uint32_t i) { P1 p; p.i = ins00_32(i, c, t) | both; p.x = A(p.i); return p; },
                       [&](const P1& p) { A(p.i) = cneg(p.x); });
             Grp::sync();
@@ -1251,9 +1252,7 @@ struct Shot {
     template <bool RES>
     __device__ __forceinline__ void array_swap(uint32_t a, uint32_t b) {
         const uint32_t n = 1u << (k - 2), ab = 1u << a, bb = 1u << b;
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n, [&](uint32_t i) { P2 p; p.i = ins00_32(i, a, b); p.x = A(p.i | ab); p.y = A(p.i | bb); return p; },
                       [&](const P2& p) { A(p.i | ab) = p.y; A(p.i | bb) = p.x; });
             Grp::sync();
@@ -1265,9 +1264,7 @@ struct Shot {
     template <bool RES>
     __device__ __forceinline__ void array_multi_cnot(uint32_t t, uint64_t mask) {
         const uint32_t n = 1u << (k - 1), tb = 1u << t, low = (uint32_t)mask;
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n,
                       [&](uint32_t i) {
                           P2 p;
@@ -1296,9 +1293,7 @@ struct Shot {
     template <bool RES>
     __device__ __forceinline__ void array_multi_cz(uint32_t c, uint64_t mask) {
         const uint32_t n = 1u << (k - 1), cb = 1u << c, low = (uint32_t)mask;
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n,
                       [&](uint32_t i) {
                           P1 p;
@@ -1323,9 +1318,7 @@ struct Shot {
     __device__ __forceinline__ void array_h(uint32_t a) {
         const uint32_t n = 1u << (k - 1), ab = 1u << a;
         const R s = (R)CGPU_INV_SQRT2;
-        if constexpr (RES) {
-            resolve_op(nullptr, 0);
-        } else {
+        if constexpr (!RES) {
             sweep(n, [&](uint32_t i) { P2 p; p.i = ins0_32(i, a); p.x = A(p.i); p.y = A(p.i | ab); return p; },
                       [&](const P2& p) {
                           A(p.i) = cscale(cadd(p.x, p.y), s);
@@ -1406,7 +1399,8 @@ struct Shot {
             // inside a fused block: the new axis is a tile axis and the copy a micro-op
             const double c[2] = {with_phase ? zr : 1.0, with_phase ? (x ? -zi : zi) : 0.0};
             resolve_op(c, 1);
-            n_mops++;  // the slot of a renormalisation
+            const double keep[2] = {1.0, 0.0};
+            resolve_op(keep, 1);  // a renormalisation here overwrites it
             bytes += (2ull << k) * sizeof(T);
             k++;
             scale_magnitude<RES>(CGPU_EXPAND_SCALE);
@@ -1664,9 +1658,11 @@ struct Shot {
         }
         int m_abs = b ^ pxv;
         if (b == 1 && pzv) negate_gamma();
+        if constexpr (kTiles) {
+            if (relabel) keep_half(b);
+        }
         if (b == 1) {
             if (relabel) {
-                if constexpr (kTiles) xo ^= half;
                 bytes += (1ull << k) * sizeof(T);
             } else if (tiled(k)) {
                 if constexpr (kTiles && !Grp::kTeam) {
@@ -1841,9 +1837,9 @@ struct Shot {
     // bit-t clear half holds (x + y) / sqrt2 and the set half (x - y) / sqrt2)
     // and summed the two halves' norms (w0 bit t clear, w1 set; each 1/2 of
     // the reference's |x +- y|^2 sums, which leaves every ratio unchanged).
-    // Branch bx keeps the half with bit t = bx: the address label flips for
-    // bx = 1 (relabel), or that half is copied down (a state held in one
-    // tile). Diagonal measurements go to diag_tail.
+    // Branch bx keeps the half with bit t = bx, by its labels (relabel), or that
+    // half is copied down (a state held in one tile). Diagonal measurements go
+    // to diag_tail.
     __device__ __forceinline__ void interfere_relabel(uint32_t fa, uint32_t t, uint32_t idx, int sign, double w0,
                                                       double w1, bool relabel) {
         const bool swapped = fa != t;
@@ -1861,15 +1857,14 @@ struct Shot {
             stop = true;
             return;
         }
-        if (bx == 1) {
-            if (relabel) {
-                if constexpr (kTiles) xo ^= 1ull << t;
-            } else {
-                const uint32_t h32 = 1u << t;
-                sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i + h32); return p; },
-                      [&](const P1& p) { A(p.i) = p.x; });
-                Grp::sync();
-            }
+        if constexpr (kTiles) {
+            if (relabel) keep_half(bx);
+        }
+        if (bx == 1 && !relabel) {
+            const uint32_t h32 = 1u << t;
+            sweep(h32, [&](uint32_t i) { P1 p; p.i = i; p.x = A(i + h32); return p; },
+                  [&](const P1& p) { A(p.i) = p.x; });
+            Grp::sync();
         }
         interfere_tail(swapped, t, idx, sign, pxv, pzv, bx, w0, w1, prob);
     }
@@ -1954,7 +1949,10 @@ struct Shot {
         return p;
     }
     // exec_exp_val (svm_kernels.inl:2031-2173)
-    __device__ __forceinline__ void exp_val(uint32_t cp, uint32_t out_idx) {
+    // `relabelled`: the state's X mask is direction px and its Z mask functional
+    // pz of the physical index.
+    __device__ __forceinline__ void exp_val(uint32_t cp, uint32_t out_idx, bool relabelled = false, uint64_t px = 0,
+                                            uint64_t pz = 0) {
         const uint64_t* mx = P.exp_x + (size_t)cp * NW;
         const uint64_t* mz = P.exp_z + (size_t)cp * NW;
         int fsign = P.exp_sign[cp] != 0;
@@ -1975,8 +1973,10 @@ struct Shot {
         double result = 0.0;
         if (!dormant_x) {
             const uint64_t am = k == 64 ? ~0ull : ((1ull << k) - 1);
-            const uint64_t xa = mx[0] & am, za = mz[0] & am;
-            const int yz = __popcll(xa & za) & 3;
+            const uint64_t lx = mx[0] & am, lz = mz[0] & am;
+            const int yz = __popcll(lx & lz) & 3;
+            const uint64_t xa = relabelled ? px : lx, za = relabelled ? pz : lz;
+            const uint64_t zoff = relabelled ? xl : 0;
             double2 iph = make_double2(yz == 0 ? 1.0 : (yz == 2 ? -1.0 : 0.0),
                                        yz == 1 ? 1.0 : (yz == 3 ? -1.0 : 0.0));
             if (fsign) iph = make_double2(-iph.x, -iph.y);
@@ -1988,7 +1988,7 @@ struct Shot {
                 double ar = (double)av.x, ai = (double)av.y;
                 const double br = (double)bv.x, bi = -(double)bv.y;
                 acc[2] = __dadd_rn(acc[2], __fma_rn(ar, ar, __dmul_rn(ai, ai)));
-                const double zs = (__popcll(j & za) & 1) ? -1.0 : 1.0;
+                const double zs = (__popcll((j ^ zoff) & za) & 1) ? -1.0 : 1.0;
                 ar *= zs;
                 ai *= zs;
                 acc[0] = __dadd_rn(acc[0], __fma_rn(br, ar, -__dmul_rn(bi, ai)));
@@ -2056,15 +2056,15 @@ struct Shot {
     // sampling handlers). Each caller instantiates only the opcodes that can
     // reach it: kScalar (the control warp of a CTA: opcodes that leave the
     // statevector alone), kState (every thread of a CTA: the others),
-    // kResolve (inside a fused block: frame and gamma of its opcodes, and
-    // their coefficients) or kAll (warp groups). One copy of everything in
+    // kResolve (inside a fused block: scalar opcodes, frame and gamma of the
+    // others, and their coefficients) or kAll (warp groups). One copy of everything in
     // each place made the kernels several times larger, and a lone CTA waited
     // for instructions more than for anything else.
     enum : int { kAll, kScalar, kState, kResolve };
     template <int MODE>
     __device__ __forceinline__ void exec(uint32_t pc, const uint4& w0) {
         constexpr bool RES = MODE == kResolve;
-        constexpr bool kSca = MODE == kAll || MODE == kScalar;  // scalar opcodes
+        constexpr bool kSca = MODE != kState;                   // scalar opcodes
         constexpr bool kSv = MODE != kScalar;                   // opcodes on the statevector
         constexpr bool kMeas = MODE == kAll || MODE == kState;
         cur_pc = pc;
@@ -2263,10 +2263,10 @@ struct Shot {
         auto issue_next = [&]() {
             if (lane == 0) mbar_expect_tx(&bars[issue_st], load_bytes);
             __syncwarp();
-            const uint64_t base = load_add + issue_base;
+            const uint64_t base = load_add ^ issue_base;
             for (uint32_t j = lane; j < nruns; j += 32)
                 if (!(j & skip))
-                    bulk_load(bufs + issue_st * TN + (j << r), v + ((base + runoff[j]) ^ lx), run_bytes,
+                    bulk_load(bufs + issue_st * TN + (j << r), v + (base ^ runoff[j] ^ lx), run_bytes,
                               &bars[issue_st]);
             issue_base = next_base(issue_base);
             issue_st = issue_st + 1 == nst ? 0 : issue_st + 1;
@@ -2301,14 +2301,14 @@ struct Shot {
             T* buf = bufs + st * TN;
             compute(buf, first + t, tbase);
             if (store_runs) {
-                const uint64_t base = store_add + tbase;
+                const uint64_t base = store_add ^ tbase;
                 if constexpr (Grp::kCta) {
                     // bulk stores issued by warp 0 (32 KiB tiles)
                     fence_async_shared();
                     Grp::sync();
                     if (issuer) {
                         for (uint32_t j = lane; j < store_runs; j += 32)
-                            bulk_store(v + ((base + runoff[j]) ^ lx), buf + (j << r), run_bytes);
+                            bulk_store(v + (base ^ runoff[j] ^ lx), buf + (j << r), run_bytes);
                         bulk_commit();
                         // Refill the stage of tile t-1 once its store (one bulk
                         // group older than tile t's) has read the buffer: by now
@@ -2406,7 +2406,7 @@ struct Shot {
                 __syncwarp();
                 for (uint32_t j = lane; j < nruns; j += 32)
                     if (!(j & skip))
-                        bulk_load(bufs + st * TN + (j << r), v + ((lbase + runoff[j]) ^ lx), run_bytes, &full[st]);
+                        bulk_load(bufs + st * TN + (j << r), v + (lbase ^ runoff[j] ^ lx), run_bytes, &full[st]);
                 loads[st]++;
                 lbase = next_base(lbase);
                 ++lt;
@@ -2427,7 +2427,7 @@ struct Shot {
                 phase ^= 1u << (8 + st);
                 if (store_runs) {
                     for (uint32_t j = lane; j < store_runs; j += 32)
-                        bulk_store(v + ((sbase + runoff[j]) ^ lx), bufs + st * TN + (j << r), run_bytes);
+                        bulk_store(v + (sbase ^ runoff[j] ^ lx), bufs + st * TN + (j << r), run_bytes);
                     bulk_commit();
                 }
                 sbase = next_base(sbase);
@@ -2510,22 +2510,38 @@ struct Shot {
         const uint32_t lane = threadIdx.x & 31;
         const uint32_t clog = r + (sizeof(T) == 8 ? 0u : 1u) - 1u;  // 16-B chunks per run, log2
         const uint32_t wmask = (1u << clog) - 1u;
-        const uint32_t load_chunks = (1u << (TC::kBits - r)) << clog;
-        const uint32_t store_chunks = store_runs << clog;
+        constexpr uint32_t COPIES = TN * (uint32_t)sizeof(T) / (16u * 32u);  // 16-B chunks per lane
+        const uint32_t store_copies = (store_runs << clog) / 32u;
+        // the run table was written by other lanes
+        __syncwarp();
+        // Chunk c of a tile is c's bits mapped linearly into the statevector, so
+        // a lane's i-th chunk is its first one XOR a term that all lanes share
+        // (lane i keeps it): half the instructions of a pass went into run
+        // numbers, table loads and shifts per chunk before.
+        auto chunk_at = [&](uint32_t c, bool& skipped) -> uint64_t {
+            const uint32_t j = c >> clog;
+            skipped = (j & skip) != 0;
+            return runoff[j] * sizeof(T) ^ ((uint64_t)(c & wmask) << 4);
+        };
+        bool lane_skip, copy_skip;
+        const uint64_t lane_off = chunk_at(lane, lane_skip);
+        const uint64_t copy_off = chunk_at((lane % COPIES) * 32u, copy_skip);
+        const uint32_t copy_skips = __ballot_sync(0xffffffffu, copy_skip);
+        char* const vb = reinterpret_cast<char*>(v);
         const uint64_t lx = xo;
         auto next_base = [C](uint64_t b) { return ((b | ~C) + 1) & C; };
         auto load_tile = [&](T* dst, uint64_t tb) {
-            const uint64_t base = load_add + tb;
-            for (uint32_t c = lane; c < load_chunks; c += 32) {
-                const uint32_t j = c >> clog, w = c & wmask;
-                if (j & skip) continue;
-                cp_async16(reinterpret_cast<uint4*>(dst + (j << r)) + w,
-                           reinterpret_cast<const uint4*>(v + ((base + runoff[j]) ^ lx)) + w);
+            const uint64_t base = (load_add ^ tb ^ lx) * sizeof(T) ^ lane_off;
+            uint4* d = reinterpret_cast<uint4*>(dst) + lane;
+#pragma unroll
+            for (uint32_t i = 0; i < COPIES; ++i) {
+                const uint64_t at = base ^ __shfl_sync(0xffffffffu, copy_off, i);
+                if (((copy_skips >> i) & 1u) == 0u && !lane_skip) cp_async16(d + 32 * i, vb + at);
             }
             cp_async_commit();
         };
-        // the run table was written by other lanes; statevector writes of
-        // the previous pass must be visible before the copies read them
+        // statevector writes of the previous pass must be visible before the
+        // copies read them
         __syncwarp();
         load_tile(bufs, 0);
         uint64_t tbase = 0;
@@ -2537,11 +2553,12 @@ struct Shot {
             if (t + 1 < ntiles) load_tile(bufs + ((t + 1) & 1u) * TN, nb);
             compute(buf, t, tbase);
             if (store_runs) {
-                const uint64_t base = store_add + tbase;
-                for (uint32_t c = lane; c < store_chunks; c += 32) {
-                    const uint32_t j = c >> clog, w = c & wmask;
-                    reinterpret_cast<uint4*>(v + ((base + runoff[j]) ^ lx))[w] =
-                        reinterpret_cast<const uint4*>(buf + (j << r))[w];
+                const uint64_t base = (store_add ^ tbase ^ lx) * sizeof(T) ^ lane_off;
+                const uint4* s = reinterpret_cast<const uint4*>(buf) + lane;
+#pragma unroll
+                for (uint32_t i = 0; i < COPIES; ++i) {
+                    const uint64_t at = base ^ __shfl_sync(0xffffffffu, copy_off, i);
+                    if (i < store_copies) *reinterpret_cast<uint4*>(vb + at) = s[32 * i];
                 }
                 __syncwarp();
             }
@@ -2569,55 +2586,61 @@ struct Shot {
     }
     __device__ __forceinline__ uint32_t run_block(uint32_t pc) {
         if (pc != plan_pc) return 0;
-        if constexpr (kDenseOk) {
-            if (K.flags & KF_DENSE) return fused_block<true>();
-        }
-        return fused_block<false>();
-    }
-    template <bool WITH_DENSE>
-    __device__ uint32_t fused_block() {
-        constexpr uint32_t MB = TC::kBits;
-        // the block's plan and the fixed part of its micro-ops, from the host
-        const BlockPlan* bp = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset);
-        {
-            constexpr uint32_t HW = sizeof(BlockPlan) / 16, OW = sizeof(PlanOp) / 16;
-            const uint4* head = reinterpret_cast<const uint4*>(K.plan + plan_at);
-            const uint4* src = reinterpret_cast<const uint4*>(K.plan_ops + __ldg(&K.plan[plan_at].first_mop));
-            const uint32_t words = HW + OW * __ldg(&K.plan[plan_at].n_mops);
-            for (uint32_t i = Grp::rank(); i < words; i += Grp::size()) {
-                if (i < HW) {
-                    reinterpret_cast<uint4*>(fuse + TC::kPlanOffset)[i] = __ldg(head + i);
-                } else {
-                    // word 0, 1: the op; 2, 3: rows and columns of its index run,
-                    // kept in coefficient slots an index-map op does not use
-                    const uint32_t q = (i - HW) / OW, w = (i - HW) % OW;
-                    const uint4 x = __ldg(src + (i - HW));
-                    MOp* m = mops() + q;
-                    if (w < 2)
-                        reinterpret_cast<uint4*>(m)[w] = x;
-                    else
-                        run_words(*m)[w - 2] = x;
-                }
-            }
-            // warm the block's instructions (read one after another below)
-            const uint32_t ni = __ldg(&K.plan[plan_at].n_instr);
-            for (uint32_t i = Grp::rank(); i < ni; i += Grp::size()) touch(P.code + 2 * (plan_pc + i));
-        }
-        Grp::sync();
-        const uint32_t pc = bp->pc, n_instr = bp->n_instr, r = bp->r, kk = bp->kk, skip = bp->skip;
-        const uint32_t term_kind = bp->term_kind;
-        const uint64_t F = bp->F, C = bp->C;
-        const bool single = Grp::kTeam && bp->single;
-        const uint32_t red_bit = bp->red_bit;
-        const bool red_local = bp->red_local != 0;
-        if (!single) set_runs(F, r);
+        const BlockPlan* g = K.plan + plan_at;
         plan_at++;
         plan_pc = __ldg(&K.plan[plan_at].pc);
-        // resolve the block's frame-dependent choices
-        n_mops = 0;
+        if (__ldg(&g->kind) == BLOCK_EXP_VAL) {
+            const uint4 w0 = fetch(pc);
+            cur_pc = pc;
+            exp_val(w0.z, w0.w, true, __ldg(&g->hb[0]), __ldg(&g->hb[1]));
+            return 1;
+        }
+        if constexpr (kDenseOk) {
+            if (K.flags & KF_DENSE) return fused_block<true>(g);
+        }
+        return fused_block<false>(g);
+    }
+    static __device__ __forceinline__ uint32_t par64(uint64_t x) { return (uint32_t)__popcll(x) & 1u; }
+
+    template <bool WITH_DENSE>
+    __device__ __forceinline__ uint32_t fused_block(const BlockPlan* g) {
+        constexpr uint32_t MB = TC::kBits, TN = 1u << MB;
+        const BlockPlan* bp = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset);
+        {
+            // the block's plan, its micro-ops and their groups
+            constexpr uint32_t HW = sizeof(BlockPlan) / 16, OW = sizeof(PlanOp) / 16, GW = sizeof(PlanGroup) / 16;
+            const uint32_t n_ops = __ldg(&g->n_ops), n_groups = __ldg(&g->n_groups);
+            const uint4* head = reinterpret_cast<const uint4*>(g);
+            const uint4* src = reinterpret_cast<const uint4*>(K.plan_ops + __ldg(&g->first_op));
+            const uint4* grp = reinterpret_cast<const uint4*>(K.plan_groups + __ldg(&g->first_group));
+            for (uint32_t i = Grp::rank(); i < HW; i += Grp::size())
+                reinterpret_cast<uint4*>(fuse + TC::kPlanOffset)[i] = __ldg(head + i);
+            for (uint32_t i = Grp::rank(); i < OW * n_ops; i += Grp::size())
+                reinterpret_cast<uint4*>(fuse + TC::kMopsOffset)[i] = __ldg(src + i);
+            for (uint32_t i = Grp::rank(); i < GW * n_groups; i += Grp::size())
+                reinterpret_cast<uint4*>(fuse + TC::kGroupsOffset)[i] = __ldg(grp + i);
+        }
+        Grp::sync();
+        const uint32_t pc = bp->pc, n_instr = bp->n_instr, r = bp->r, kk = bp->kk;
+        const uint32_t term_kind = bp->term_kind, nruns = 1u << (MB - r);
+        const bool single = Grp::kTeam && bp->single;
+        if (!single) {
+            // run offsets of a tile: what its high basis vectors span
+            uint64_t* runoff = reinterpret_cast<uint64_t*>(fuse + fuse_tables_offset());
+            for (uint32_t j = Grp::rank(); j < nruns; j += Grp::size()) {
+                uint64_t x = 0;
+#pragma unroll
+                for (uint32_t b = 0; b < 6; ++b) x ^= ((j >> b) & 1u) ? bp->hb[b] : 0ull;
+                runoff[j] = x;
+            }
+        }
+        // the block's opcodes in order: frame-dependent choices of those on the
+        // statevector, the others as they stand
+        n_slots = 0;
+        any_scale = false;
         const uint32_t rend = term_kind ? bp->term_pc : pc + n_instr;
-        for (uint32_t q = pc; q < rend; ++q) exec<kResolve>(q, fetch(q));
-        const int nm = (int)bp->n_mops;
+        for (uint32_t q = pc; q < rend && !stop; ++q) exec<kResolve>(q, fetch(q));
+        if (stop) return n_instr;  // the shot ended inside the block
         uint32_t tfa = 0, tt = 0, tidx = 0;
         int tsign = 0;
         if (term_kind) {
@@ -2628,121 +2651,79 @@ struct Shot {
             tidx = w0.z;
             tsign = (((w0.x >> 16) & 0xffu) & CLIFFT_FLAG_SIGN) ? 1 : 0;
         }
+        uint32_t dense0 = 0, dense1 = 0, dmask = 0;
         if constexpr (kDenseOk && WITH_DENSE) {
-            Grp::sync();  // the resolved micro-ops, read by every thread
-            MOp* mm = mops();
-            uint32_t dmask = 0;
-            int j1 = 0;
-            const int j0 = find_dense(mm, (int)bp->n_body, (int)K.dense_min_weight, bp->fresh_local, dmask, j1);
-            if (j0 >= 0) {
+            dense0 = bp->dense0;
+            dense1 = bp->dense1;
+            dmask = bp->dense_mask;
+            Grp::sync();  // the coefficients, read by every thread
+            if (dense1) {
                 if (Grp::rank() < 16)
-                    compose_dense(mm, j0, j1, dmask, Grp::rank(),
+                    compose_dense(ops(), coef(0), dense0, dense1, dmask, Grp::rank(),
                                   reinterpret_cast<float*>(fuse + TC::dense_b_offset(K.stages)));
                 fence_async_shared();  // the B operand, read by the tensor cores
-                Grp::sync();
-                if (Grp::rank() == 0) {
-                    mm[j0].kind = M_DENSE;
-                    mm[j0].req = dmask;
-                    for (int j = j0 + 1; j < j1; ++j) mm[j].kind = M_NOP;
-                    // the dense run split some index runs: compile what is left
-                    compile_index_runs(mm, nm, (1u << MB) / (uint32_t)compute_threads());
-                }
             }
         }
         Grp::sync();
-        const MOp* mops = this->mops();
         const int tid = Grp::rank(), nthr = compute_threads();
+        const uint32_t n_groups = bp->n_groups;
+        const PlanGroup* groups = reinterpret_cast<const PlanGroup*>(fuse + TC::kGroupsOffset);
         cur_site = 6;
-        constexpr uint32_t TN = 1u << MB;
-        const uint32_t rpt = TN / (uint32_t)nthr;  // amplitudes per thread in a register-staged run
         double acc[2] = {0.0, 0.0};
-        const uint32_t nruns = 1u << (MB - r);
-        // an X-basis terminator's H is the block's last micro-op: applied
-        // together with the half-norm sums
-        const int nmo = term_kind >= 2 ? nm - 1 : nm;
+        const uint64_t xlb = xl;
+        const bool store = bp->store != 0;
+        const uint32_t n_ops = bp->n_ops;
         auto body = [&](T* buf, uint64_t, uint64_t tbase) {
-            for (int j = 0; j < nmo;) {
-                if (mops[j].kind == M_NOP) {
-                    ++j;
-                    continue;
+            // the tile's part of every condition: one lane per micro-op, shared
+            // by ballots (a 64-bit parity per op and thread costs more than
+            // most ops)
+            uint32_t tp0, tp1;
+            {
+                const uint32_t i = threadIdx.x & 31u;
+                bool p0 = false, p1 = false;
+                if (i < n_ops) {
+                    const PlanOp& m = ops()[i];
+                    const uint64_t gl = (m.flags & MF_LINEAR) ? tbase : (tbase ^ xlb);
+                    p0 = par64(gl & m.ell[0]);
+                    p1 = par64(gl & m.ell[1]);
                 }
+                tp0 = __ballot_sync(0xffffffffu, p0);
+                tp1 = __ballot_sync(0xffffffffu, p1);
+            }
+            bool dense_left = dense1 != 0;
+            for (uint32_t gi = 0; gi < n_groups; ++gi) {
+                const PlanGroup& gr = groups[gi];
                 if constexpr (kDenseOk && WITH_DENSE) {
-                    if (mops[j].kind == M_DENSE) {
-                        apply_dense(mops[j].req, buf, tid);
+                    if (dense_left && gr.op0 >= dense1) {
+                        apply_dense(dmask, buf, tid);
                         csync();
-                        ++j;
-                        continue;
+                        dense_left = false;
                     }
                 }
-                int e = j;
-                while (e < nmo && index_map_kind(mops[e].kind)) ++e;
-                if (e - j >= 2 && rpt <= kMaxRunAmps) {
-                    if (kMaxRunAmps >= 16 && rpt == 16)
-                        apply_index_run<(kMaxRunAmps >= 16 ? 16 : 8)>(mops, j, e, buf, tid, nthr, tbase);
-                    else if (rpt == 8)
-                        apply_index_run<8>(mops, j, e, buf, tid, nthr, tbase);
-                    else
-                        apply_index_run<4>(mops, j, e, buf, tid, nthr, tbase);
-                    j = e;
-                    continue;
-                }
-                apply_micro(mops[j], buf, tid, nthr, tbase);
+                run_group(gr, buf, tid, nthr, tp0, tp1, gi + 1 == n_groups && term_kind,
+                          par64((tbase ^ xlb) & bp->side_ell), single ? 1u << kk : TN, store, acc);
                 csync();
-                ++j;
             }
-            if (term_kind >= 2) {
-                // H on the measured axis, summing the norms of both outputs
-                const uint32_t a = red_bit, ab = 1u << a;
-                const R s = (R)CGPU_INV_SQRT2;
-                double q0 = 0.0, q1 = 0.0;
-                // (a single tile may be filled only up to 2^kk: its top axis is measured)
-                const uint32_t half = single ? 1u << (kk - 1) : TN >> 1;
-                for (uint32_t i = tid; i < half; i += nthr) {
-                    const uint32_t i0 = ins0_32(i, a);
-                    const T x = buf[i0], y = buf[i0 | ab];
-                    const T u = cscale(cadd(x, y), s), w = cscale(csub(x, y), s);
-                    buf[i0] = u;
-                    buf[i0 | ab] = w;
-                    q0 += cnorm_d(u);
-                    q1 += cnorm_d(w);
+            if constexpr (kDenseOk && WITH_DENSE) {
+                if (dense_left) {
+                    apply_dense(dmask, buf, tid);
+                    csync();
                 }
-                acc[0] += q0;
-                acc[1] += q1;
-            } else if (term_kind) {
-                // the measured axis' two half-norms of this tile
-                double q0 = 0.0, q1 = 0.0;
-                if (red_local) {
-                    const uint32_t filled = single ? 1u << kk : TN;
-                    for (uint32_t l = tid; l < filled; l += nthr) {
-                        const double q = cnorm_d(buf[l]);
-                        if ((l >> red_bit) & 1u)
-                            q1 += q;
-                        else
-                            q0 += q;
-                    }
-                } else {
-                    for (uint32_t l = tid; l < TN; l += nthr) q0 += cnorm_d(buf[l]);
-                    if ((tbase >> red_bit) & 1u) {
-                        q1 = q0;
-                        q0 = 0.0;
-                    }
-                }
-                acc[0] += q0;
-                acc[1] += q1;
             }
-            csync();
         };
         if (single) {
             // a team's private state: the tile is in its buffer already
             if (tid < nthr) body(v, 0, 0);
             __syncthreads();
-            moved += (nm ? (1ull << kk) : 0ull) * sizeof(T);
-        } else {
+            moved += (store ? (1ull << kk) : 0ull) * sizeof(T);
+        } else if (store || term_kind) {
+            const uint64_t C = bp->C;
+            const uint32_t skip = bp->skip, sruns = store ? nruns : 0;
             if constexpr (Grp::kWS)
-                stream_tiles_ws(1ull << (kk - MB), C, r, nm ? nruns : 0, skip, body);
+                stream_tiles_ws(1ull << (kk - MB), C, r, sruns, skip, body);
             else
-                stream_tiles(1ull << (kk - MB), C, r, 0, 0, nm ? nruns : 0, skip, body);
-            moved += (((1ull << kk) >> bp->n_fresh) + (nm ? (1ull << kk) : 0ull)) * sizeof(T);
+                stream_tiles(1ull << (kk - MB), C, r, 0, 0, sruns, skip, body);
+            moved += (((1ull << kk) >> bp->n_fresh) + (store ? (1ull << kk) : 0ull)) * sizeof(T);
             if constexpr (Grp::kTeam) {
                 if (!term_kind) team_sync();
             }
@@ -2750,6 +2731,9 @@ struct Shot {
         if (term_kind) {
             state_reduce<2>(acc);
             if (!stop) {
+                // the swaps that made the measured axis the top physical bit
+                for (uint32_t c = 0; c < bp->n_cx; ++c)
+                    if (par64(xl & bp->cx_fun[c])) xl ^= bp->cx_dir[c];
                 if (term_kind == 1) {
                     bytes += (1ull << k) * sizeof(T);
                     diag_tail(tt, tidx, tsign, acc[0], acc[1], !single);
@@ -2758,362 +2742,305 @@ struct Shot {
                 }
             }
         }
+        if (!stop && bp->cols_n) normalise(bp->cols_at, bp->cols_n);
         return n_instr;
     }
 
-    // Micro-ops that map every amplitude to one position (CNOT, SWAP,
-    // multi-CNOT: bit maps on the tile index) and / or multiply it by a
-    // factor that depends on its position (CZ, multi-CZ, PHASE).
-    static __device__ __forceinline__ bool index_map_kind(uint8_t kind) {
-        return kind == M_CNOT || kind == M_SWAP || kind == M_MCNOT || kind == M_CZ || kind == M_MCZ ||
-               kind == M_PHASE;
-    }
-    // Condition of a conditional micro-op at tile position p, given its
-    // tile-global parity gp: every `req` bit set and, with MF_PARITY, odd
-    // parity of the `par` bits and gp.
-    static __device__ __forceinline__ bool micro_on(const MOp& m, uint32_t p, uint32_t gp) {
-        return (p & m.req) == m.req && (!(m.flags & MF_PARITY) || ((__popc(p & m.par) ^ gp) & 1u));
-    }
-    static constexpr uint32_t kMaxRunAmps = sizeof(R) == 4 ? 16u : 8u;  // register budget of a staged run
-    // A run of index-map micro-ops is compiled once per block into an affine
-    // map over GF(2) of tile positions: after the run's first j ops an
-    // amplitude that started at position p0 sits at P_j = L_j p0 ^ b_j, where
-    // the linear part L_j depends only on the ops' tile-local bits and the
-    // offset b_j also on the tile's global bits (global controls, the global
-    // part of a multi gate's parity). CNOT / multi-CNOT / SWAP only update
-    // (L, b); a diagonal op's condition is an AND of affine bits of P_j, each
-    // the parity of p0 & row (the rows of L_j it reads) ^ a per-tile constant.
-    // The rows of each diagonal op and the final map's columns are kept in
-    // coefficient slots those ops do not use.
-    struct RunRows {
-        uint16_t row[3];
-        uint8_t n, pad;
-    };
-    // words 2 and 3 of a PlanOp: [RunRows, first column half][columns]; one
-    // 32-byte area behind the coefficient slot an index-map op may use
-    static __device__ __forceinline__ uint4* run_words(MOp& m) { return reinterpret_cast<uint4*>(&m.c[2]); }
-    static __device__ __forceinline__ RunRows* run_rows(MOp& m) { return reinterpret_cast<RunRows*>(&m.c[2]); }
-    static __device__ __forceinline__ const RunRows* run_rows(const MOp& m) {
-        return reinterpret_cast<const RunRows*>(&m.c[2]);
-    }
-    static __device__ __forceinline__ uint16_t* run_cols(MOp& m) { return reinterpret_cast<uint16_t*>(&m.c[2]) + 4; }
-    static __device__ __forceinline__ const uint16_t* run_cols(const MOp& m) {
-        return reinterpret_cast<const uint16_t*>(&m.c[2]) + 4;
-    }
-    // Compiles every run the tile loop will stage (the same boundaries: at
-    // least two consecutive index-map ops and rpt <= kMaxRunAmps). Run by one
-    // thread.
-    static __device__ void compile_index_runs(MOp* mops, int nm, uint32_t rpt) {
-        constexpr uint32_t MB = TC::kBits;
-        for (int j = 0; j < nm;) {
-            int e = j;
-            while (e < nm && index_map_kind(mops[e].kind)) ++e;
-            if (!(e - j >= 2 && rpt <= kMaxRunAmps)) {
-                ++j;
-                continue;
-            }
-            uint16_t rows[MB];  // P bit i = parity(p0 & rows[i]) ^ b bit i
-            for (uint32_t i = 0; i < MB; ++i) rows[i] = (uint16_t)(1u << i);
-            for (int q = j; q < e; ++q) {
-                MOp& m = mops[q];
-                auto par_row = [&](uint32_t par) {
-                    uint16_t x = 0;
-                    for (uint32_t w = par; w; w &= w - 1) x ^= rows[__ffs(w) - 1];
-                    return x;
-                };
-                switch (m.kind) {
-                    case M_CNOT:
-                        if (m.req) rows[m.a] ^= rows[__ffs(m.req) - 1];
-                        break;
-                    case M_MCNOT: rows[m.a] ^= par_row(m.par); break;
-                    case M_SWAP: {
-                        const uint16_t t = rows[m.a];
-                        rows[m.a] = rows[m.b];
-                        rows[m.b] = t;
-                        break;
-                    }
-                    default: {  // M_CZ, M_MCZ, M_PHASE
-                        RunRows* rr = run_rows(m);
-                        int n = 0;
-                        for (uint32_t w = m.req; w; w &= w - 1) rr->row[n++] = rows[__ffs(w) - 1];
-                        if (m.flags & MF_PARITY) rr->row[n++] = par_row(m.par);
-                        rr->n = (uint8_t)n;
-                        break;
-                    }
-                }
-            }
-            uint16_t* fc = run_cols(mops[j]);
-            for (uint32_t c = 0; c < MB; ++c) {
-                uint32_t col = 0;
-                for (uint32_t i = 0; i < MB; ++i) col |= ((rows[i] >> c) & 1u) << i;
-                fc[c] = (uint16_t)col;
-            }
-            j = e;
-        }
-    }
-    // A compiled run mops[j0, j1) in one pass over the tile: each thread
-    // reads RPT amplitudes (positions tid + q * nthr) into registers, follows
-    // the run's affine offset through its ops (scalar work per tile), applies
-    // every diagonal factor in the run's order to the amplitudes it hits (the
-    // same operations, in the same order, as one micro-op at a time), then
-    // writes each amplitude at its final position. The barrier between the
-    // read and write phases makes the in-place permutation safe.
-    template <int RPT>
-    static __device__ void apply_index_run(const MOp* mops, int j0, int j1, T* tile, int tid, int nthr,
-                                           uint64_t tbase) {
-        constexpr uint32_t MB = TC::kBits;
-        constexpr uint32_t QB = RPT == 16 ? 4u : (RPT == 8 ? 3u : 2u);  // bits of the register index q
-        constexpr uint32_t ALL = (1u << RPT) - 1u;
-        const uint32_t lg = MB - QB;  // p0 = tid | q << lg
-        T v[RPT];
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) v[q] = tile[tid + q * nthr];
-        // mask over q of parity(p0 & row) ^ k
-        auto bits = [&](uint32_t row, uint32_t k) -> uint32_t {
-            const uint32_t r = row >> lg;
-            uint32_t m = ((r & 1u) ? (0xAAAAu & ALL) : 0u) ^ ((r & 2u) ? (0xCCCCu & ALL) : 0u);
-            if (QB > 2) m ^= (r & 4u) ? (0xF0F0u & ALL) : 0u;
-            if (QB > 3) m ^= (r & 8u) ? (0xFF00u & ALL) : 0u;
-            const uint32_t t = ((uint32_t)__popc((uint32_t)tid & row & ((1u << lg) - 1u)) ^ k) & 1u;
-            return m ^ (0u - t) & ALL;
-        };
-        uint32_t b = 0;  // the run's affine offset so far
-        for (int j = j0; j < j1; ++j) {
-            const MOp& m = mops[j];
-            const uint64_t greq = m.greq;
-            if ((tbase & greq) != greq) continue;  // the op is the identity on this tile
-            const uint32_t kind = m.kind;
-            if (kind == M_CNOT) {
-                const uint32_t req = m.req;
-                b ^= (req ? ((b >> (__ffs(req) - 1)) & 1u) : 1u) << m.a;
-            } else if (kind == M_MCNOT) {
-                b ^= (((uint32_t)__popc(b & m.par) ^ (uint32_t)__popcll(tbase & m.gpar)) & 1u) << m.a;
-            } else if (kind == M_SWAP) {
-                const uint32_t d = ((b >> m.a) ^ (b >> m.b)) & 1u;
-                b ^= (0u - d) & ((1u << m.a) | (1u << m.b));
-            } else {
-                const RunRows rr = *run_rows(m);
-                uint32_t hit = ALL;
-                int n = 0;
-                for (uint32_t w = m.req; w; w &= w - 1) hit &= bits(rr.row[n++], (b >> (__ffs(w) - 1)) & 1u);
-                if (m.flags & MF_PARITY)
-                    hit &= bits(rr.row[n], ((uint32_t)__popc(b & m.par) ^ (uint32_t)__popcll(tbase & m.gpar)) & 1u);
-                if (kind == M_PHASE) {
-                    const T ph = m.c[0];
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) {
-                        const T w = cmul(v[q], ph);
-                        v[q] = ((hit >> q) & 1u) ? w : v[q];
-                    }
-                } else {
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) v[q] = ((hit >> q) & 1u) ? cneg(v[q]) : v[q];
-                }
-            }
-        }
-        // final positions: L p0 ^ b, L applied column by column
-        const uint16_t* fc = run_cols(mops[j0]);
-        uint32_t lt = b;
-        for (uint32_t i = 0; i < lg; ++i) lt ^= ((tid >> i) & 1u) ? (uint32_t)fc[i] : 0u;
-        uint32_t cq[QB];
-#pragma unroll
-        for (uint32_t i = 0; i < QB; ++i) cq[i] = fc[lg + i];
-        csync();
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-            uint32_t pq = lt;
-#pragma unroll
-            for (uint32_t i = 0; i < QB; ++i)
-                if ((q >> i) & 1) pq ^= cq[i];
-            tile[pq] = v[q];
-        }
-        csync();
+    // Collapse of a planned measurement onto outcome b: the half with physical
+    // top bit b ^ (xl's) becomes the state by the address label, and the labels
+    // of its amplitudes take up the measured axis' direction.
+    __device__ __forceinline__ void keep_half(int b) {
+        const BlockPlan* bp = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset);
+        const uint64_t top = 1ull << (bp->kk - 1);
+        if ((b != 0) != ((xl & top) != 0)) xo ^= top;
+        if (b) xl ^= bp->dvec;
+        xl &= top - 1;
     }
 
-    // One micro-op on a shared-memory tile of 2^TILE_BITS amplitudes whose
-    // tile-global index bits are tbase; the arithmetic matches the unfused
-    // opcode handlers exactly.
-    static __device__ __forceinline__ void apply_micro(const MOp& m, T* tile, int tid, int nthr, uint64_t tbase) {
-        constexpr uint32_t MB = TC::kBits;
-        if ((tbase & m.greq) != m.greq) return;  // the op is the identity on this tile
-        const uint32_t gp = (uint32_t)__popcll(tbase & m.gpar) & 1u;
-        const uint32_t a = m.a, b = m.b;
-        const uint32_t ab = 1u << a, bb = 1u << b;
-        switch (m.kind) {
-            case M_CNOT:
-            case M_MCNOT:
-                for (uint32_t i = tid; i < (1u << (MB - 1)); i += nthr) {
-                    const uint32_t i0 = ins0_32(i, a);
-                    if (micro_on(m, i0, gp)) {
-                        T x = tile[i0];
-                        tile[i0] = tile[i0 | ab];
-                        tile[i0 | ab] = x;
+    // Back to logical order once the state is at most one tile: amplitude i
+    // comes from M i ^ xl. A team's CTAs do it as they take their own copies.
+    __device__ __forceinline__ void normalise(uint32_t at, uint32_t n) {
+        uint64_t* cols = reinterpret_cast<uint64_t*>(fuse + fuse_tables_offset());
+        Grp::sync();
+        for (uint32_t a = Grp::rank(); a < n; a += Grp::size()) cols[a] = __ldg(K.plan_cols + at + a);
+        Grp::sync();
+        if constexpr (Grp::kTeam) {
+            undo_n = n;
+        } else {
+            T* buf = reinterpret_cast<T*>(fuse + TC::kBufOffset);
+            for (uint32_t i = Grp::rank(); i < (1u << n); i += Grp::size()) buf[i] = v[mapped(i, n) ^ xo];
+            Grp::sync();
+            for (uint32_t i = Grp::rank(); i < (1u << n); i += Grp::size()) v[xo ^ i] = buf[i];
+            xl = 0;
+            fence_async_shared();  // the buffer is a target of bulk loads
+            Grp::sync();
+        }
+    }
+
+    // A group of micro-ops in registers: every thread takes cosets of the span
+    // of the group's three directions (base: the unit index spread around the
+    // pivots), applies the ops in order and writes the amplitudes back. One
+    // shared-memory pass and one barrier per group, whatever it holds; lanes
+    // differ in the lowest free position bits, so accesses are conflict-free
+    // unless a direction's pivot is among the lowest four. In the last group
+    // of a measured block the norms of both halves of the measured axis are
+    // summed on the way (positions below `filled` only: a private state need
+    // not fill its tile). tp0 / tp1: the tile's part of the ops' conditions.
+    // Bound by issued instructions and their latency (16 warps per SM, 3.5
+    // active per scheduler, one instruction per two cycles; DRAM 20 % busy), so
+    // the plan decides all it can: leading EXPANDs read one half, norms are
+    // summed over fixed registers, the last swaps are only store addresses
+    // (k = 16, 10^4 shots 8.3 -> 6.4 ms; k = 24, 148 shots 32 -> 26 ms). Eight
+    // amplitudes, not sixteen: the unrolled code of an op is what warps wait
+    // for (before these savings k = 16 10.5 with 16, 9.3 ms with 8; k = 24 43
+    // and 37 ms). `gr` stays in shared memory: its copy in registers cost
+    // spills (8.2 against 6.4 ms).
+    __device__ __forceinline__ void run_group(const PlanGroup& gr, T* tile, int tid, int nthr, uint32_t tp0,
+                                              uint32_t tp1, bool sum, uint32_t side_tile, uint32_t filled, bool store,
+                                              double (&acc)[2]) {
+        constexpr uint32_t UNITS = (1u << TC::kBits) / kRegs, ALL = (1u << kRegs) - 1u;
+        const uint4* op = reinterpret_cast<const uint4*>(ops());
+        const uint32_t side_lam = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset)->side_lam;
+        const uint32_t o1 = gr.qv[0], o2 = gr.qv[1], o4 = gr.qv[2];
+        const uint32_t o3 = o1 ^ o2, o5 = o1 ^ o4, o6 = o2 ^ o4, o7 = o3 ^ o4;
+        for (uint32_t u = (uint32_t)tid; u < UNITS; u += (uint32_t)nthr) {
+            const uint32_t base = ins0_32(ins0_32(ins0_32(u, gr.piv[0]), gr.piv[1]), gr.piv[2]);
+            const uint32_t pos[kRegs] = {base,      base ^ o1, base ^ o2, base ^ o3,
+                                   base ^ o4, base ^ o5, base ^ o6, base ^ o7};
+            T x[kRegs];
+            // leading EXPANDs read the clear half only
+            const uint32_t n_exp = any_scale ? 0u : gr.n_exp;
+            if (n_exp == 0)
+                load_expand<0>(x, tile, pos, op);
+            else if (n_exp == 1)
+                load_expand<1>(x, tile, pos, op + 2 * gr.op0);
+            else if (n_exp == 2)
+                load_expand<2>(x, tile, pos, op + 2 * gr.op0);
+            else
+                load_expand<3>(x, tile, pos, op + 2 * gr.op0);
+            // where a condition holds over the register indices
+            auto cond = [&](uint32_t lam, uint32_t qpat, uint32_t tp, uint32_t i) -> uint32_t {
+                const uint32_t t = ((uint32_t)__popc(base & lam) ^ (tp >> i)) & 1u;
+                return (qpat ^ (0u - t)) & ALL;
+            };
+            for (uint32_t i = gr.op0 + n_exp; i < gr.op1; ++i) {
+                const uint4 h = op[2 * i];  // kind, j, n_cond, flags | lam | qpat | slot, pad, delta
+                const uint32_t kind = h.x & 0xffu, j = (h.x >> 8) & 0xffu, flags = h.x >> 24;
+                const T* cf = coef(h.w & 0xffu);
+                const uint32_t c0 = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                switch (kind) {
+                    case M_PHASE: {
+                        const T ph = cf[0];
+#pragma unroll
+                        for (uint32_t q = 0; q < kRegs; ++q) {
+                            const T w = cmul(x[q], ph);
+                            x[q] = ((c0 >> q) & 1u) ? w : x[q];
+                        }
+                        break;
+                    }
+                    case M_NEG: {
+                        uint32_t hit = c0;
+                        if (((h.x >> 16) & 0xffu) > 1u) hit &= cond(h.y >> 16, h.z >> 16, tp1, i);
+#pragma unroll
+                        for (uint32_t q = 0; q < kRegs; ++q) {
+                            const R sg = sign_of(hit, q);
+                            x[q].x *= sg;
+                            x[q].y *= sg;
+                        }
+                        break;
+                    }
+                    case M_U4: apply_u4(x, c0, cond(h.y >> 16, h.z >> 16, tp1, i), cf); break;
+                    case M_EXPAND: {
+                        const T ph = cf[0];
+                        const bool copy = (flags & MF_COPY) != 0;
+                        pair_op(j, [&](auto J) { expand_pairs<decltype(J)::value>(x, c0, ph, copy); });
+                        if (any_scale) {
+                            const T c = cf[16];  // the next slot
+                            if (c.y != (R)0) {
+#pragma unroll
+                                for (uint32_t q = 0; q < kRegs; ++q) x[q] = cscale(x[q], c.x);
+                            }
+                        }
+                        break;
+                    }
+                    case M_CX: pair_op(j, [&](auto J) { swap_pairs<decltype(J)::value>(x, c0); }); break;
+                    case M_H: pair_op(j, [&](auto J) { h_pairs<decltype(J)::value>(x, c0); }); break;
+                    default: pair_op(j, [&](auto J) { u2_pairs<decltype(J)::value>(x, c0, cf); }); break;  // M_U2
+                }
+            }
+            if (sum) {
+                // in trees over fixed registers where the measured bit is
+                // that of one direction, or of none
+                double w[kRegs], q0, q1;
+#pragma unroll
+                for (uint32_t q = 0; q < kRegs; ++q) {
+                    w[q] = cnorm_d(x[q]);
+                    if (Grp::kTeam && pos[q] >= filled) w[q] = 0.0;
+                }
+                const uint32_t j = gr.side_j;
+                if (j < SIDE_ANY) {
+                    pair_op(j, [&](auto J) { sum_halves<decltype(J)::value>(w, q0, q1); });
+                    if (j == SIDE_NONE) {
+                        q0 += q1;
+                        q1 = 0.0;
+                    }
+                } else {
+                    const uint32_t qp = gr.side_qpat;
+                    q0 = q1 = 0.0;
+#pragma unroll
+                    for (uint32_t q = 0; q < kRegs; ++q) {
+                        if ((qp >> q) & 1u)
+                            q1 += w[q];
+                        else
+                            q0 += w[q];
                     }
                 }
-                break;
-            case M_CZ:
-            case M_MCZ:
-            case M_PHASE: {
-                // positions with every `req` bit set (at most two bits)
-                const uint32_t nreq = (uint32_t)__popc(m.req);
-                const uint32_t r0 = m.req ? (uint32_t)__ffs(m.req) - 1 : 0u;
-                const uint32_t r1 = nreq > 1 ? (uint32_t)__ffs(m.req & (m.req - 1)) - 1 : 0u;
-                const T ph = m.c[0];
-                for (uint32_t i = tid; i < (1u << (MB - nreq)); i += nthr) {
-                    const uint32_t idx = (nreq == 0 ? i : (nreq == 1 ? ins0_32(i, r0) : ins00_32(i, r0, r1))) | m.req;
-                    if (!micro_on(m, idx, gp)) continue;
-                    tile[idx] = m.kind == M_PHASE ? cmul(tile[idx], ph) : cneg(tile[idx]);
-                }
-                break;
+                const bool flip = (((uint32_t)__popc(base & side_lam) ^ side_tile) & 1u) != 0;
+                acc[0] += flip ? q1 : q0;
+                acc[1] += flip ? q0 : q1;
             }
-            case M_SWAP:
-                for (uint32_t i = tid; i < (1u << (MB - 2)); i += nthr) {
-                    uint32_t base = ins00_32(i, a, b);
-                    T x = tile[base | ab];
-                    tile[base | ab] = tile[base | bb];
-                    tile[base | bb] = x;
-                }
-                break;
-            case M_H: {
-                const R s = (R)CGPU_INV_SQRT2;
-                for (uint32_t i = tid; i < (1u << (MB - 1)); i += nthr) {
-                    uint32_t i0 = ins0_32(i, a);
-                    T x = tile[i0], y = tile[i0 | ab];
-                    tile[i0] = cscale(cadd(x, y), s);
-                    tile[i0 | ab] = cscale(csub(x, y), s);
-                }
-                break;
-            }
-            case M_U2: {
-                const T m00 = m.c[0], m01 = m.c[1], m10 = m.c[2], m11 = m.c[3];
-                for (uint32_t i = tid; i < (1u << (MB - 1)); i += nthr) {
-                    uint32_t i0 = ins0_32(i, a);
-                    T x = tile[i0], y = tile[i0 | ab];
-                    tile[i0] = cmac(cmul(m00, x), m01, y);
-                    tile[i0 | ab] = cmac(cmul(m10, x), m11, y);
-                }
-                break;
-            }
-            case M_U4: {
-                // FP32: the 16 coefficients held in registers; FP64 reads them
-                // from shared memory (its registers are spoken for)
-                constexpr bool kHoist = sizeof(R) == 4;
-                T cm[kHoist ? 16 : 1];
-                if constexpr (kHoist) {
+            if (store) {
+                uint32_t to = base;
+                if (gr.n_fin) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) cm[j] = m.c[j];
+                    for (uint32_t c = 0; c < 2; ++c)
+                        to ^= ((uint32_t)__popc(base & gr.fin_lam[c]) ^ (tp0 >> (gr.op1 + c))) & 1u ? gr.fin_dir[c] : 0u;
                 }
-                auto coef = [&](int j) -> T {
-                    if constexpr (kHoist)
-                        return cm[j];
-                    else
-                        return m.c[j];
-                };
-                for (uint32_t i = tid; i < (1u << (MB - 2)); i += nthr) {
-                    uint32_t q = ins00_32(i, a, b);
-                    T x0 = tile[q], x1 = tile[q | ab], x2 = tile[q | bb], x3 = tile[q | ab | bb];
-                    T y[4];
+                const uint32_t s1 = gr.sv[0], s2 = gr.sv[1], s4 = gr.sv[2], s3 = s1 ^ s2;
+                const uint32_t out[kRegs] = {to,      to ^ s1,      to ^ s2,      to ^ s3,
+                                             to ^ s4, to ^ s4 ^ s1, to ^ s4 ^ s2, to ^ s4 ^ s3};
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        T acc = cmul(coef(4 * r), x0);
-                        acc = cmac(acc, coef(4 * r + 1), x1);
-                        acc = cmac(acc, coef(4 * r + 2), x2);
-                        acc = cmac(acc, coef(4 * r + 3), x3);
-                        y[r] = acc;
-                    }
-                    tile[q] = y[0];
-                    tile[q | ab] = y[1];
-                    tile[q | bb] = y[2];
-                    tile[q | ab | bb] = y[3];
-                }
-                break;
+                for (uint32_t q = 0; q < kRegs; ++q) tile[out[q]] = x[q];
             }
-            case M_EXPAND: {
-                // the new axis' set half from its clear half (x the phase)
-                const T ph = m.c[0];
-                const bool copy = (m.flags & MF_COPY) != 0;
-                for (uint32_t i = tid; i < (1u << (MB - 1)); i += nthr) {
-                    const uint32_t i0 = ins0_32(i, a);
-                    tile[i0 | ab] = copy ? tile[i0] : cmul(tile[i0], ph);
-                }
-                break;
+        }
+    }
+    template <int V>
+    struct Int {
+        static constexpr int value = V;
+    };
+    // f on direction j of the group, j known to the compiler
+    template <class F>
+    static __device__ __forceinline__ void pair_op(uint32_t j, F f) {
+        if (j == 0)
+            f(Int<0>{});
+        else if (j == 1)
+            f(Int<1>{});
+        else
+            f(Int<2>{});
+    }
+    static constexpr uint32_t kRegs = 1u << kGroupDirs;
+    // The registers of a coset, the first N ops being EXPANDs along directions
+    // 0 .. N - 1 (op: their headers).
+    template <int N>
+    __device__ __forceinline__ void load_expand(T (&x)[kRegs], const T* tile, const uint32_t (&pos)[kRegs],
+                                                const uint4* op) const {
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; q += 1u << N) x[q] = tile[pos[q]];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const bool copy = (op[2 * j].x >> 24) & MF_COPY;
+            const T ph = coef(op[2 * j].w & 0xffu)[0];
+#pragma unroll
+            for (uint32_t q = 0; q < kRegs; ++q)
+                if (((q & ((1u << N) - 1u)) >> j) == 0) x[q | (1u << j)] = copy ? x[q] : cmul(x[q], ph);
+        }
+    }
+    template <int J>
+    static __device__ __forceinline__ void sum_halves(const double (&w)[kRegs], double& q0, double& q1) {
+        constexpr int A = J == 0 ? 2 : 1, B = J == 2 ? 2 : 4, H = 1 << J;
+        q0 = (w[0] + w[A]) + (w[B] + w[A + B]);
+        q1 = (w[H] + w[H + A]) + (w[H + B] + w[H + A + B]);
+    }
+    template <int J>
+    static __device__ __forceinline__ void expand_pairs(T (&x)[kRegs], uint32_t side, T ph, bool copy) {
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; ++q)
+            if (!(q & (1u << J))) {
+                const bool on = (side >> q) & 1u;
+                const T a = on ? x[q | (1u << J)] : x[q], w = copy ? a : cmul(a, ph);
+                x[q] = on ? w : a;
+                x[q | (1u << J)] = on ? a : w;
             }
-            case M_SCALE: {
-                const R g = m.c[0].x;
-                for (uint32_t i = tid; i < (1u << MB); i += nthr) tile[i] = cscale(tile[i], g);
-                break;
+    }
+    template <int J>
+    static __device__ __forceinline__ void swap_pairs(T (&x)[kRegs], uint32_t hit) {
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; ++q)
+            if (!(q & (1u << J))) {
+                const bool on = (hit >> q) & 1u;
+                const T a = x[q], b = x[q | (1u << J)];
+                x[q] = on ? b : a;
+                x[q | (1u << J)] = on ? a : b;
             }
-            default: break;
+    }
+    // side: bit q set when register q holds the logical 1 of its pair. With
+    // a = register q, b = its partner: (a + b, a - b) / sqrt2, or (b - a, b + a)
+    // / sqrt2 (the same roundings: sums commute and negation is exact)
+    template <int J>
+    static __device__ __forceinline__ void h_pairs(T (&x)[kRegs], uint32_t side) {
+        const R s = (R)CGPU_INV_SQRT2;
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; ++q)
+            if (!(q & (1u << J))) {
+                // (a + b, a - b), the other way round where the set half comes
+                // first: a factor of +-1 costs nothing in an FMA
+                const R sg = sign_of(side, q);
+                const T a = x[q], b = x[q | (1u << J)];
+                x[q] = cscale(T{fma(a.x, sg, b.x), fma(a.y, sg, b.y)}, s);
+                x[q | (1u << J)] = cscale(T{fma(b.x, -sg, a.x), fma(b.y, -sg, a.y)}, s);
+            }
+    }
+    // -1 where bit q is set, 1 elsewhere
+    static __device__ __forceinline__ R sign_of(uint32_t bits, uint32_t q) {
+        const uint32_t sign = (bits << (31u - q)) & 0x80000000u;
+        if constexpr (sizeof(R) == 4)
+            return __uint_as_float(sign | 0x3f800000u);
+        else
+            return __hiloint2double((int)(sign | 0x3ff00000u), 0);
+    }
+    template <int J>
+    static __device__ __forceinline__ void u2_pairs(T (&x)[kRegs], uint32_t side, const T* c) {
+        const T m00 = c[0], m01 = c[1], m10 = c[2], m11 = c[3];
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; ++q)
+            if (!(q & (1u << J))) {
+                const bool on = (side >> q) & 1u;
+                const T a = on ? x[q | (1u << J)] : x[q], b = on ? x[q] : x[q | (1u << J)];
+                const T u = cmac(cmul(m00, a), m01, b), w = cmac(cmul(m10, a), m11, b);
+                x[q] = on ? w : u;
+                x[q | (1u << J)] = on ? u : w;
+            }
+    }
+    // directions 0 (the low axis) and 1 of the group; s0, s1: their sides
+    static __device__ __forceinline__ void apply_u4(T (&x)[kRegs], uint32_t s0, uint32_t s1, const T* c) {
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; q += 4) {
+            const bool f0 = (s0 >> q) & 1u, f1 = (s1 >> q) & 1u;
+            auto flip = [&](T (&y)[4]) {
+                const T a0 = f0 ? y[1] : y[0], a1 = f0 ? y[0] : y[1], a2 = f0 ? y[3] : y[2], a3 = f0 ? y[2] : y[3];
+                y[0] = f1 ? a2 : a0;
+                y[1] = f1 ? a3 : a1;
+                y[2] = f1 ? a0 : a2;
+                y[3] = f1 ? a1 : a3;
+            };
+            T in[4] = {x[q], x[q + 1], x[q + 2], x[q + 3]}, y[4];
+            flip(in);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                T a = cmul(c[4 * r], in[0]);
+                a = cmac(a, c[4 * r + 1], in[1]);
+                a = cmac(a, c[4 * r + 2], in[2]);
+                y[r] = cmac(a, c[4 * r + 3], in[3]);
+            }
+            flip(y);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) x[q + r] = y[r];
         }
     }
 
     // ---- dense blocks on the tensor cores (KF_DENSE, FP32 CTA groups)
     // the dense-block code exists only in the kernel instances built for it
     static constexpr bool kDenseOk = DENSE && sizeof(R) == 4 && Grp::kCta;
-    // Tile-local bits a micro-op moves or reads, or ~0u when it cannot join a
-    // dense run (an expansion, a renormalisation, a condition on tile-global
-    // bits).
-    static __device__ __forceinline__ uint32_t dense_bits(const MOp& m) {
-        if (m.greq || ((m.flags & MF_PARITY) && m.gpar)) return ~0u;
-        const uint32_t cond = m.req | ((m.flags & MF_PARITY) ? m.par : 0u);
-        switch (m.kind) {
-            case M_H:
-            case M_U2: return 1u << m.a;
-            case M_SWAP:
-            case M_U4: return (1u << m.a) | (1u << m.b);
-            case M_CNOT:
-            case M_MCNOT: return (1u << m.a) | cond;
-            case M_CZ:
-            case M_MCZ:
-            case M_PHASE: return cond;
-            default: return ~0u;
-        }
-    }
-    // Work a micro-op costs on the CUDA cores, in passes over the tile
-    static __device__ __forceinline__ int dense_weight(uint8_t kind) {
-        return kind == M_U4 ? 4 : (kind == M_U2 ? 2 : 1);
-    }
-    // The heaviest run of micro-ops in [0, n) on at most four tile-local bits
-    // that holds a mixing op (H, U2, U4) and is worth a GEMM (weight >=
-    // min_weight; the first of equal weights): returns its first op (-1:
-    // none), its end in j1 and its
-    // four bits in dmask, padded with the highest free tile bits outside
-    // `avoid`. The bits of axes the block creates are avoided: until their
-    // EXPAND their set half of the tile is not loaded, and a GEMM would
-    // multiply that memory (possibly NaN / Inf) by the zero coefficients of
-    // the identity on a padding bit.
-    static __device__ int find_dense(const MOp* mops, int n, int min_weight, uint32_t avoid, uint32_t& dmask,
-                                     int& j1) {
-        constexpr uint32_t MB = TC::kBits;
-        int best = -1, best_w = min_weight - 1;
-        uint32_t best_bits = 0;
-        for (int j = 0; j < n; ++j) {
-            uint32_t bits = 0;
-            bool mix = false;
-            int w = 0, e = j;
-            for (; e < n; ++e) {
-                const uint32_t b = dense_bits(mops[e]);
-                if (b == ~0u || __popc(bits | b) > 4) break;
-                bits |= b;
-                mix |= mops[e].kind == M_H || mops[e].kind == M_U2 || mops[e].kind == M_U4;
-                w += dense_weight(mops[e].kind);
-            }
-            if (e - j >= 2 && mix && w > best_w) {
-                best = j;
-                best_w = w;
-                best_bits = bits;
-                j1 = e;
-            }
-        }
-        if (best >= 0) {
-            // padding from the top: groups then vary in the low tile bits,
-            // which spreads a warp's accesses over the shared-memory banks
-            for (int q = (int)MB - 1; __popc(best_bits) < 4 && q >= 0; --q)
-                if (!((avoid >> q) & 1u)) best_bits |= 1u << q;
-            dmask = best_bits;
-        }
-        return best;
-    }
     // Column `col` of the 16 x 16 matrix U of micro-ops [j0, j1) on the four
     // bits of dmask (index bit q = the q-th lowest bit of dmask), composed in
     // FP64 by applying each op to the basis vector e_col with the arithmetic
@@ -3121,8 +3048,8 @@ struct Shot {
     // of the outputs, columns k = 2 col + c' of the inputs) into the K-major
     // B operand: element (n, k) at byte (k / 4) * 512 + (n / 8) * 128 +
     // (n % 8) * 16 + (k % 4) * 4, TF32 high parts first, low parts 4 KiB on.
-    static __device__ __noinline__ void compose_dense(const MOp* mops, int j0, int j1, uint32_t dmask, int col,
-                                                       float* bop) {
+    static __device__ __noinline__ void compose_dense(const PlanOp* op, const T* coefs, uint32_t j0, uint32_t j1,
+                                                       uint32_t dmask, int col, float* bop) {
         uint32_t dbit[4];
         {
             uint32_t w = dmask;
@@ -3141,74 +3068,66 @@ struct Shot {
         auto cd = [](const T& c) { return make_double2((double)c.x, (double)c.y); };
         auto mul = [](double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); };
         auto add = [](double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); };
-        for (int j = j0; j < j1; ++j) {
-            const MOp& m = mops[j];
-            const bool use_par = (m.flags & MF_PARITY) != 0;
-            const uint32_t req = dm(m.req), par = use_par ? dm(m.par) : 0u;
-            auto on = [&](uint32_t i) { return (i & req) == req && (!use_par || (__popc(i & par) & 1)); };
-            const uint32_t ab = dm(1u << (m.a & 31u)), bb = dm(1u << (m.b & 31u));
+        for (uint32_t j = j0; j < j1; ++j) {
+            const PlanOp& m = op[j];
+            const T* c = coefs + 16 * m.slot;
+            const uint32_t l0 = dm(m.lam[0]), l1 = m.n_cond > 1 ? dm(m.lam[1]) : 0u, d0 = dm(m.delta);
+            auto on = [&](uint32_t i) {
+                return (__popc(i & l0) & 1) != 0 && (m.n_cond < 2 || (__popc(i & l1) & 1) != 0);
+            };
             switch (m.kind) {
-                case M_CNOT:
-                case M_MCNOT:
-                    for (uint32_t i = 0; i < 16; ++i)
-                        if (!(i & ab) && on(i)) {
-                            const double2 t = v[i];
-                            v[i] = v[i | ab];
-                            v[i | ab] = t;
-                        }
-                    break;
-                case M_CZ:
-                case M_MCZ:
-                    for (uint32_t i = 0; i < 16; ++i)
-                        if (on(i)) v[i] = make_double2(-v[i].x, -v[i].y);
-                    break;
                 case M_PHASE: {
-                    const double2 ph = cd(m.c[0]);
+                    const double2 ph = cd(c[0]);
                     for (uint32_t i = 0; i < 16; ++i)
                         if (on(i)) v[i] = mul(v[i], ph);
                     break;
                 }
-                case M_SWAP:
+                case M_NEG:
                     for (uint32_t i = 0; i < 16; ++i)
-                        if ((i & ab) && !(i & bb)) {
-                            const uint32_t o = i ^ ab ^ bb;
+                        if (on(i)) v[i] = make_double2(-v[i].x, -v[i].y);
+                    break;
+                case M_CX:
+                    for (uint32_t i = 0; i < 16; ++i) {
+                        const uint32_t o = i ^ d0;
+                        if (i < o && on(i)) {
                             const double2 t = v[i];
                             v[i] = v[o];
                             v[o] = t;
                         }
+                    }
                     break;
                 case M_H:
                     for (uint32_t i = 0; i < 16; ++i)
-                        if (!(i & ab)) {
-                            const double2 x = v[i], y = v[i | ab];
+                        if (!on(i)) {
+                            const double2 x = v[i], y = v[i ^ d0];
                             v[i] = make_double2((x.x + y.x) * CGPU_INV_SQRT2, (x.y + y.y) * CGPU_INV_SQRT2);
-                            v[i | ab] = make_double2((x.x - y.x) * CGPU_INV_SQRT2, (x.y - y.y) * CGPU_INV_SQRT2);
+                            v[i ^ d0] = make_double2((x.x - y.x) * CGPU_INV_SQRT2, (x.y - y.y) * CGPU_INV_SQRT2);
                         }
                     break;
                 case M_U2: {
-                    const double2 m00 = cd(m.c[0]), m01 = cd(m.c[1]), m10 = cd(m.c[2]), m11 = cd(m.c[3]);
+                    const double2 m00 = cd(c[0]), m01 = cd(c[1]), m10 = cd(c[2]), m11 = cd(c[3]);
                     for (uint32_t i = 0; i < 16; ++i)
-                        if (!(i & ab)) {
-                            const double2 x = v[i], y = v[i | ab];
+                        if (!on(i)) {
+                            const double2 x = v[i], y = v[i ^ d0];
                             v[i] = add(mul(m00, x), mul(m01, y));
-                            v[i | ab] = add(mul(m10, x), mul(m11, y));
+                            v[i ^ d0] = add(mul(m10, x), mul(m11, y));
                         }
                     break;
                 }
-                case M_U4:
+                case M_U4:  // unit axes here: l0 / l1 are the two axes' own bits
                     for (uint32_t i = 0; i < 16; ++i)
-                        if (!(i & ab) && !(i & bb)) {
-                            const double2 x[4] = {v[i], v[i | ab], v[i | bb], v[i | ab | bb]};
+                        if (!(i & l0) && !(i & l1)) {
+                            const double2 x[4] = {v[i], v[i | l0], v[i | l1], v[i | l0 | l1]};
                             double2 y[4];
                             for (int r = 0; r < 4; ++r) {
-                                double2 acc = mul(cd(m.c[4 * r]), x[0]);
-                                for (int c = 1; c < 4; ++c) acc = add(acc, mul(cd(m.c[4 * r + c]), x[c]));
-                                y[r] = acc;
+                                double2 a = mul(cd(c[4 * r]), x[0]);
+                                for (int q = 1; q < 4; ++q) a = add(a, mul(cd(c[4 * r + q]), x[q]));
+                                y[r] = a;
                             }
                             v[i] = y[0];
-                            v[i | ab] = y[1];
-                            v[i | bb] = y[2];
-                            v[i | ab | bb] = y[3];
+                            v[i | l0] = y[1];
+                            v[i | l1] = y[2];
+                            v[i | l0 | l1] = y[3];
                         }
                     break;
                 default: break;
@@ -3551,6 +3470,7 @@ struct Shot {
     }
     __device__ __forceinline__ void load_state() {
         xo = 0;  // amplitudes come back in logical order
+        xl = 0;
         const unsigned char* d = K.seg_state + shot * K.seg_stride;
         const uint64_t* w = reinterpret_cast<const uint64_t*>(d);
 #pragma unroll
@@ -3577,7 +3497,6 @@ struct Shot {
         discarded = (q[7] & 2u) != 0;
         reachable = (q[7] & 4u) != 0;
         solo = false;
-        n_mops = 0;
         rec_dirty = false;
         forced = (K.flags & KF_FORCED_MEAS) ? K.forced_meas + shot * P.slots : nullptr;
         meas_prob = nullptr;
@@ -3594,9 +3513,11 @@ struct Shot {
         // SchrodingerState::reset (svm_state.cc:220-267): only v[0] needs a
         // value; every other amplitude is written by EXPAND before it is read.
         xo = 0;
+        xl = 0;
         if constexpr (Grp::kTeam) {
             v = reinterpret_cast<T*>(fuse + TC::kBufOffset);
             priv = true;
+            undo_n = 0;
         }
         f.clear();
         gamma = make_double2(1.0, 0.0);
@@ -3610,7 +3531,6 @@ struct Shot {
         bytes = 0;
         moved = 0;
         solo = false;
-        n_mops = 0;
         rec_dirty = false;
         forced = (K.flags & KF_FORCED_MEAS) ? K.forced_meas + shot * P.slots : nullptr;
         meas_prob = (K.flags & KF_TRACE) && K.out_meas_prob ? K.out_meas_prob + shot * P.slots : nullptr;
@@ -3637,6 +3557,22 @@ struct Shot {
         Grp::sync();
     }
 
+    // logical amplitude i at the end of the program
+    __device__ __forceinline__ T final_amplitude(uint64_t i) {
+        if constexpr (kTiles) {
+            if (K.plan != nullptr && k > (uint32_t)TC::kBits) {
+                const BlockPlan* e = K.plan + plan_at;
+                while (__ldg(&e->kind) != BLOCK_END) ++e;  // (an early stop leaves blocks behind)
+                const uint32_t n = e->cols_n, at = e->cols_at;
+                if (n) {
+                    uint64_t p = xl;
+                    for (uint32_t a = 0; a < n; ++a) p ^= ((i >> a) & 1u) ? __ldg(K.plan_cols + at + a) : 0ull;
+                    return v[p ^ xo];
+                }
+            }
+        }
+        return A(i);
+    }
     __device__ __forceinline__ void finish(Tally& tally) {
         const bool survived = !discarded && reachable;
         const int r = Grp::rank();
@@ -3703,8 +3639,9 @@ struct Shot {
             for (uint64_t i = r; i < stride; i += Grp::size()) {
                 double re = 0.0, im = 0.0;
                 if (i < n) {
-                    re = (double)A(i).x;
-                    im = (double)A(i).y;
+                    const T x = final_amplitude(i);
+                    re = (double)x.x;
+                    im = (double)x.y;
                 }
                 row[2 * i] = re;
                 row[2 * i + 1] = im;

@@ -1,17 +1,12 @@
 // svm_plan.cu -- host-side formation of fused blocks (see svm_plan.h).
 //
-// Rules (the device executes exactly what is planned here):
-//   * Only the axes an opcode moves amplitudes along must be tile axes:
-//     targets of CNOT / multi-CNOT / SWAP / H / U2 / U4, the new axis of an
-//     EXPAND, the measured axis of an X-basis measurement. Other axes enter
-//     a micro-op's condition through tile-global index bits.
-//   * Tile axes are padded with the lowest free axes, and a tile is at most
-//     64 contiguous runs.
-//   * An EXPAND takes two micro-op slots: a renormalisation may follow it.
-//   * An active measurement ends its block.
+// A block takes opcodes until a micro-op slot, the tile's span, an EXP_VAL or a
+// POSTSELECT stops it; opcodes that leave the statevector alone are run where
+// they stand while the block is resolved. An active measurement ends it.
 
 #include "svm_plan.h"
 
+#include <algorithm>
 #include <cstring>
 
 #include "svm_kernel.cuh"
@@ -26,7 +21,7 @@ constexpr uint32_t kNoPlan = 0xffffffffu;
 constexpr uint32_t kSingleMinRank = 9;
 
 struct Instr {
-    uint32_t op, flags, a1, a2;
+    uint32_t op, flags, a1, a2, p0;
     uint64_t mask;
 };
 
@@ -36,6 +31,7 @@ Instr decode(const uint8_t* code, uint32_t pc) {
     uint16_t a1, a2;
     std::memcpy(&a1, I + 4, 2);
     std::memcpy(&a2, I + 6, 2);
+    std::memcpy(&x.p0, I + 8, 4);
     std::memcpy(&x.mask, I + 8, 8);
     x.op = I[0];
     if (x.op >= CLIFFT_OP_MEAS_DORMANT_STATIC_FORCED && x.op <= CLIFFT_OP_SWAP_MEAS_INTERFERE_FORCED)
@@ -47,284 +43,676 @@ Instr decode(const uint8_t* code, uint32_t pc) {
 }
 
 uint32_t popc(uint64_t x) { return (uint32_t)__builtin_popcountll(x); }
+uint32_t parity(uint64_t x) { return popc(x) & 1u; }
+uint32_t top_bit(uint64_t x) { return 63u - (uint32_t)__builtin_clzll(x); }
+
+bool is_expand(uint32_t op) { return op >= CLIFFT_OP_EXPAND && op <= CLIFFT_OP_EXPAND_ROT; }
+bool is_active_meas(uint32_t op) {
+    return op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE;
+}
+bool is_permutation(uint32_t op) {
+    return op == CLIFFT_OP_ARRAY_CNOT || op == CLIFFT_OP_ARRAY_MULTI_CNOT || op == CLIFFT_OP_ARRAY_SWAP;
+}
+// runs inside a block without touching the statevector (a POSTSELECT may end
+// the shot's segment and stays outside)
+bool is_scalar(uint32_t op) {
+    return frame_op(op) || op == CLIFFT_OP_MEAS_DORMANT_STATIC || op == CLIFFT_OP_MEAS_DORMANT_RANDOM ||
+           op == CLIFFT_OP_APPLY_PAULI || op == CLIFFT_OP_NOISE || op == CLIFFT_OP_NOISE_BLOCK ||
+           op == CLIFFT_OP_READOUT_NOISE || op == CLIFFT_OP_DETECTOR || op == CLIFFT_OP_OBSERVABLE;
+}
+
+// Where the logical axes lie: directions (columns of M) and bits (rows of M^-1).
+struct Layout {
+    uint32_t k = 0;
+    uint64_t col[64], ell[64];
+    void expand() {
+        col[k] = ell[k] = 1ull << k;
+        ++k;
+    }
+    uint64_t ell_of(uint64_t axes) const {
+        uint64_t x = 0;
+        for (; axes; axes &= axes - 1) x ^= ell[__builtin_ctzll(axes)];
+        return x;
+    }
+    uint64_t col_of(uint64_t axes) const {
+        uint64_t x = 0;
+        for (; axes; axes &= axes - 1) x ^= col[__builtin_ctzll(axes)];
+        return x;
+    }
+    // a permutation opcode: the amplitudes stay, their labels change
+    void permute(const Instr& x) {
+        switch (x.op) {
+            case CLIFFT_OP_ARRAY_CNOT:
+                col[x.a1] ^= col[x.a2];
+                ell[x.a2] ^= ell[x.a1];
+                break;
+            case CLIFFT_OP_ARRAY_MULTI_CNOT:
+                for (uint64_t w = x.mask; w; w &= w - 1) col[__builtin_ctzll(w)] ^= col[x.a1];
+                ell[x.a1] ^= ell_of(x.mask);
+                break;
+            default:
+                std::swap(col[x.a1], col[x.a2]);
+                std::swap(ell[x.a1], ell[x.a2]);
+        }
+    }
+    // the amplitudes move: p ^= dir where parity(p & fun) (fun . dir = 0)
+    void move(uint64_t dir, uint64_t fun) {
+        for (uint32_t a = 0; a < k; ++a) {
+            if (parity(col[a] & fun)) col[a] ^= dir;
+            if (parity(ell[a] & dir)) ell[a] ^= fun;
+        }
+    }
+    bool identity() const {
+        for (uint32_t a = 0; a < k; ++a)
+            if (col[a] != 1ull << a || ell[a] != 1ull << a) return false;
+        return true;
+    }
+};
+
+// Span of tile vectors in reduced echelon form, pivots at the highest bits.
+struct Span {
+    std::vector<uint64_t> v;  // by insertion
+    uint64_t reduce(uint64_t x) const {
+        for (uint64_t b : v)
+            if ((x >> top_bit(b)) & 1u) x ^= b;
+        return x;
+    }
+    bool add(uint64_t x) {
+        x = reduce(x);
+        if (!x) return false;
+        const uint32_t p = top_bit(x);
+        for (uint64_t& b : v)
+            if ((b >> p) & 1u) b ^= x;
+        v.push_back(x);
+        return true;
+    }
+};
+
+struct Tile {
+    uint32_t r = 0;
+    std::vector<uint64_t> basis;  // position bit j -> physical vector (j < r: bit j)
+    std::vector<uint32_t> pivot;
+    // `need` padded with the lowest unit vectors to 2^bits indices
+    static Tile of(const Span& need, uint32_t bits) {
+        Span s = need;
+        for (uint32_t a = 0; s.v.size() < bits; ++a) s.add(1ull << a);
+        Tile t;
+        while (t.r < 64 && s.reduce(1ull << t.r) == 0) ++t.r;
+        t.r = std::min(t.r, bits);
+        // the low run as unit vectors, the rest without its bits
+        const uint64_t low = (1ull << t.r) - 1;
+        Span high;
+        for (uint64_t b : s.v) high.add(b & ~low);
+        std::sort(high.v.begin(), high.v.end());  // by pivot
+        for (uint32_t j = 0; j < t.r; ++j) {
+            t.basis.push_back(1ull << j);
+            t.pivot.push_back(j);
+        }
+        for (uint64_t b : high.v) {
+            t.basis.push_back(b);
+            t.pivot.push_back(top_bit(b));
+        }
+        return t;
+    }
+    uint32_t position(uint64_t vec) const {  // of a vector in the span
+        uint32_t l = 0;
+        for (uint32_t j = r; j < basis.size(); ++j)
+            if ((vec >> pivot[j]) & 1u) {
+                l |= 1u << j;
+                vec ^= basis[j];
+            }
+        return l | (uint32_t)vec;
+    }
+    uint16_t functional(uint64_t ell) const {
+        uint32_t m = 0;
+        for (uint32_t j = 0; j < basis.size(); ++j) m |= parity(basis[j] & ell) << j;
+        return (uint16_t)m;
+    }
+    uint64_t pivots() const {
+        uint64_t m = 0;
+        for (uint32_t p : pivot) m |= 1ull << p;
+        return m;
+    }
+};
+
+// A micro-op before its tile is known.
+struct Op {
+    uint8_t kind = 0, flags = 0, slot = 0, n_cond = 0;
+    uint64_t dir[2] = {0, 0};
+    uint64_t ell[2] = {0, 0};
+};
 
 struct Builder {
     const uint8_t* code;
     uint32_t n;
     PlanGeometry g;
+    const uint64_t *exp_x, *exp_z;
+    uint32_t exp_words;
+    bool relabel = false;
     PlanSet out;
+    Layout m;            // of the current tiled region
+    bool dirty = false;  // it may differ from the logical order
 
-    uint64_t tile_axes(uint64_t need, uint32_t& r) const {
-        uint64_t F = need;
-        for (uint32_t a = 0; popc(F) < g.bits; ++a) F |= 1ull << a;
-        r = (uint32_t)__builtin_ctzll(~F);
-        return F;
-    }
-    bool is_expand(uint32_t op) const { return op >= CLIFFT_OP_EXPAND && op <= CLIFFT_OP_EXPAND_ROT; }
-    bool is_active_meas(uint32_t op) const {
-        return op >= CLIFFT_OP_MEAS_ACTIVE_DIAGONAL && op <= CLIFFT_OP_SWAP_MEAS_INTERFERE;
-    }
-    // the opcode touches the statevector at active rank k
-    bool touches(const Instr& x, uint32_t k) const {
+    bool touches(const Instr& x) const {
         switch (x.op) {
             case CLIFFT_OP_ARRAY_T:
             case CLIFFT_OP_ARRAY_T_DAG:
             case CLIFFT_OP_ARRAY_ROT:
-            case CLIFFT_OP_ARRAY_U2: return x.a1 < k;
+            case CLIFFT_OP_ARRAY_U2: return x.a1 < m.k;
             case CLIFFT_OP_EXP_VAL: return true;
             default:
                 return (x.op >= CLIFFT_OP_ARRAY_CNOT && x.op <= CLIFFT_OP_EXPAND_ROT) || is_active_meas(x.op);
         }
     }
 
-    // ---- micro-ops of a block with tile axes F
-    struct Emit {
-        uint64_t F;
-        std::vector<PlanOp>& ops;
-        uint8_t bit(uint32_t axis) const {
-            return (F >> axis) & 1u ? (uint8_t)popc(F & ((1ull << axis) - 1)) : (uint8_t)0xff;
-        }
-        uint32_t local(uint64_t axes) const {
-            uint32_t m = 0;
-            for (uint64_t w = axes & F; w; w &= w - 1) m |= 1u << bit((uint32_t)__builtin_ctzll(w));
-            return m;
-        }
-        void operator()(uint8_t kind, uint32_t a, uint32_t b, uint64_t req, uint64_t par, uint8_t flags) {
-            PlanOp m{};
-            m.kind = kind;
-            m.a = bit(a);
-            m.b = bit(b);
-            m.flags = flags;
-            m.req = local(req);
-            m.par = local(par);
-            m.greq = req & ~F;
-            m.gpar = par & ~F;
-            ops.push_back(m);
-        }
-    };
-    void emit(Emit& e, const Instr& x, uint32_t k) const {
-        const uint64_t b1 = 1ull << (x.a1 & 63), b2 = 1ull << (x.a2 & 63);
+    // micro-ops of one opcode; advances the layout and the slot count
+    void emit(const Instr& x, Layout& l, bool moves, std::vector<Op>& ops, uint32_t& slots) const {
+        auto along = [&](uint8_t kind, uint32_t a) {
+            Op o;
+            o.kind = kind;
+            o.dir[0] = l.col[a];
+            o.ell[0] = l.ell[a];
+            o.n_cond = 1;
+            return o;
+        };
+        auto diagonal = [&](uint8_t kind, uint64_t e0, uint64_t e1) {
+            Op o;
+            o.kind = kind;
+            o.ell[0] = e0;
+            o.ell[1] = e1;
+            o.n_cond = e1 ? 2 : 1;
+            return o;
+        };
+        auto with_slot = [&](Op o) {
+            o.slot = (uint8_t)slots++;
+            ops.push_back(o);
+        };
         switch (x.op) {
-            case CLIFFT_OP_ARRAY_CNOT: e(M_CNOT, x.a2, x.a2, b1, 0, 0); break;
-            case CLIFFT_OP_ARRAY_CZ: e(M_CZ, x.a1, x.a2, b1 | b2, 0, 0); break;
-            case CLIFFT_OP_ARRAY_SWAP: e(M_SWAP, x.a1, x.a2, 0, 0, 0); break;
-            case CLIFFT_OP_ARRAY_MULTI_CNOT: e(M_MCNOT, x.a1, x.a1, 0, x.mask & ~b1, MF_PARITY); break;
-            case CLIFFT_OP_ARRAY_MULTI_CZ: e(M_MCZ, x.a1, x.a1, b1, x.mask, MF_PARITY); break;
-            case CLIFFT_OP_ARRAY_H: e(M_H, x.a1, x.a1, 0, 0, 0); break;
+            case CLIFFT_OP_ARRAY_CNOT:
+            case CLIFFT_OP_ARRAY_MULTI_CNOT:
+            case CLIFFT_OP_ARRAY_SWAP:
+                if (moves) {
+                    // a conditional swap along the target (SWAP: along both axes, where their bits differ)
+                    Op o;
+                    o.kind = M_CX;
+                    o.n_cond = 1;
+                    if (x.op == CLIFFT_OP_ARRAY_SWAP) {
+                        o.dir[0] = l.col[x.a1] ^ l.col[x.a2];
+                        o.ell[0] = l.ell[x.a1] ^ l.ell[x.a2];
+                    } else if (x.op == CLIFFT_OP_ARRAY_CNOT) {
+                        o.dir[0] = l.col[x.a2];
+                        o.ell[0] = l.ell[x.a1];
+                    } else {
+                        o.dir[0] = l.col[x.a1];
+                        o.ell[0] = l.ell_of(x.mask);
+                    }
+                    // consecutive CNOTs of one control are one swap along all their targets
+                    if (x.op == CLIFFT_OP_ARRAY_CNOT && !ops.empty() && ops.back().kind == M_CX &&
+                        ops.back().ell[0] == o.ell[0] && g.max_ops > 1 && !g.dense_min_weight)
+                        ops.back().dir[0] ^= o.dir[0];
+                    else if (o.ell[0])
+                        ops.push_back(o);
+                    if (!ops.empty() && ops.back().kind == M_CX && !ops.back().dir[0]) ops.pop_back();
+                } else {
+                    l.permute(x);
+                }
+                break;
+            case CLIFFT_OP_ARRAY_CZ: ops.push_back(diagonal(M_NEG, l.ell[x.a1], l.ell[x.a2])); break;
+            case CLIFFT_OP_ARRAY_MULTI_CZ:
+                if (x.mask) ops.push_back(diagonal(M_NEG, l.ell[x.a1], l.ell_of(x.mask)));
+                break;
+            case CLIFFT_OP_ARRAY_H: ops.push_back(along(M_H, x.a1)); break;
             case CLIFFT_OP_ARRAY_S:
-            case CLIFFT_OP_ARRAY_S_DAG: e(M_PHASE, x.a1, x.a1, b1, 0, 0); break;
+            case CLIFFT_OP_ARRAY_S_DAG: with_slot(diagonal(M_PHASE, l.ell[x.a1], 0)); break;
             case CLIFFT_OP_ARRAY_T:
             case CLIFFT_OP_ARRAY_T_DAG:
             case CLIFFT_OP_ARRAY_ROT:
-                if (x.a1 < k) e(M_PHASE, x.a1, x.a1, b1, 0, 0);
+                if (x.a1 < l.k) with_slot(diagonal(M_PHASE, l.ell[x.a1], 0));
                 break;
             case CLIFFT_OP_ARRAY_U2:
-                if (x.a1 < k) e(M_U2, x.a1, x.a1, 0, 0, 0);
+                if (x.a1 < l.k) with_slot(along(M_U2, x.a1));
                 break;
-            case CLIFFT_OP_ARRAY_U4: e(M_U4, x.a1, x.a2, 0, 0, 0); break;
+            case CLIFFT_OP_ARRAY_U4: {
+                Op o = along(M_U4, x.a1);
+                o.dir[1] = l.col[x.a2];
+                o.ell[1] = l.ell[x.a2];
+                o.n_cond = 2;
+                with_slot(o);
+                break;
+            }
             case CLIFFT_OP_EXPAND:
             case CLIFFT_OP_EXPAND_T:
             case CLIFFT_OP_EXPAND_T_DAG:
-            case CLIFFT_OP_EXPAND_ROT:
-                e(M_EXPAND, x.a1, x.a1, 0, 0, x.op == CLIFFT_OP_EXPAND ? MF_COPY : 0);
-                e(M_NOP, x.a1, x.a1, 0, 0, 0);  // becomes M_SCALE when the shot renormalises here
+            case CLIFFT_OP_EXPAND_ROT: {
+                l.expand();
+                Op o = along(M_EXPAND, l.k - 1);
+                o.flags = x.op == CLIFFT_OP_EXPAND ? MF_COPY : 0;
+                with_slot(o);
+                slots++;  // a renormalisation
                 break;
+            }
             default: break;
         }
     }
 
-    // ---- index runs as affine maps over GF(2) (see apply_index_run)
-    static bool index_map(uint8_t kind) {
-        return kind == M_CNOT || kind == M_SWAP || kind == M_MCNOT || kind == M_CZ || kind == M_MCZ ||
-               kind == M_PHASE;
-    }
-    void compile_runs(PlanOp* m, uint32_t count) const {
-        for (uint32_t j = 0; j < count;) {
-            uint32_t e = j;
-            while (e < count && index_map(m[e].kind)) ++e;
-            if (e - j < 2) {
-                ++j;
-                continue;
-            }
-            uint16_t rows[12];
-            for (uint32_t i = 0; i < g.bits; ++i) rows[i] = (uint16_t)(1u << i);
-            for (uint32_t q = j; q < e; ++q) {
-                PlanOp& o = m[q];
-                auto parity_row = [&] {
-                    uint16_t x = 0;
-                    for (uint32_t w = o.par; w; w &= w - 1) x ^= rows[__builtin_ctz(w)];
-                    return x;
-                };
-                if (o.kind == M_CNOT) {
-                    if (o.req) rows[o.a] ^= rows[__builtin_ctz(o.req)];
-                } else if (o.kind == M_MCNOT) {
-                    rows[o.a] ^= parity_row();
-                } else if (o.kind == M_SWAP) {
-                    std::swap(rows[o.a], rows[o.b]);
-                } else {
-                    uint8_t c = 0;
-                    for (uint32_t w = o.req; w; w &= w - 1) o.row[c++] = rows[__builtin_ctz(w)];
-                    if (o.flags & MF_PARITY) o.row[c++] = parity_row();
-                    o.n_rows = c;
+    // ---- groups of micro-ops that share a pass over the tile
+    void close_group(uint32_t op0, uint32_t op1, std::vector<uint32_t> dirs, const BlockPlan& b, bool last) {
+        PlanGroup gr{};
+        if (last && b.side_lam) {
+            // at most one direction on which the measured bit changes, as far
+            // as the ops leave their directions free: the sums of both halves
+            // are then over fixed registers
+            auto bound = [&](uint32_t j) {
+                for (uint32_t i = op0; i < op1 - b.n_cx; ++i) {
+                    const PlanOp& o = out.ops[b.first_op + i];
+                    if (o.delta && (o.j == j || (o.kind == M_U4 && j < 2))) return true;
                 }
-            }
-            for (uint32_t c = 0; c < g.bits; ++c) {
-                uint32_t col = 0;
-                for (uint32_t i = 0; i < g.bits; ++i) col |= ((rows[i] >> c) & 1u) << i;
-                m[j].cols[c] = (uint16_t)col;
-            }
-            j = e;
+                return false;
+            };
+            uint32_t at = ~0u;
+            for (uint32_t j = 0; j < dirs.size(); ++j)
+                if (parity(dirs[j] & b.side_lam) && (at == ~0u || (!bound(at) && bound(j)))) at = j;
+            for (uint32_t j = 0; j < dirs.size(); ++j)
+                if (at != ~0u && j != at && parity(dirs[j] & b.side_lam) && !bound(j)) dirs[j] ^= dirs[at];
         }
+        Span s;
+        uint32_t pivots = 0;
+        for (uint32_t d : dirs) s.add(d);
+        for (uint64_t v : s.v) pivots |= 1u << top_bit(v);
+        for (uint32_t a = g.bits; a-- > 0 && dirs.size() < kGroupDirs;)
+            if (!((pivots >> a) & 1u)) {
+                dirs.push_back(1u << a);
+                pivots |= 1u << a;
+            }
+        uint32_t w = pivots;
+        for (uint32_t j = 0; j < kGroupDirs; ++j, w &= w - 1) {
+            gr.qv[j] = (uint16_t)dirs[j];
+            gr.piv[j] = (uint8_t)__builtin_ctz(w);
+        }
+        auto pattern = [&](uint32_t lam) {
+            uint32_t p = 0;
+            for (uint32_t q = 0; q < (1u << kGroupDirs); ++q) {
+                uint32_t x = 0;
+                for (uint32_t j = 0; j < kGroupDirs; ++j)
+                    if ((q >> j) & 1u) x ^= dirs[j];
+                p |= parity(x & lam) << q;
+            }
+            return (uint16_t)p;
+        };
+        gr.op0 = (uint8_t)op0;
+        gr.op1 = (uint8_t)op1;
+        if (last && b.n_cx) {
+            // the swaps before a measurement, by the stores: both conditions
+            // on the position before them
+            gr.n_fin = (uint8_t)b.n_cx;
+            gr.op1 = (uint8_t)(op1 - b.n_cx);
+        }
+        for (uint32_t i = op0; i < op1; ++i) {
+            PlanOp& o = out.ops[b.first_op + i];
+            for (int c = 0; c < 2; ++c) o.qpat[c] = pattern(o.lam[c]);
+            if (i == op0 + gr.n_exp && o.kind == M_EXPAND && o.j == gr.n_exp && o.qpat[0] == kPattern[o.j] &&
+                (o.lam[0] & ~pivots) == 0)
+                gr.n_exp++;
+        }
+        for (uint32_t j = 0; j < kGroupDirs; ++j) {
+            gr.sv[j] = gr.qv[j];
+            for (uint32_t i = gr.op1; i < op1; ++i)
+                if (parity(out.ops[b.first_op + i].lam[0] & gr.qv[j])) gr.sv[j] ^= out.ops[b.first_op + i].delta;
+        }
+        for (uint32_t c = 0; c < gr.n_fin; ++c) {
+            gr.fin_lam[c] = out.ops[b.first_op + gr.op1 + c].lam[0];
+            gr.fin_dir[c] = out.ops[b.first_op + gr.op1 + c].delta;
+        }
+        if (last) gr.side_qpat = pattern(b.side_lam);
+        gr.side_j = gr.side_qpat ? SIDE_ANY : SIDE_NONE;
+        for (uint8_t j = 0; j < kGroupDirs; ++j)
+            if (gr.side_qpat == kPattern[j]) gr.side_j = j;
+        out.groups.push_back(gr);
+    }
+    static constexpr uint16_t kPattern[kGroupDirs] = {0xaa, 0xcc, 0xf0};  // bit j of the register index
+
+    // The heaviest run of ops on at most four tile bits that mixes amplitudes
+    // (H, U2, U4) and is worth a GEMM (weight U4 4, U2 2, others 1; the first
+    // of equal weights), its bits padded from the top of the tile but never
+    // with the bits of an axis the block creates: until its EXPAND that half
+    // of the tile is not loaded, and the GEMM would multiply that memory (NaN or
+    // Inf possible) by the zero coefficients of the identity.
+    void find_dense(BlockPlan& b, uint64_t tile_bits, uint32_t avoid) {
+        const PlanOp* ops = out.ops.data() + b.first_op;
+        auto bits_of = [&](const PlanOp& o) -> uint32_t {
+            if (o.kind == M_EXPAND) return ~0u;
+            if ((o.ell[0] | o.ell[1]) & ~tile_bits) return ~0u;  // depends on tile-global bits
+            uint32_t x = o.lam[0] | (o.n_cond > 1 ? o.lam[1] : 0u);
+            if (o.kind == M_CX) x |= o.delta;
+            return x;
+        };
+        int best_w = int(g.dense_min_weight) - 1;
+        for (uint32_t j = 0; j < b.n_ops; ++j) {
+            uint32_t bits = 0, e = j;
+            bool mix = false;
+            int w = 0;
+            for (; e < b.n_ops; ++e) {
+                const uint32_t x = bits_of(ops[e]);
+                if (x == ~0u || popc(bits | x) > 4) break;
+                bits |= x;
+                mix |= ops[e].kind == M_H || ops[e].kind == M_U2 || ops[e].kind == M_U4;
+                w += ops[e].kind == M_U4 ? 4 : ops[e].kind == M_U2 ? 2 : 1;
+            }
+            if (e - j >= 2 && mix && w > best_w) {
+                best_w = w;
+                b.dense0 = j;
+                b.dense1 = e;
+                b.dense_mask = bits;
+            }
+        }
+        if (b.dense1)
+            for (int q = int(g.bits) - 1; popc(b.dense_mask) < 4 && q >= 0; --q)
+                if (!((avoid >> q) & 1u)) b.dense_mask |= 1u << q;
     }
 
-    // The block that starts at pc with active rank k; returns the number of
-    // instructions it takes, 0 for none.
-    uint32_t block(uint32_t pc, uint32_t k) {
-        const bool wide = g.max_ops > 1;
-        const bool single = k <= g.bits;
-        if (single && !(g.team && k >= kSingleMinRank)) return 0;
-        uint64_t need = 0, fresh = 0;
-        uint32_t slots = 0, sweeps = 0, kk = k, end = pc, term = 0, term_kind = 0;
+    // The block that starts at pc; returns the number of instructions it
+    // takes, 0 for none. Advances the layout past it.
+    uint32_t block(uint32_t pc) {
+        const bool wide = g.max_ops > 1, single = m.k <= g.bits;
+        if (single && !(g.team && m.k >= kSingleMinRank)) return 0;
+        const bool moves = !relabel || single;  // permutations move amplitudes
+        Layout l = m;
+        Span need;
+        std::vector<Op> ops;
+        uint32_t slots = 0, work = 0, end = pc, last = pc, n_fresh = 0;
+        uint32_t term = 0, term_kind = 0;
+        uint64_t cx_dir[2] = {0, 0}, cx_fun[2] = {0, 0}, side = 0;
+        uint32_t n_cx = 0;
+        // the directions of all ops so far; false when no tile holds them
+        auto fits = [&](Span& s) {
+            for (const Op& o : ops)
+                for (uint64_t d : o.dir)
+                    if (d) s.add(d);
+            if (s.v.size() > g.bits) return false;
+            return single || g.bits - Tile::of(s, g.bits).r <= (uint32_t)kMaxRunsLog2;
+        };
         for (; end < n; ++end) {
             const Instr x = decode(code, end);
-            uint64_t nd = 0;
-            uint32_t cost = 0, tk = 0;
-            bool expand = false, ok = true;
-            if (frame_op(x.op)) continue;
-            switch (x.op) {
-                case CLIFFT_OP_ARRAY_CNOT: nd = 1ull << x.a2; cost = 1; break;
-                case CLIFFT_OP_ARRAY_MULTI_CNOT: nd = 1ull << x.a1; cost = 1; break;
-                case CLIFFT_OP_ARRAY_SWAP:
-                case CLIFFT_OP_ARRAY_U4: nd = (1ull << x.a1) | (1ull << x.a2); cost = 1; break;
-                case CLIFFT_OP_ARRAY_H: nd = 1ull << x.a1; cost = 1; break;
-                case CLIFFT_OP_ARRAY_CZ:
-                case CLIFFT_OP_ARRAY_MULTI_CZ:
-                case CLIFFT_OP_ARRAY_S:
-                case CLIFFT_OP_ARRAY_S_DAG: cost = 1; break;
-                case CLIFFT_OP_ARRAY_T:
-                case CLIFFT_OP_ARRAY_T_DAG:
-                case CLIFFT_OP_ARRAY_ROT: cost = x.a1 < kk ? 1 : 0; break;
-                case CLIFFT_OP_ARRAY_U2:
-                    if (x.a1 < kk) {
-                        nd = 1ull << x.a1;
-                        cost = 1;
-                    }
-                    break;
-                case CLIFFT_OP_EXPAND:
-                case CLIFFT_OP_EXPAND_T:
-                case CLIFFT_OP_EXPAND_T_DAG:
-                case CLIFFT_OP_EXPAND_ROT:
-                    ok = wide && !(single && kk == g.bits);
-                    nd = 1ull << kk;
-                    cost = 2;
-                    expand = true;
-                    break;
-                case CLIFFT_OP_MEAS_ACTIVE_DIAGONAL:
-                    ok = wide;
-                    tk = 1;
-                    if (single) nd = 1ull << (kk - 1);
-                    break;
-                case CLIFFT_OP_MEAS_ACTIVE_INTERFERE:
-                    ok = wide;
-                    tk = 2;
-                    nd = 1ull << (kk - 1);
-                    cost = 1;
-                    break;
-                case CLIFFT_OP_SWAP_MEAS_INTERFERE:
-                    ok = wide;
-                    tk = x.a1 != x.a2 ? 3 : 2;
-                    nd = (1ull << x.a1) | (1ull << x.a2);
-                    cost = tk == 3 ? 2 : 1;
-                    break;
-                default: ok = false;
+            if (is_scalar(x.op)) {
+                if (!wide && !frame_op(x.op)) break;
+                continue;
             }
-            if (!ok) break;
-            const uint64_t cand = need | nd;
-            if (popc(cand) > g.bits || slots + cost > g.max_ops) break;
-            if (nd && !single) {
-                uint32_t r;
-                tile_axes(cand, r);
-                if (g.bits - r > (uint32_t)kMaxRunsLog2) break;
+            if (x.op == CLIFFT_OP_EXP_VAL || x.op == CLIFFT_OP_POSTSELECT) break;
+            Layout l2 = l;
+            uint32_t slots2 = slots;
+            const std::vector<Op> keep = ops;
+            uint32_t n_cx2 = 0;
+            uint64_t d2[2] = {0, 0}, f2[2] = {0, 0};
+            uint32_t tk = 0;
+            if (is_expand(x.op)) {
+                if (!wide || (single && l.k == g.bits)) break;
+                emit(x, l2, moves, ops, slots2);
+            } else if (is_active_meas(x.op)) {
+                if (!wide) break;
+                const uint32_t t = l.k - 1;
+                tk = x.op == CLIFFT_OP_MEAS_ACTIVE_DIAGONAL ? 1
+                     : (x.op == CLIFFT_OP_SWAP_MEAS_INTERFERE && x.a1 != x.a2) ? 3 : 2;
+                if (tk == 3) {
+                    Instr sw = x;
+                    sw.op = CLIFFT_OP_ARRAY_SWAP;
+                    emit(sw, l2, moves, ops, slots2);
+                }
+                if (tk >= 2) {
+                    Op o;
+                    o.kind = M_H;
+                    o.dir[0] = l2.col[t];
+                    o.ell[0] = l2.ell[t];
+                    o.n_cond = 1;
+                    ops.push_back(o);
+                }
+                side = l2.ell[t];
+                // make the measured bit the top physical bit
+                auto swap_along = [&](uint64_t dir, uint64_t fun) {
+                    Op o;
+                    o.kind = M_CX;
+                    o.flags = MF_LINEAR;
+                    o.dir[0] = dir;
+                    // as a condition on the index before the first swap
+                    o.ell[0] = fun ^ (n_cx2 && parity(fun & d2[0]) ? f2[0] : 0ull);
+                    o.n_cond = 1;
+                    ops.push_back(o);
+                    d2[n_cx2] = dir;
+                    f2[n_cx2++] = fun;
+                    l2.move(dir, fun);
+                };
+                const uint64_t tb = 1ull << t;
+                if (l2.ell[t] != tb) {
+                    if (!(l2.ell[t] & tb)) swap_along(1ull << top_bit(l2.ell[t]), tb);
+                    if (l2.ell[t] != tb) swap_along(tb, l2.ell[t] ^ tb);
+                }
+            } else {
+                emit(x, l2, moves, ops, slots2);
             }
-            need = cand;
-            slots += cost;
-            if (expand) {
-                fresh |= 1ull << kk;
-                kk++;
-            } else if (cost && !tk) {
-                sweeps++;
+            // the slots a coefficient or a moved opcode takes (a measurement's
+            // own swaps have room beyond max_ops)
+            Span s;
+            if (ops.size() - n_cx2 > g.max_ops || slots2 > g.max_ops || !fits(s)) {
+                ops = keep;
+                break;
             }
+            need = s;
+            l = l2;
+            slots = slots2;
+            if (is_expand(x.op))
+                ++n_fresh;
+            else if (touches_at(x, l.k) && !tk)
+                ++work;
+            last = end + 1;
             if (tk) {
                 term = end++;
                 term_kind = tk;
+                n_cx = n_cx2;
+                for (int c = 0; c < 2; ++c) {
+                    cx_dir[c] = d2[c];
+                    cx_fun[c] = f2[c];
+                }
+                break;
+            }
+            if (!wide) {
+                ++end;
                 break;
             }
         }
+        end = last;  // what follows the last opcode on the statevector needs no block
         // a block of EXPANDs alone costs more than the plain expansions
-        if (sweeps < 1 && !term_kind) return 0;
-        BlockPlan p{};
-        p.pc = pc;
-        p.n_instr = end - pc;
-        p.F = tile_axes(single ? 0 : need, p.r);
-        p.C = single ? 0 : ((kk == 64) ? ~0ull : ((1ull << kk) - 1)) & ~p.F;
-        p.kk = kk;
-        p.single = single;
-        p.n_fresh = popc(fresh);
-        p.term_kind = term_kind;
-        p.term_pc = term;
-        for (uint64_t w = fresh; w; w &= w - 1) {
-            const uint32_t at = popc(p.F & ((w & (~w + 1)) - 1));
-            p.fresh_local |= 1u << at;
-            if (!single) p.skip |= 1u << (at - p.r);
+        if (work < 1 && !term_kind) return 0;
+        BlockPlan b{};
+        const Tile t = Tile::of(single ? Span{} : need, g.bits);
+        b.kind = BLOCK_PASS;
+        b.pc = pc;
+        b.n_instr = end - pc;
+        b.kk = l.k;
+        b.r = t.r;
+        b.single = single;
+        b.n_fresh = n_fresh;
+        b.term_kind = term_kind;
+        b.term_pc = term;
+        b.n_cx = n_cx;
+        for (int c = 0; c < 2; ++c) {
+            b.cx_dir[c] = cx_dir[c];
+            b.cx_fun[c] = cx_fun[c];
         }
-        p.first_mop = (uint32_t)out.ops.size();
-        Emit e{p.F, out.ops};
-        uint32_t rank = k;
-        for (uint32_t q = pc; q < (term_kind ? term : end); ++q) {
-            const Instr x = decode(code, q);
-            emit(e, x, rank);
-            if (is_expand(x.op)) rank++;
+        b.C = single ? 0 : ((l.k == 64 ? ~0ull : (1ull << l.k) - 1) & ~t.pivots());
+        for (uint32_t j = t.r; j < g.bits; ++j) b.hb[j - t.r] = t.basis[j];
+        uint32_t fresh_local = 0;
+        for (uint32_t a = l.k - n_fresh; a < l.k && n_fresh; ++a) {
+            fresh_local |= t.position(1ull << a);
+            if (!single) b.skip |= t.position(1ull << a) >> t.r;
         }
-        p.n_body = (uint32_t)out.ops.size() - p.first_mop;
         if (term_kind) {
-            const Instr x = decode(code, term);
-            const uint32_t fa = x.a1, tt = term_kind == 3 ? x.a2 : x.a1;
-            if (term_kind == 3) e(M_SWAP, fa, tt, 0, 0, 0);
-            if (term_kind >= 2) e(M_H, tt, tt, 0, 0, 0);
-            p.red_local = (p.F >> tt) & 1u;
-            p.red_bit = p.red_local ? popc(p.F & ((1ull << tt) - 1)) : tt;
+            b.dvec = l.col[l.k - 1];
+            b.side_ell = side;
+            b.side_lam = t.functional(side);
         }
-        p.n_mops = (uint32_t)out.ops.size() - p.first_mop;
-        compile_runs(out.ops.data() + p.first_mop, p.n_mops);
-        out.blocks.push_back(p);
+        b.store = !ops.empty();
+        b.first_op = (uint32_t)out.ops.size();
+        b.n_ops = (uint32_t)ops.size();
+        for (const Op& o : ops) {
+            PlanOp p{};
+            p.kind = o.kind;
+            p.flags = o.flags;
+            p.slot = o.slot;
+            p.n_cond = o.n_cond;
+            for (int c = 0; c < o.n_cond; ++c) {
+                p.lam[c] = t.functional(o.ell[c]);
+                p.ell[c] = o.ell[c];
+            }
+            if (o.dir[0]) p.delta = (uint16_t)t.position(o.dir[0]);
+            out.ops.push_back(p);
+        }
+        if (g.dense_min_weight) find_dense(b, t.pivots(), fresh_local);
+        // groups
+        auto join_again = [](const Op& o, const Tile& tile, std::vector<uint32_t>& into) {
+            for (uint64_t d : o.dir) {
+                if (!d) continue;
+                const uint32_t v = tile.position(d);
+                if (std::find(into.begin(), into.end(), v) == into.end()) into.push_back(v);
+            }
+        };
+        b.first_group = (uint32_t)out.groups.size();
+        std::vector<uint32_t> dirs;
+        uint32_t op0 = 0;
+        auto close = [&](uint32_t op1, bool fin) {
+            close_group(op0, op1, dirs, b, fin);
+            dirs.clear();
+            op0 = op1;
+        };
+        const uint32_t fin0 = b.n_ops - b.n_cx;
+        for (uint32_t i = 0; i < b.n_ops; ++i) {
+            if (b.dense1 && i == b.dense0) {
+                // its own pass: the ops become one matrix
+                if (i > op0) close(i, false);
+                op0 = b.dense1;
+                i = b.dense1 - 1;
+                continue;
+            }
+            const Op& o = ops[i];
+            if (!o.dir[0]) continue;
+            auto try_join = [&]() -> bool {
+                std::vector<uint32_t> want{t.position(o.dir[0])};
+                if (o.kind == M_U4) want.push_back(t.position(o.dir[1]));
+                uint32_t j = 0;
+                for (uint32_t w = 0; w < want.size(); ++w) {
+                    const auto at = std::find(dirs.begin(), dirs.end(), want[w]);
+                    uint32_t idx = uint32_t(at - dirs.begin());
+                    if (at == dirs.end()) {
+                        Span s;
+                        for (uint32_t d : dirs) s.add(d);
+                        if (dirs.size() >= kGroupDirs || !s.reduce(want[w])) return false;
+                        dirs.push_back(want[w]);
+                    }
+                    if (o.kind == M_U4 && idx != w) return false;  // U4 owns the first two directions
+                    if (w == 0) j = idx;
+                }
+                out.ops[b.first_op + i].j = (uint8_t)j;
+                return true;
+            };
+            const std::vector<uint32_t> before = dirs;
+            if (!try_join()) {
+                dirs = before;
+                // the two swaps before a measurement stay together
+                if (i > fin0) {
+                    i = fin0;
+                    dirs.clear();
+                    for (uint32_t q = op0; q < fin0; ++q) join_again(ops[q], t, dirs);
+                }
+                close(i, false);
+                --i;  // again, in the new group
+            }
+        }
+        // the closing group also sums a measured axis' halves; a dense run at
+        // the very end leaves an empty one for that
+        if (b.n_ops > op0 || term_kind) close(b.n_ops, true);
+        b.n_groups = (uint32_t)out.groups.size() - b.first_group;
+        // the layout after the block
+        m = l;
+        if (term_kind) {
+            const uint32_t top = --m.k;
+            const uint64_t live = (1ull << top) - 1;
+            for (uint32_t a = 0; a < top; ++a) {
+                m.col[a] &= live;  // already without the top bit
+                m.ell[a] &= live;
+            }
+        }
+        if (!moves && !l.identity()) dirty = true;
+        if (dirty && m.k <= g.bits) {
+            b.cols_at = (uint32_t)out.cols.size();
+            b.cols_n = m.k;
+            for (uint32_t a = 0; a < m.k; ++a) out.cols.push_back(m.col[a]);
+            reset_layout();
+        }
+        out.blocks.push_back(b);
         return end - pc;
+    }
+    // an opcode (not an EXPAND) that works on the statevector at rank k
+    static bool touches_at(const Instr& x, uint32_t k) {
+        switch (x.op) {
+            case CLIFFT_OP_ARRAY_T:
+            case CLIFFT_OP_ARRAY_T_DAG:
+            case CLIFFT_OP_ARRAY_ROT:
+            case CLIFFT_OP_ARRAY_U2: return x.a1 < k;
+            default: return x.op >= CLIFFT_OP_ARRAY_CNOT && x.op <= CLIFFT_OP_ARRAY_U4;
+        }
+    }
+    void reset_layout() {
+        const uint32_t k = m.k;
+        m.k = 0;
+        while (m.k < k) m.expand();
+        dirty = false;
     }
 
     void build() {
-        uint32_t k = 0;
+        relabel = g.max_ops > 1 && !g.dense_min_weight;
+        for (uint32_t pc = 0; pc < n; ++pc)
+            if (decode(code, pc).op == CLIFFT_OP_POSTSELECT) relabel = false;  // segments save states in logical order
         for (uint32_t pc = 0; pc < n;) {
             const Instr x = decode(code, pc);
             uint32_t used = 0;
-            // a CTA's control warp runs opcodes that do not touch the
-            // statevector by itself; a warp offers every opcode to a block
-            if (!frame_op(x.op) && (!g.cta || touches(x, k))) used = block(pc, k);
-            for (uint32_t q = pc; q < pc + (used ? used : 1); ++q) {
-                const uint32_t op = decode(code, q).op;
-                if (is_expand(op)) ++k;
-                if (is_active_meas(op)) --k;
+            if (x.op == CLIFFT_OP_EXP_VAL) {
+                if (dirty) {
+                    BlockPlan b{};
+                    b.kind = BLOCK_EXP_VAL;
+                    b.pc = pc;
+                    b.n_instr = 1;
+                    b.kk = m.k;
+                    const uint64_t act = m.k == 64 ? ~0ull : (1ull << m.k) - 1;
+                    b.hb[0] = m.col_of(exp_x[size_t(x.p0) * exp_words] & act);
+                    b.hb[1] = m.ell_of(exp_z[size_t(x.p0) * exp_words] & act);
+                    out.blocks.push_back(b);
+                    used = 1;
+                }
+            } else if (!is_scalar(x.op) && touches(x)) {
+                used = block(pc);
             }
-            pc += used ? used : 1;
+            if (!used) {
+                if (is_expand(x.op)) m.expand();
+                if (is_active_meas(x.op)) --m.k;
+                used = 1;
+            }
+            pc += used;
         }
         BlockPlan last{};
+        last.kind = BLOCK_END;
         last.pc = kNoPlan;
+        if (dirty) {
+            last.cols_at = (uint32_t)out.cols.size();
+            last.cols_n = m.k;
+            for (uint32_t a = 0; a < m.k; ++a) out.cols.push_back(m.col[a]);
+        }
         out.blocks.push_back(last);
     }
 };
 
 }  // namespace
 
-PlanSet plan_blocks(const uint8_t* code, uint32_t n_code, const PlanGeometry& g) {
-    Builder b{code, n_code, g, {}};
+PlanSet plan_blocks(const uint8_t* code, uint32_t n_code, const PlanGeometry& g, const uint64_t* exp_x,
+                    const uint64_t* exp_z, uint32_t exp_words) {
+    Builder b{code, n_code, g, exp_x, exp_z, exp_words};
     b.build();
     return std::move(b.out);
 }

@@ -1,7 +1,22 @@
 // Fused blocks formed on the host. Which opcodes share one pass over the
-// statevector depends only on the program (opcodes, axes, active ranks) and on
-// the tile geometry, so the blocks of a program are planned once per geometry
-// and a shot only fills in what its Pauli frame decides: the coefficients.
+// statevector, and where every amplitude lies, depends only on the program
+// (opcodes, axes, active ranks) and on the tile geometry, so the blocks of a
+// program are planned once per geometry and a shot only fills in what its
+// Pauli frame decides: the coefficients.
+//
+// Index spaces. Logical amplitude i of a tiled state lies at physical index
+// p = M i ^ xl, with M an invertible matrix over GF(2) and xl a vector that
+// measurement outcomes decide. CNOT, multi-CNOT and SWAP only change M
+// (relabelling: no amplitude moves); what the other opcodes need of M is
+// planned:
+//   * logical axis a is the direction M e_a (moving along it flips those
+//     physical bits), and its bit at p is the parity of (p ^ xl) & ell_a, a row
+//     of M^-1;
+//   * a tile is a coset of a span of 2^bits physical indices that contains the
+//     directions its opcodes move along; tile position l stands for
+//     base ^ (low r bits of l) ^ the high basis vectors that l's other bits pick;
+//   * a measured axis is first made the top physical bit (in-tile conditional
+//     swaps), so that the half that is kept is contiguous.
 #pragma once
 
 #include <cstdint>
@@ -9,55 +24,103 @@
 
 namespace cgpu {
 
+enum : uint8_t {
+    M_PHASE,   // times c[0] where every condition holds
+    M_NEG,     // negated where every condition holds
+    M_CX,      // swapped along a direction where the condition holds
+    M_H,       // (x + y, x - y) / sqrt2 along a direction
+    M_U2,      // 2 x 2 matrix along a direction
+    M_U4,      // 4 x 4 matrix along the first two directions of its group
+    M_EXPAND,  // the clear half copied (times c[0]) onto the set half; then times the next slot's
+               // c[0].x if its c[0].y is not zero (a renormalisation)
+};
+enum : uint8_t {
+    MF_COPY = 0x1,    // EXPAND without a phase
+    MF_LINEAR = 0x2,  // the condition is on the physical index (it does not see xl)
+};
+
+// A micro-op. Condition c holds at tile position l of a tile at `base` when
+// the parity of l & lam[c], base & ell[c] and xl & ell[c] is odd. For the
+// opcodes along a direction, condition 0 tells the side (its logical bit; U4:
+// conditions 0 and 1 those of its two axes).
+struct PlanOp {
+    uint8_t kind, j, n_cond, flags;  // j: which of its group's directions
+    uint16_t lam[2];
+    uint16_t qpat[2];  // lam over the group's 2^q register indices, as a bit mask
+    uint8_t slot, pad;  // coefficients
+    uint16_t delta;     // the direction in tile positions (U4: its low axis)
+    uint64_t ell[2];
+};
+static_assert(sizeof(PlanOp) == 32, "copied in 16-byte words");
+
+// Consecutive micro-ops that one pass over the tile applies in registers: a
+// thread holds the 8 amplitudes that the group's directions connect.
+struct PlanGroup {
+    uint16_t qv[3];      // directions (tile positions); unused ones are free unit vectors
+    uint8_t op0, op1;
+    uint8_t piv[3];      // their pivot bits, ascending: a coset's base has them clear
+    uint8_t n_fin;       // swaps before a measurement (ops from op1), made by where the amplitudes are stored
+    uint16_t side_qpat;  // last group of a measured block: the measured axis' bit
+    uint8_t n_exp;       // leading EXPANDs along directions 0, 1, .. whose clear halves are the
+                         // registers with those index bits clear
+    uint8_t side_j;      // side_qpat is that of direction 0..2, SIDE_NONE: zero, SIDE_ANY: another
+    uint16_t sv[3];      // where a coset is stored: its base, moved along the swaps' directions as
+                         // their conditions there say, and these directions
+    uint16_t fin_lam[2], fin_dir[2];  // the swaps: conditions and directions (none: 0)
+    uint16_t pad;
+};
+enum : uint8_t { SIDE_NONE = 3, SIDE_ANY = 4 };
+static_assert(sizeof(PlanGroup) == 32, "copied in 16-byte words");
+
+enum : uint32_t { BLOCK_PASS, BLOCK_EXP_VAL, BLOCK_END };
+
 // One fused block: instructions [pc, pc + n_instr) of the device stream.
+// BLOCK_EXP_VAL: an EXP_VAL on a relabelled state (hb[0], hb[1]: its X mask as
+// a direction, its Z mask as a functional). BLOCK_END closes the list (pc =
+// 0xffffffff); its columns are M at the end of the program.
 struct BlockPlan {
-    uint64_t F;          // tile axes
-    uint64_t C;          // the other axes of the 2^kk amplitudes
-    uint32_t pc;         // 0xffffffff closes the list
-    uint32_t n_instr;
-    uint32_t first_mop;  // its micro-ops in the plan's PlanOp array
-    uint32_t n_mops;     // with a terminating measurement's own (SWAP, H)
-    uint32_t n_body;     // without them
+    uint64_t C;       // physical bits that number the tiles
+    uint64_t hb[6];   // high basis vectors of a tile
+    uint64_t dvec;    // measured axis: its direction
+    uint64_t cx_dir[2], cx_fun[2];  // the swaps that make it the top bit, as maps of xl
+    uint32_t kind;
+    uint32_t pc, n_instr;
+    uint32_t first_op, n_ops, first_group, n_groups;
     uint32_t r;          // log2 of a tile's contiguous runs
     uint32_t kk;         // active rank while the block streams
     uint32_t skip;       // run-index bits of the axes the block creates (not loaded)
-    uint32_t n_fresh;    // how many axes it creates
-    uint32_t fresh_local;  // their tile-local bits
+    uint32_t n_fresh;    // how many
+    uint32_t store;      // the pass changes the state
     uint32_t term_kind;  // measurement ending it: 0 none, 1 diagonal, 2 X basis, 3 X basis with a fused swap
     uint32_t term_pc;
-    uint32_t red_local;  // the measured axis is a tile axis ...
-    uint32_t red_bit;    // ... with this local bit, or its tile-global bit
+    uint32_t n_cx;
+    uint32_t side_lam;   // the measured axis' bit over tile positions
+    uint64_t side_ell;   // and as a functional
     uint32_t single;     // the state is one tile, already in shared memory
-    uint32_t pad;
+    uint32_t cols_at, cols_n;  // columns of M (PlanSet::cols) to undo it after the block; 0: nothing to undo
+    uint32_t dense0, dense1, dense_mask;  // dense geometry: ops [dense0, dense1) as one matrix on those four tile bits
 };
-static_assert(sizeof(BlockPlan) == 80 && sizeof(BlockPlan) % 16 == 0, "copied in 16-byte words");
-
-// The frame-independent part of a micro-op, laid out like the head of
-// MicroOpT, then what an index run keeps in unused coefficient slots: the
-// rows of a diagonal op and (first op of a run) the columns of the final map.
-struct PlanOp {
-    uint8_t kind, a, b, flags;
-    uint32_t req, par, pad;
-    uint64_t greq, gpar;
-    uint16_t row[3];
-    uint8_t n_rows, pad2;
-    uint16_t cols[12];
-};
-static_assert(sizeof(PlanOp) == 64, "copied in 16-byte words");
+static_assert(sizeof(BlockPlan) % 16 == 0, "copied in 16-byte words");
 
 struct PlanGeometry {
     uint32_t bits;     // log2 of the amplitudes per tile
     uint32_t max_ops;  // micro-op slots per block (1: one opcode per pass)
-    bool cta;          // a CTA per shot (scalar opcodes between blocks run on its control warp)
-    bool team;         // ... which keeps states of at most one tile in shared memory
+    bool team;         // a team of CTAs, which keeps states of at most one tile in shared memory
+    uint32_t dense_min_weight;  // > 0: find runs for the tensor cores (no relabelling then)
 };
+constexpr uint32_t kGroupDirs = 3;  // log2 of the amplitudes a thread holds
+constexpr uint32_t kExtraOps = 2;  // micro-ops beyond max_ops: the swaps before a measurement
 
 struct PlanSet {
-    std::vector<BlockPlan> blocks;  // by pc, closed by a block with pc = 0xffffffff
+    std::vector<BlockPlan> blocks;  // by pc, closed by BLOCK_END
     std::vector<PlanOp> ops;
+    std::vector<PlanGroup> groups;
+    std::vector<uint64_t> cols;
 };
 
-// The blocks of the device instruction stream `code` (32 bytes each).
-PlanSet plan_blocks(const uint8_t* code, uint32_t n_code, const PlanGeometry& g);
+// The blocks of the device instruction stream `code` (32 bytes each). exp_x /
+// exp_z: first words of the EXP_VAL masks, `exp_words` words apart.
+PlanSet plan_blocks(const uint8_t* code, uint32_t n_code, const PlanGeometry& g, const uint64_t* exp_x,
+                    const uint64_t* exp_z, uint32_t exp_words);
 
 }  // namespace cgpu
