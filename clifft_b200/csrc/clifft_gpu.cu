@@ -931,26 +931,35 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
 }
 
 // Team size for an untuned launch of `shots` shots (as a group request), or 0
-// when a warp per shot is the better shape. A launch of C CTAs per shot runs
+// when a warp per shot (states up to 1 MiB) or a CTA of 128 threads per shot
+// (larger ones, three resident per SM) is the better shape. A launch of C CTAs per shot runs
 // ceil(shots / teams) rounds, each of which costs about
 //     kOpUs x (opcodes on the statevector) + kTileUs x (tiles they cover) / C:
 // every CTA of a team interprets the whole program, so the first part does
 // not shrink with C; a CTA that has its SM to itself computes its tiles
 // faster (kAlone). Warps take all shots in one round, at
 //     kWarpOpUs x opcodes + kWarpTileUs x (warp tiles they cover).
-// Measured (B200): k = 24 FP32, 147 opcodes, 117216 tiles: 76 ms / C + 0.8 ms;
-// k = 20 FP32, 394 opcodes, 75336 tiles: 85 ms / C + 1.5 ms; k = 18 FP64, 73
-// opcodes, 2670 tiles: 2.1 ms / C + 0.5 ms. One shot of the k = 24 program
-// takes 1.0 ms with 296 CTAs, 57 ms with one; 148 shots 41 ms with teams of
-// two, 60 ms with one CTA each. Warps against teams of one, FP32: k = 14, 296
-// shots 0.37 / 0.32 ms, 592 shots 0.38 / 0.64 ms; k = 16, 296 shots 0.89 /
-// 0.51, 592 shots 0.91 / 1.00; k = 17, 592 shots 1.89 / 1.48, 1000 shots
-// 2.1 / 2.8; k = 12 0.16 / 0.18 at any count.
+// CTAs of 128 threads take the shots in rounds of three per SM, at
+//     kOpUs x opcodes + kCtaTileUs x tiles.
+// Opcodes and tiles are counted before blocks form: what a tile costs depends
+// on how many opcodes share a pass (0.43 us at k = 24, 147 opcodes; 0.6 us at
+// k = 18; 1.08 us at k = 20, 394 opcodes that mix amplitudes), and kTileUs
+// lies between.
+// Measured (B200), ms: one shot of k = 24 FP32 0.85 with 296 CTAs, 19 with two,
+// 37 with one; 148 shots 26 with teams of two, 38 with one CTA each, 123 with
+// all CTAs on each shot in turn; k = 20, 150 shots 82 / 64 / 56 / 61 / 81 with
+// teams of 1 / 4 / 8..16 / 37 / 74. Warps against teams of one, FP32: k = 14,
+// 296 shots 0.33 / 0.30, 592 shots 0.34 / 0.58; k = 16, 296 shots 0.87 / 0.44,
+// 592 shots 0.87 / 0.85, 1000 shots 0.95 / 1.62; k = 17, 592 shots 1.60 / 1.14,
+// 1000 shots 1.76 / 2.21; k = 12 0.17 / 0.17 up to 64 shots, 0.17 / 0.21 from
+// 150 on. CTAs of 128 threads against teams of one: k = 17 FP64, 296 shots
+// 0.87 / 1.02, 1000 shots 2.7 / 4.0; k = 18 FP64, 296 shots 2.15 / 2.11, 1000
+// shots 6.9 / 8.3; k = 18 FP32, 296 shots 1.36 / 1.03, 1000 shots 4.07 / 4.02.
 uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_t shots, uint32_t max_resident) {
     constexpr double kOpUs = 3.2, kTileUs = 0.8, kAlone = 0.7, kWarpOpUs = 2.3;
     constexpr uint32_t kPerSm = 2;
     const bool fp64 = precision == CLIFFT_GPU_FP64;
-    const double kWarpTileUs = fp64 ? 0.44 : 0.37;
+    const double kWarpTileUs = fp64 ? 0.44 : 0.37, kCtaTileUs = fp64 ? 0.775 : 1.1;
     const uint32_t peak = p.meta.peak_rank;
     const uint32_t bits = fp64 ? TileCfg<double, true>::kBits : TileCfg<float, true>::kBits;
     const uint32_t warp_bits = fp64 ? TileCfg<double, false>::kBits : TileCfg<float, false>::kBits;
@@ -989,8 +998,14 @@ uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_
         consider(teams, std::min<uint64_t>(cap / teams, peak_tiles));
         if (teams <= uint64_t(sms)) consider(teams, 1);
     }
-    // a warp per shot is the default up to 1 MiB
-    if (state_bytes <= (size_t(1) << 20) && kWarpOpUs * ops + kWarpTileUs * warp_tiles <= best) return 0;
+    // a warp per shot is the default up to 1 MiB, then a CTA of 128 threads
+    if (state_bytes <= (size_t(1) << 20)) {
+        if (kWarpOpUs * ops + kWarpTileUs * warp_tiles <= best) return 0;
+    } else {
+        uint64_t at_once = std::max<uint64_t>(1, std::min<uint64_t>(3ull * sms, (free_b / 2) / state_bytes));
+        if (max_resident) at_once = std::min<uint64_t>(at_once, max_resident);
+        if (double((shots + at_once - 1) / at_once) * (kOpUs * ops + kCtaTileUs * tiles) < best) return 0;
+    }
     return team_request(ctas);
 }
 
