@@ -940,7 +940,8 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
 // faster (kAlone). Warps take all shots in one round, at
 //     kWarpOpUs x opcodes + kWarpTileUs x (warp tiles they cover).
 // CTAs of 128 threads take the shots in rounds of three per SM, at
-//     kOpUs x opcodes + kCtaTileUs x tiles.
+//     kOpUs x opcodes + kCtaTileUs x tiles;
+// they are considered for more shots than two rounds of teams of one take.
 // Opcodes and tiles are counted before blocks form: what a tile costs depends
 // on how many opcodes share a pass (0.43 us at k = 24, 147 opcodes; 0.6 us at
 // k = 18; 1.08 us at k = 20, 394 opcodes that mix amplitudes), and kTileUs
@@ -952,9 +953,9 @@ LaunchPlan plan_launch(const clifft_gpu_program& p, uint32_t precision, uint32_t
 // 296 shots 0.33 / 0.30, 592 shots 0.34 / 0.58; k = 16, 296 shots 0.87 / 0.44,
 // 592 shots 0.87 / 0.85, 1000 shots 0.95 / 1.62; k = 17, 592 shots 1.60 / 1.14,
 // 1000 shots 1.76 / 2.21; k = 12 0.17 / 0.17 up to 64 shots, 0.17 / 0.21 from
-// 150 on. CTAs of 128 threads against teams of one: k = 17 FP64, 296 shots
-// 0.87 / 1.02, 1000 shots 2.7 / 4.0; k = 18 FP64, 296 shots 2.15 / 2.11, 1000
-// shots 6.9 / 8.3; k = 18 FP32, 296 shots 1.36 / 1.03, 1000 shots 4.07 / 4.02.
+// 150 on. CTAs of 128 threads against teams of one: k = 17 FP64, 1000 shots
+// 2.7 / 4.0; k = 18 FP64, 296 shots 2.15 / 2.11, 592 shots 4.5 / 4.2, 1000
+// shots 6.9 / 8.3; k = 18 FP32, 592 shots 2.76 / 2.05, 1000 shots 4.07 / 4.02.
 uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_t shots, uint32_t max_resident) {
     constexpr double kOpUs = 3.2, kTileUs = 0.8, kAlone = 0.7, kWarpOpUs = 2.3;
     constexpr uint32_t kPerSm = 2;
@@ -1001,7 +1002,7 @@ uint32_t team_heuristic(const clifft_gpu_program& p, uint32_t precision, uint64_
     // a warp per shot is the default up to 1 MiB, then a CTA of 128 threads
     if (state_bytes <= (size_t(1) << 20)) {
         if (kWarpOpUs * ops + kWarpTileUs * warp_tiles <= best) return 0;
-    } else {
+    } else if (shots > 2 * cap) {  // two rounds of teams of one are still the better choice (592 shots: 4.2 / 4.6 ms)
         uint64_t at_once = std::max<uint64_t>(1, std::min<uint64_t>(3ull * sms, (free_b / 2) / state_bytes));
         if (max_resident) at_once = std::min<uint64_t>(at_once, max_resident);
         if (double((shots + at_once - 1) / at_once) * (kOpUs * ops + kCtaTileUs * tiles) < best) return 0;
