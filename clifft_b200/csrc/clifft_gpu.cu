@@ -699,7 +699,7 @@ clifft_gpu_program::Plans block_plans(clifft_gpu_program& p, uint32_t precision,
     if (e.dev) return e;
     auto geometry = [&](auto cfg) {
         using TC = decltype(cfg);
-        return PlanGeometry{uint32_t(TC::kBits), L.fuse ? uint32_t(TC::kMops) : 1u, team,
+        return PlanGeometry{uint32_t(TC::kBits), L.fuse ? uint32_t(TC::kMops) : 1u, cta, team,
                             L.dense ? dense_min_weight() : 0u};
     };
     const PlanGeometry g = precision == CLIFFT_GPU_FP32

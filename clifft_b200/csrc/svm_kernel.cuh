@@ -495,9 +495,9 @@ struct Tally {
 //     Such programs, and those with a POSTSELECT, are not relabelled.
 // Measured (B200), kernel ms, blocks that end at a scalar opcode and move
 // amplitudes for CNOT and SWAP -> these: k = 16 FP32, 10^4 shots 7.0 -> 6.4 and
-// k = 14 2.84 -> 2.42 (warps); k = 18 FP32, 4000 shots 16.8 -> 10.9; k = 20,
-// 394 opcodes, 150 shots 69 -> 53; k = 24, 148 shots 41 -> 26, one shot 1.02 ->
-// 0.86. The streamed bytes shrink 2.2 to 3.3 times, so HBM is no longer the
+// k = 14 2.84 -> 2.46 (warps); k = 18 FP32, 4000 shots 16.8 -> 10.8; k = 20,
+// 394 opcodes, 150 shots 69 -> 48; k = 24, 148 shots 41 -> 23.5, one shot 1.02
+// -> 0.86. The streamed bytes shrink 2.2 to 3.3 times, so HBM is no longer the
 // bound; what is: the instructions per tile, at 16 warps per SM.
 constexpr int kMaxStages = 4;      // tile buffers (tiles in flight) per shot group: 2..4, chosen per launch
 constexpr int kMaxRunsLog2 = 6;    // at most 64 contiguous runs per tile
@@ -2800,47 +2800,72 @@ struct Shot {
                                               double (&acc)[2]) {
         constexpr uint32_t UNITS = (1u << TC::kBits) / kRegs, ALL = (1u << kRegs) - 1u;
         const uint4* op = reinterpret_cast<const uint4*>(ops());
-        const uint32_t side_lam = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset)->side_lam;
+        const BlockPlan* bp = reinterpret_cast<const BlockPlan*>(fuse + TC::kPlanOffset);
+        // the tile's part of the axis bits
+        auto axis = [&](uint32_t j) -> uint32_t {
+            const uint32_t at = gr.axis_at[j];
+            return ((at & 32u) ? tp1 : tp0) >> (at & 31u);
+        };
+        uint32_t a0 = 0, a1 = 0, a2 = 0;
+        const bool axes = kAxes && gr.axes != 0;
+        if (axes) a0 = axis(0), a1 = axis(1), a2 = axis(2);
         const uint32_t o1 = gr.qv[0], o2 = gr.qv[1], o4 = gr.qv[2];
+        // FP32 keeps these in registers; FP64 has none to spare and reads them
+        // again per coset (k = 20, 150 shots 86 against 93 ms; FP32 49 against 48)
+        constexpr bool KEEP = sizeof(R) == 4;
+        const uint32_t g0 = gr.op0, g1 = gr.op1, gx = any_scale ? 0u : gr.n_exp;
         const uint32_t o3 = o1 ^ o2, o5 = o1 ^ o4, o6 = o2 ^ o4, o7 = o3 ^ o4;
         for (uint32_t u = (uint32_t)tid; u < UNITS; u += (uint32_t)nthr) {
-            const uint32_t base = ins0_32(ins0_32(ins0_32(u, gr.piv[0]), gr.piv[1]), gr.piv[2]);
+            uint32_t base = ins0_32(ins0_32(ins0_32(u, gr.piv[0]), gr.piv[1]), gr.piv[2]);
+            if (axes) {
+                const uint32_t b0 = (uint32_t)__popc(base & gr.axis_lam[0]) ^ a0;
+                const uint32_t b1 = (uint32_t)__popc(base & gr.axis_lam[1]) ^ a1;
+                const uint32_t b2 = (uint32_t)__popc(base & gr.axis_lam[2]) ^ a2;
+                base ^= ((b0 & 1u) ? o1 : 0u) ^ ((b1 & 1u) ? o2 : 0u) ^ ((b2 & 1u) ? o4 : 0u);
+            }
             const uint32_t pos[kRegs] = {base,      base ^ o1, base ^ o2, base ^ o3,
                                    base ^ o4, base ^ o5, base ^ o6, base ^ o7};
             T x[kRegs];
+            const uint32_t op0 = KEEP ? g0 : gr.op0, op1 = KEEP ? g1 : gr.op1;
+            const uint32_t n_exp = KEEP ? gx : any_scale ? 0u : gr.n_exp;
             // leading EXPANDs read the clear half only
-            const uint32_t n_exp = any_scale ? 0u : gr.n_exp;
             if (n_exp == 0)
                 load_expand<0>(x, tile, pos, op);
             else if (n_exp == 1)
-                load_expand<1>(x, tile, pos, op + 2 * gr.op0);
+                load_expand<1>(x, tile, pos, op + 2 * op0);
             else if (n_exp == 2)
-                load_expand<2>(x, tile, pos, op + 2 * gr.op0);
+                load_expand<2>(x, tile, pos, op + 2 * op0);
             else
-                load_expand<3>(x, tile, pos, op + 2 * gr.op0);
+                load_expand<3>(x, tile, pos, op + 2 * op0);
             // where a condition holds over the register indices
             auto cond = [&](uint32_t lam, uint32_t qpat, uint32_t tp, uint32_t i) -> uint32_t {
                 const uint32_t t = ((uint32_t)__popc(base & lam) ^ (tp >> i)) & 1u;
                 return (qpat ^ (0u - t)) & ALL;
             };
-            for (uint32_t i = gr.op0 + n_exp; i < gr.op1; ++i) {
+            for (uint32_t i = op0 + n_exp; i < op1; ++i) {
                 const uint4 h = op[2 * i];  // kind, j, n_cond, flags | lam | qpat | slot, pad, delta
                 const uint32_t kind = h.x & 0xffu, j = (h.x >> 8) & 0xffu, flags = h.x >> 24;
                 const T* cf = coef(h.w & 0xffu);
-                const uint32_t c0 = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
                 switch (kind) {
                     case M_PHASE: {
                         const T ph = cf[0];
+                        if (kAxes && (flags & MF_PLAIN)) {
+                            pair_op(j, [&](auto J) { phase_half<decltype(J)::value>(x, ph); });
+                            break;
+                        }
+                        const uint32_t hit = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                        if (!hit) break;
 #pragma unroll
                         for (uint32_t q = 0; q < kRegs; ++q) {
                             const T w = cmul(x[q], ph);
-                            x[q] = ((c0 >> q) & 1u) ? w : x[q];
+                            x[q] = ((hit >> q) & 1u) ? w : x[q];
                         }
                         break;
                     }
                     case M_NEG: {
-                        uint32_t hit = c0;
+                        uint32_t hit = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
                         if (((h.x >> 16) & 0xffu) > 1u) hit &= cond(h.y >> 16, h.z >> 16, tp1, i);
+                        if (!hit) break;
 #pragma unroll
                         for (uint32_t q = 0; q < kRegs; ++q) {
                             const R sg = sign_of(hit, q);
@@ -2849,11 +2874,20 @@ struct Shot {
                         }
                         break;
                     }
-                    case M_U4: apply_u4(x, c0, cond(h.y >> 16, h.z >> 16, tp1, i), cf); break;
+                    case M_U4:
+                        if constexpr (kAxes)
+                            apply_u4(x, axis_bit(0), axis_bit(1), cf);
+                        else
+                            apply_u4(x, cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i), cond(h.y >> 16, h.z >> 16, tp1, i), cf);
+                        break;
                     case M_EXPAND: {
                         const T ph = cf[0];
                         const bool copy = (flags & MF_COPY) != 0;
-                        pair_op(j, [&](auto J) { expand_pairs<decltype(J)::value>(x, c0, ph, copy); });
+                        const uint32_t side = kAxes ? 0u : cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                        pair_op(j, [&](auto J) {
+                            constexpr int V = decltype(J)::value;
+                            expand_pairs<V>(x, kAxes ? axis_bit(V) : side, ph, copy);
+                        });
                         if (any_scale) {
                             const T c = cf[16];  // the next slot
                             if (c.y != (R)0) {
@@ -2863,9 +2897,23 @@ struct Shot {
                         }
                         break;
                     }
-                    case M_CX: pair_op(j, [&](auto J) { swap_pairs<decltype(J)::value>(x, c0); }); break;
-                    case M_H: pair_op(j, [&](auto J) { h_pairs<decltype(J)::value>(x, c0); }); break;
-                    default: pair_op(j, [&](auto J) { u2_pairs<decltype(J)::value>(x, c0, cf); }); break;  // M_U2
+                    case M_CX: {
+                        const uint32_t hit = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                        pair_op(j, [&](auto J) { swap_pairs<decltype(J)::value>(x, hit); });
+                        break;
+                    }
+                    case M_H: {
+                        const uint32_t side = cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                        pair_op(j, [&](auto J) { h_pairs<decltype(J)::value>(x, side); });
+                        break;
+                    }
+                    default: {  // M_U2
+                        const uint32_t side = kAxes ? 0u : cond(h.y & 0xffffu, h.z & 0xffffu, tp0, i);
+                        pair_op(j, [&](auto J) {
+                            constexpr int V = decltype(J)::value;
+                            u2_pairs<V>(x, kAxes ? axis_bit(V) : side, cf);
+                        });
+                    }
                 }
             }
             if (sum) {
@@ -2877,7 +2925,7 @@ struct Shot {
                     w[q] = cnorm_d(x[q]);
                     if (Grp::kTeam && pos[q] >= filled) w[q] = 0.0;
                 }
-                const uint32_t j = gr.side_j;
+                const uint32_t j = bp->side_j;
                 if (j < SIDE_ANY) {
                     pair_op(j, [&](auto J) { sum_halves<decltype(J)::value>(w, q0, q1); });
                     if (j == SIDE_NONE) {
@@ -2885,7 +2933,7 @@ struct Shot {
                         q1 = 0.0;
                     }
                 } else {
-                    const uint32_t qp = gr.side_qpat;
+                    const uint32_t qp = bp->side_qpat;
                     q0 = q1 = 0.0;
 #pragma unroll
                     for (uint32_t q = 0; q < kRegs; ++q) {
@@ -2895,18 +2943,19 @@ struct Shot {
                             q0 += w[q];
                     }
                 }
-                const bool flip = (((uint32_t)__popc(base & side_lam) ^ side_tile) & 1u) != 0;
+                const bool flip = (((uint32_t)__popc(base & bp->side_lam) ^ side_tile) & 1u) != 0;
                 acc[0] += flip ? q1 : q0;
                 acc[1] += flip ? q0 : q1;
             }
             if (store) {
-                uint32_t to = base;
-                if (gr.n_fin) {
+                uint32_t to = base, s1 = o1, s2 = o2, s4 = o4;
+                if (sum && bp->n_cx) {
 #pragma unroll
                     for (uint32_t c = 0; c < 2; ++c)
-                        to ^= ((uint32_t)__popc(base & gr.fin_lam[c]) ^ (tp0 >> (gr.op1 + c))) & 1u ? gr.fin_dir[c] : 0u;
+                        to ^= ((uint32_t)__popc(base & bp->fin_lam[c]) ^ (tp0 >> (gr.op1 + c))) & 1u ? bp->fin_dir[c] : 0u;
+                    s1 = bp->sv[0], s2 = bp->sv[1], s4 = bp->sv[2];
                 }
-                const uint32_t s1 = gr.sv[0], s2 = gr.sv[1], s4 = gr.sv[2], s3 = s1 ^ s2;
+                const uint32_t s3 = s1 ^ s2;
                 const uint32_t out[kRegs] = {to,      to ^ s1,      to ^ s2,      to ^ s3,
                                              to ^ s4, to ^ s4 ^ s1, to ^ s4 ^ s2, to ^ s4 ^ s3};
 #pragma unroll
@@ -2950,6 +2999,15 @@ struct Shot {
         constexpr int A = J == 0 ? 2 : 1, B = J == 2 ? 2 : 4, H = 1 << J;
         q0 = (w[0] + w[A]) + (w[B] + w[A + B]);
         q1 = (w[H] + w[H + A]) + (w[H + B] + w[H + A + B]);
+    }
+    static constexpr bool kAxes = Grp::kCta;
+    // register indices with bit j set
+    static __device__ __forceinline__ constexpr uint32_t axis_bit(int j) { return j == 0 ? 0xaau : j == 1 ? 0xccu : 0xf0u; }
+    template <int J>
+    static __device__ __forceinline__ void phase_half(T (&x)[kRegs], T ph) {
+#pragma unroll
+        for (uint32_t q = 0; q < kRegs; ++q)
+            if (q & (1u << J)) x[q] = cmul(x[q], ph);
     }
     template <int J>
     static __device__ __forceinline__ void expand_pairs(T (&x)[kRegs], uint32_t side, T ph, bool copy) {
@@ -3011,7 +3069,7 @@ struct Shot {
                 x[q | (1u << J)] = on ? u : w;
             }
     }
-    // directions 0 (the low axis) and 1 of the group; s0, s1: their sides
+    // U4 along directions 0 and 1
     static __device__ __forceinline__ void apply_u4(T (&x)[kRegs], uint32_t s0, uint32_t s1, const T* c) {
 #pragma unroll
         for (uint32_t q = 0; q < kRegs; q += 4) {

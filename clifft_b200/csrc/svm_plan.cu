@@ -296,77 +296,148 @@ struct Builder {
     }
 
     // ---- groups of micro-ops that share a pass over the tile
-    void close_group(uint32_t op0, uint32_t op1, std::vector<uint32_t> dirs, const BlockPlan& b, bool last) {
-        PlanGroup gr{};
-        if (last && b.side_lam) {
-            // at most one direction on which the measured bit changes, as far
-            // as the ops leave their directions free: the sums of both halves
-            // are then over fixed registers
-            auto bound = [&](uint32_t j) {
-                for (uint32_t i = op0; i < op1 - b.n_cx; ++i) {
-                    const PlanOp& o = out.ops[b.first_op + i];
-                    if (o.delta && (o.j == j || (o.kind == M_U4 && j < 2))) return true;
-                }
-                return false;
-            };
-            uint32_t at = ~0u;
-            for (uint32_t j = 0; j < dirs.size(); ++j)
-                if (parity(dirs[j] & b.side_lam) && (at == ~0u || (!bound(at) && bound(j)))) at = j;
-            for (uint32_t j = 0; j < dirs.size(); ++j)
-                if (at != ~0u && j != at && parity(dirs[j] & b.side_lam) && !bound(j)) dirs[j] ^= dirs[at];
-        }
+    struct Dir {
+        uint32_t v;
+        bool free;  // not an op's own: only the span matters
+        bool axis;  // has an axis bit (lam, ell, at)
+        uint32_t lam;
+        uint64_t ell;
+        uint8_t at;
+    };
+    using Dirs = std::vector<Dir>;
+    static bool in_span(const Dirs& dirs, uint32_t v) {
         Span s;
-        uint32_t pivots = 0;
-        for (uint32_t d : dirs) s.add(d);
-        for (uint64_t v : s.v) pivots |= 1u << top_bit(v);
-        for (uint32_t a = g.bits; a-- > 0 && dirs.size() < kGroupDirs;)
-            if (!((pivots >> a) & 1u)) {
-                dirs.push_back(1u << a);
-                pivots |= 1u << a;
+        for (const Dir& d : dirs) s.add(d.v);
+        return s.reduce(v) == 0;
+    }
+    // v without its part along the directions that have an axis bit
+    static uint32_t off_axes(const Dirs& dirs, uint32_t v) {
+        uint32_t x = v;
+        for (const Dir& d : dirs)
+            if (d.axis && parity(d.lam & v)) x ^= d.v;
+        return x;
+    }
+    static bool has_axis(const Dirs& dirs, uint32_t j, uint64_t ell) { return dirs[j].axis && dirs[j].ell == ell; }
+    // Adds what micro-op i moves along to a group's directions; false when it
+    // needs a group of its own: no direction left, or axis bits that would no
+    // longer be those of the register index.
+    static bool join(Dirs& dirs, PlanOp& o, uint8_t i, const uint32_t* want, uint32_t n_want) {
+        if (o.flags & MF_LINEAR) {  // a swap before a measurement: stored, not moved
+            if (in_span(dirs, want[0])) return true;
+            if (dirs.size() >= kGroupDirs) return false;
+            dirs.push_back({off_axes(dirs, want[0]), true, false, 0, 0, 0});
+            return true;
+        }
+        for (uint32_t w = 0; w < n_want; ++w) {
+            uint32_t idx = 0;
+            while (idx < dirs.size() && dirs[idx].v != want[w]) ++idx;
+            if (idx == dirs.size()) {
+                if (idx >= kGroupDirs || in_span(dirs, want[w]) || off_axes(dirs, want[w]) != want[w]) return false;
+                dirs.push_back({want[w], false, false, 0, 0, 0});
             }
-        uint32_t w = pivots;
-        for (uint32_t j = 0; j < kGroupDirs; ++j, w &= w - 1) {
-            gr.qv[j] = (uint16_t)dirs[j];
+            if (o.kind == M_U4 && idx != w) return false;  // U4 owns the first two directions
+            if (o.kind != M_CX) {
+                if (dirs[idx].axis) {
+                    if (dirs[idx].ell != o.ell[w]) return false;
+                } else {
+                    for (uint32_t q = 0; q < dirs.size(); ++q)
+                        if (parity(o.lam[w] & dirs[q].v) != (q == idx)) return false;
+                    dirs[idx] = {want[w], false, true, o.lam[w], o.ell[w], uint8_t(i | (w ? 32u : 0u))};
+                }
+            }
+            if (w == 0) o.j = (uint8_t)idx;
+        }
+        return true;
+    }
+    void close_group(uint32_t op0, uint32_t op1, Dirs dirs, BlockPlan& b, bool last) {
+        PlanGroup gr{};
+        const uint32_t fin0 = last ? op1 - b.n_cx : op1;
+        PlanOp* ops = out.ops.data() + b.first_op;
+        // directions left over: axis bits of phases, then any
+        for (uint32_t i = op0; i < fin0 && dirs.size() < kGroupDirs; ++i) {
+            const PlanOp& o = ops[i];
+            if (o.kind != M_PHASE || !o.lam[0]) continue;
+            bool clear = true;
+            for (const Dir& d : dirs) clear = clear && !parity(o.lam[0] & d.v);
+            if (clear) dirs.push_back({off_axes(dirs, 1u << top_bit(o.lam[0])), false, true, o.lam[0], o.ell[0], (uint8_t)i});
+        }
+        for (uint32_t a = g.bits; a-- > 0 && dirs.size() < kGroupDirs;)
+            if (!in_span(dirs, 1u << a)) dirs.push_back({off_axes(dirs, 1u << a), true, false, 0, 0, 0});
+        if (last && b.term_kind) {
+            // the measured bit changes along at most one free direction
+            uint32_t at = kGroupDirs;
+            for (uint32_t j = 0; j < kGroupDirs; ++j) {
+                if (!dirs[j].free || !parity(dirs[j].v & b.side_lam)) continue;
+                if (at == kGroupDirs)
+                    at = j;
+                else
+                    dirs[j].v ^= dirs[at].v;
+            }
+        }
+        // Finding register 0 costs about 20 instructions per coset. A U2 or U4
+        // saves more in selects, two phases in multiplications; H applies its
+        // sides as signs and saves less. Warps, at two cosets per thread and
+        // tile, pay for the code alone (k = 16, 10^4 shots 6.7 ms with it, 6.4
+        // without); teams gain (k = 20, 394 opcodes, 150 shots 53 -> 48 ms).
+        Span s;
+        uint32_t pivots = 0, gain = 0;
+        for (const Dir& d : dirs) s.add(d.v);
+        for (uint64_t v : s.v) pivots |= 1u << top_bit(v);
+        // a fresh axis is a physical bit of the tile: nothing outside adds to
+        // it, and it is clear where the pivots are
+        auto fresh = [&](const PlanOp& o) { return o.kind == M_EXPAND && !(o.lam[0] & ~pivots); };
+        for (uint32_t i = op0; i < fin0; ++i) {
+            const bool needs = ops[i].kind == M_U2 || ops[i].kind == M_U4 || (ops[i].kind == M_EXPAND && !fresh(ops[i]));
+            gain += needs ? 2 : ops[i].kind == M_PHASE ? 1 : 0;
+        }
+        const bool axes = g.axes && gain >= 2;
+        for (uint32_t j = 0, w = pivots; j < kGroupDirs; ++j, w &= w - 1) {
+            gr.qv[j] = (uint16_t)dirs[j].v;
             gr.piv[j] = (uint8_t)__builtin_ctz(w);
+            const bool flips = axes && dirs[j].axis && !fresh(ops[dirs[j].at & 31]);
+            gr.axis_lam[j] = flips ? (uint16_t)dirs[j].lam : 0;
+            gr.axis_at[j] = flips ? dirs[j].at : 31;
         }
         auto pattern = [&](uint32_t lam) {
             uint32_t p = 0;
             for (uint32_t q = 0; q < (1u << kGroupDirs); ++q) {
                 uint32_t x = 0;
                 for (uint32_t j = 0; j < kGroupDirs; ++j)
-                    if ((q >> j) & 1u) x ^= dirs[j];
+                    if ((q >> j) & 1u) x ^= dirs[j].v;
                 p |= parity(x & lam) << q;
             }
             return (uint16_t)p;
         };
+        gr.axes = axes;
         gr.op0 = (uint8_t)op0;
-        gr.op1 = (uint8_t)op1;
-        if (last && b.n_cx) {
-            // the swaps before a measurement, by the stores: both conditions
-            // on the position before them
-            gr.n_fin = (uint8_t)b.n_cx;
-            gr.op1 = (uint8_t)(op1 - b.n_cx);
+        gr.op1 = (uint8_t)fin0;
+        for (uint32_t i = op0; i < op1; ++i)
+            for (int c = 0; c < 2; ++c) ops[i].qpat[c] = pattern(ops[i].lam[c]);
+        for (uint32_t i = op0; i < fin0; ++i) {
+            PlanOp& o = ops[i];
+            if (i == op0 + gr.n_exp && o.kind == M_EXPAND && o.j == gr.n_exp && (axes || fresh(o))) gr.n_exp++;
+            if (o.kind == M_PHASE && axes)
+                for (uint8_t j = 0; j < kGroupDirs; ++j)
+                    if (has_axis(dirs, j, o.ell[0])) {
+                        o.flags |= MF_PLAIN;
+                        o.j = j;
+                    }
         }
-        for (uint32_t i = op0; i < op1; ++i) {
-            PlanOp& o = out.ops[b.first_op + i];
-            for (int c = 0; c < 2; ++c) o.qpat[c] = pattern(o.lam[c]);
-            if (i == op0 + gr.n_exp && o.kind == M_EXPAND && o.j == gr.n_exp && o.qpat[0] == kPattern[o.j] &&
-                (o.lam[0] & ~pivots) == 0)
-                gr.n_exp++;
+        if (last && b.term_kind) {
+            for (uint32_t j = 0; j < kGroupDirs; ++j) {
+                b.sv[j] = gr.qv[j];
+                for (uint32_t i = fin0; i < op1; ++i)
+                    if (parity(ops[i].lam[0] & gr.qv[j])) b.sv[j] ^= ops[i].delta;
+            }
+            for (uint32_t i = fin0; i < op1; ++i) {
+                b.fin_lam[i - fin0] = ops[i].lam[0];
+                b.fin_dir[i - fin0] = ops[i].delta;
+            }
+            b.side_qpat = (uint8_t)pattern(b.side_lam);
+            b.side_j = b.side_qpat ? SIDE_ANY : SIDE_NONE;
+            for (uint8_t j = 0; j < kGroupDirs; ++j)
+                if (b.side_qpat == kPattern[j]) b.side_j = j;
         }
-        for (uint32_t j = 0; j < kGroupDirs; ++j) {
-            gr.sv[j] = gr.qv[j];
-            for (uint32_t i = gr.op1; i < op1; ++i)
-                if (parity(out.ops[b.first_op + i].lam[0] & gr.qv[j])) gr.sv[j] ^= out.ops[b.first_op + i].delta;
-        }
-        for (uint32_t c = 0; c < gr.n_fin; ++c) {
-            gr.fin_lam[c] = out.ops[b.first_op + gr.op1 + c].lam[0];
-            gr.fin_dir[c] = out.ops[b.first_op + gr.op1 + c].delta;
-        }
-        if (last) gr.side_qpat = pattern(b.side_lam);
-        gr.side_j = gr.side_qpat ? SIDE_ANY : SIDE_NONE;
-        for (uint8_t j = 0; j < kGroupDirs; ++j)
-            if (gr.side_qpat == kPattern[j]) gr.side_j = j;
         out.groups.push_back(gr);
     }
     static constexpr uint16_t kPattern[kGroupDirs] = {0xaa, 0xcc, 0xf0};  // bit j of the register index
@@ -567,15 +638,8 @@ struct Builder {
         }
         if (g.dense_min_weight) find_dense(b, t.pivots(), fresh_local);
         // groups
-        auto join_again = [](const Op& o, const Tile& tile, std::vector<uint32_t>& into) {
-            for (uint64_t d : o.dir) {
-                if (!d) continue;
-                const uint32_t v = tile.position(d);
-                if (std::find(into.begin(), into.end(), v) == into.end()) into.push_back(v);
-            }
-        };
         b.first_group = (uint32_t)out.groups.size();
-        std::vector<uint32_t> dirs;
+        Dirs dirs, dirs_at_fin;
         uint32_t op0 = 0;
         auto close = [&](uint32_t op1, bool fin) {
             close_group(op0, op1, dirs, b, fin);
@@ -591,39 +655,21 @@ struct Builder {
                 i = b.dense1 - 1;
                 continue;
             }
-            const Op& o = ops[i];
-            if (!o.dir[0]) continue;
-            auto try_join = [&]() -> bool {
-                std::vector<uint32_t> want{t.position(o.dir[0])};
-                if (o.kind == M_U4) want.push_back(t.position(o.dir[1]));
-                uint32_t j = 0;
-                for (uint32_t w = 0; w < want.size(); ++w) {
-                    const auto at = std::find(dirs.begin(), dirs.end(), want[w]);
-                    uint32_t idx = uint32_t(at - dirs.begin());
-                    if (at == dirs.end()) {
-                        Span s;
-                        for (uint32_t d : dirs) s.add(d);
-                        if (dirs.size() >= kGroupDirs || !s.reduce(want[w])) return false;
-                        dirs.push_back(want[w]);
-                    }
-                    if (o.kind == M_U4 && idx != w) return false;  // U4 owns the first two directions
-                    if (w == 0) j = idx;
-                }
-                out.ops[b.first_op + i].j = (uint8_t)j;
-                return true;
-            };
-            const std::vector<uint32_t> before = dirs;
-            if (!try_join()) {
-                dirs = before;
-                // the two swaps before a measurement stay together
-                if (i > fin0) {
-                    i = fin0;
-                    dirs.clear();
-                    for (uint32_t q = op0; q < fin0; ++q) join_again(ops[q], t, dirs);
-                }
-                close(i, false);
-                --i;  // again, in the new group
+            if (i == fin0) dirs_at_fin = dirs;
+            if (!ops[i].dir[0]) continue;
+            const uint32_t want[2] = {t.position(ops[i].dir[0]), ops[i].kind == M_U4 ? (uint32_t)t.position(ops[i].dir[1]) : 0u};
+            Dirs joined = dirs;
+            if (join(joined, out.ops[b.first_op + i], (uint8_t)i, want, ops[i].kind == M_U4 ? 2 : 1)) {
+                dirs = std::move(joined);
+                continue;
             }
+            // the two swaps before a measurement stay together
+            if (i > fin0) {
+                i = fin0;
+                dirs = dirs_at_fin;
+            }
+            close(i, false);
+            --i;  // again, in the new group
         }
         // the closing group also sums a measured axis' halves; a dense run at
         // the very end leaves an empty one for that

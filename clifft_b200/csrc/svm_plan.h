@@ -37,12 +37,13 @@ enum : uint8_t {
 enum : uint8_t {
     MF_COPY = 0x1,    // EXPAND without a phase
     MF_LINEAR = 0x2,  // the condition is on the physical index (it does not see xl)
+    MF_PLAIN = 0x4,   // PHASE: the condition is the axis bit of its group's direction j
 };
 
 // A micro-op. Condition c holds at tile position l of a tile at `base` when
 // the parity of l & lam[c], base & ell[c] and xl & ell[c] is odd. For the
-// opcodes along a direction, condition 0 tells the side (its logical bit; U4:
-// conditions 0 and 1 those of its two axes).
+// opcodes along a direction, condition 0 is its axis bit (U4: conditions 0 and 1
+// those of its two axes).
 struct PlanOp {
     uint8_t kind, j, n_cond, flags;  // j: which of its group's directions
     uint16_t lam[2];
@@ -54,24 +55,24 @@ struct PlanOp {
 static_assert(sizeof(PlanOp) == 32, "copied in 16-byte words");
 
 // Consecutive micro-ops that one pass over the tile applies in registers: a
-// thread holds the 8 amplitudes that the group's directions connect.
+// thread holds the 8 amplitudes that the group's directions connect. With
+// `axes` set, register 0 is the one whose axis bits (one per direction: the
+// parity of the tile position with axis_lam and the tile's part of condition
+// axis_at) are all clear, so register q has the axis bits of q and U2, U4,
+// EXPAND and the phases of those axes need no conditions.
 struct PlanGroup {
-    uint16_t qv[3];      // directions (tile positions); unused ones are free unit vectors
+    uint16_t qv[3];        // directions (tile positions); unused ones are free vectors
     uint8_t op0, op1;
-    uint8_t piv[3];      // their pivot bits, ascending: a coset's base has them clear
-    uint8_t n_fin;       // swaps before a measurement (ops from op1), made by where the amplitudes are stored
-    uint16_t side_qpat;  // last group of a measured block: the measured axis' bit
-    uint8_t n_exp;       // leading EXPANDs along directions 0, 1, .. whose clear halves are the
-                         // registers with those index bits clear
-    uint8_t side_j;      // side_qpat is that of direction 0..2, SIDE_NONE: zero, SIDE_ANY: another
-    uint16_t sv[3];      // where a coset is stored: its base, moved along the swaps' directions as
-                         // their conditions there say, and these directions
-    uint16_t fin_lam[2], fin_dir[2];  // the swaps: conditions and directions (none: 0)
-    uint16_t pad;
+    uint8_t piv[3];        // pivot bits of their span, ascending: one position of a coset has them clear
+    uint8_t n_exp;         // leading EXPANDs along directions 0, 1, ..
+    uint16_t axis_lam[3];  // 0: no axis bit, or one that is clear where the pivots are
+    uint8_t axis_at[3];    // micro-op of the block, + 32 for its condition 1; 31: none
+    uint8_t axes;          // any of them set
+    uint8_t pad[10];
 };
-enum : uint8_t { SIDE_NONE = 3, SIDE_ANY = 4 };
 static_assert(sizeof(PlanGroup) == 32, "copied in 16-byte words");
 
+enum : uint8_t { SIDE_NONE = 3, SIDE_ANY = 4 };
 enum : uint32_t { BLOCK_PASS, BLOCK_EXP_VAL, BLOCK_END };
 
 // One fused block: instructions [pc, pc + n_instr) of the device stream.
@@ -99,12 +100,21 @@ struct BlockPlan {
     uint32_t single;     // the state is one tile, already in shared memory
     uint32_t cols_at, cols_n;  // columns of M (PlanSet::cols) to undo it after the block; 0: nothing to undo
     uint32_t dense0, dense1, dense_mask;  // dense geometry: ops [dense0, dense1) as one matrix on those four tile bits
+    // the last group of a measured block: register indices (side_qpat) on which
+    // the measured bit differs from register 0's, whether that is a direction's
+    // index bit (0..2; SIDE_NONE: on none, SIDE_ANY: another pattern), and the
+    // swaps that make the measured bit the top one, by the addresses stored
+    // to: register 0's, moved along fin_dir where fin_lam (and the tile's part
+    // of the ops after the group) holds, then along sv
+    uint16_t sv[3], fin_lam[2], fin_dir[2];
+    uint8_t side_qpat, side_j;
 };
 static_assert(sizeof(BlockPlan) % 16 == 0, "copied in 16-byte words");
 
 struct PlanGeometry {
     uint32_t bits;     // log2 of the amplitudes per tile
     uint32_t max_ops;  // micro-op slots per block (1: one opcode per pass)
+    bool axes;         // groups may find their register 0 by axis bits (CTAs)
     bool team;         // a team of CTAs, which keeps states of at most one tile in shared memory
     uint32_t dense_min_weight;  // > 0: find runs for the tensor cores (no relabelling then)
 };
