@@ -271,11 +271,12 @@ void clifft_gpu_batch_free(clifft_gpu_batch* batch);
  * parameter vectors (args->phases, batch x num_rot_params, or NULL to use the
  * program's own payloads for every row) the call returns every EXP_VAL row
  * (exp_vals, batch x num_exp_vals) and its derivatives (grads, batch x
- * num_exp_vals x num_rot_params). The kernel runs each (vector, EXP_VAL) pair
- * forward to the EXP_VAL, then back through the bytecode, undoing each
- * instruction with its inverse (no per-instruction state is stored) and
- * accumulating the derivatives in FP64; args->precision selects the
- * statevector precision. Programs with measurements, noise, classical records
+ * num_exp_vals x num_rot_params). A program without ARRAY_H is a phase
+ * polynomial, whose derivatives are one transform per (vector, EXP_VAL) pair;
+ * otherwise the kernel runs each pair forward to the EXP_VAL, then back
+ * through the bytecode, undoing each instruction with its inverse (no
+ * per-instruction state is stored) and accumulating the derivatives in FP64;
+ * args->precision selects the statevector precision. Programs with measurements, noise, classical records
  * or fused U2 / U4 nodes are rejected (CLIFFT_GPU_EINVAL).
  */
 typedef struct clifft_gpu_grad_args {
