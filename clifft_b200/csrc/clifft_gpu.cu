@@ -238,7 +238,9 @@ uint32_t validate(const clifft_program_image& im) {
 // tests/golden/programs shrink 3x to 12x (memory grid 4145 -> 1018, k = 24
 // 8204 -> 692 instructions), and an interpreted frame opcode costs a shot 200
 // to 570 cycles whatever it does. A run of at least kMinStar gates is
-// condensed; a pair costs about the same either way.
+// condensed; a pair costs about the same either way. The unused second half of
+// a Pauli correction holds its mask (frames of one word) and that of a record
+// parity its list, when that has at most kInlineTargets entries.
 struct CodeStream {
     std::vector<uint8_t> bytes;    // 32 bytes per instruction
     std::vector<uint32_t> origin;  // index of each one's (first) instruction in the image
@@ -307,6 +309,19 @@ CodeStream condense(const clifft_program_image& im, uint32_t nwt) {
         c.origin.push_back(i);
         if (!dop) {
             std::memcpy(J, I, 32);
+            const uint32_t p0 = rd32(I + 8);
+            if (I[0] == CLIFFT_OP_APPLY_PAULI && nwt == 1) {
+                const uint64_t mask[2] = {im.num_words ? im.pauli_x[p0] : 0, im.num_words ? im.pauli_z[p0] : 0};
+                std::memcpy(J + 16, mask, 16);
+                if (im.pauli_sign[p0]) J[2] |= DFLAG_PAULI_SIGN;
+            } else if (I[0] == CLIFFT_OP_DETECTOR || I[0] == CLIFFT_OP_POSTSELECT || I[0] == CLIFFT_OP_OBSERVABLE) {
+                const bool obs = I[0] == CLIFFT_OP_OBSERVABLE;
+                const uint32_t* off = (obs ? im.observable_offsets : im.detector_offsets) + p0;
+                const uint32_t* tg = (obs ? im.observable_targets : im.detector_targets) + off[0];
+                uint32_t w[1 + kInlineTargets] = {off[1] - off[0]};
+                for (uint32_t t = 0; w[0] <= kInlineTargets && t < w[0]; ++t) w[1 + t] = tg[t];
+                std::memcpy(J + 16, w, sizeof(w));
+            }
         } else {
             uint64_t m[kMaxWords] = {};
             for (uint32_t j = i; j < end; ++j) {

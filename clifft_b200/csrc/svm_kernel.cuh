@@ -183,6 +183,10 @@ enum : uint32_t {
     DOP_CNOT_GATHER = 65,
     DOP_CZ_FAN = 66,
 };
+// device-only flag of an APPLY_PAULI that carries its mask: the mask's sign
+constexpr uint32_t DFLAG_PAULI_SIGN = 0x80u;
+// record lists of at most this many entries travel in their instruction
+constexpr uint32_t kInlineTargets = 3;
 __host__ __device__ constexpr bool frame_op(uint32_t op) { return op <= CLIFFT_OP_FRAME_SWAP || op >= DOP_CNOT_FAN; }
 
 enum : int {
@@ -1948,8 +1952,24 @@ struct Shot {
             rec_dirty = true;
         }
     }
+    // Parity of the records in list l, which instruction cur_pc carries when it
+    // is short: one load at a known address instead of three dependent ones
+    // (400000 post-selected shots of the k = 5 memory 2.24 -> 2.13 ms with the
+    // Pauli masks, which travel likewise). Not in CTA groups: their kernels
+    // are at the edge of what the compiler inlines, and these lines pushed the
+    // teams' over it (k = 24, one shot 0.86 -> 1.70 ms).
+    static constexpr bool kInlineLists = !Grp::kCta;
     __device__ __forceinline__ int list_parity(const uint32_t* off, const uint32_t* tg, uint32_t l) {
         int p = 0;
+        if constexpr (kInlineLists) {
+            const uint4 in = __ldg(P.code + 2 * cur_pc + 1);
+            if (in.x <= kInlineTargets) {
+                if (in.x > 0) p = bit_of(rec, in.y, S);
+                if (in.x > 1) p ^= bit_of(rec, in.z, S);
+                if (in.x > 2) p ^= bit_of(rec, in.w, S);
+                return p;
+            }
+        }
         const uint32_t e = __ldg(off + l + 1);
         for (uint32_t i = __ldg(off + l); i < e; ++i) p ^= bit_of(rec, __ldg(tg + i), S);
         return p;
@@ -2014,6 +2034,18 @@ struct Shot {
         switch (op) {
             case CLIFFT_OP_APPLY_PAULI:
                 flush_records();
+                if constexpr (NW == 1 && kInlineLists) {
+                    const uint4 m = __ldg(P.code + 2 * cur_pc + 1);
+                    if (bit_of(rec, p1, S)) {
+                        const uint64_t mx = ((uint64_t)m.y << 32) | m.x, mz = ((uint64_t)m.w << 32) | m.z;
+                        const bool odd = (__popcll(f.x[0] & mz) & 1) != 0;
+                        f.x[0] ^= mx;
+                        f.z[0] ^= mz;
+                        if (odd) negate_gamma();
+                        if (fl & DFLAG_PAULI_SIGN) negate_gamma();
+                    }
+                    break;
+                }
                 if (bit_of(rec, p1, S))
                     apply_pauli(P.pauli_x + (size_t)p0 * NW, P.pauli_z + (size_t)p0 * NW,
                                 P.pauli_sign[p0] != 0);
